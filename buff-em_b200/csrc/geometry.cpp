@@ -287,7 +287,25 @@ int upload_geometry(bg_geometry *g) {
       bfV.push_back(make_int4(F.iV1 + vo, F.iV2 + vo, F.iV3 + vo, (int)no));
       area.push_back(F.area);
       radius.push_back(F.radius);
+      g->bf_rmax = std::max(g->bf_rmax, F.radius);
     }
+    // twice the largest distance of a vertex from the middle of the bounding box
+    double lo[3], hi[3], far2 = 0.0;
+    for (int k = 0; k < 3; k++) lo[k] = hi[k] = o.nv ? o.V[k] : 0.0;
+    for (int v = 0; v < o.nv; v++)
+      for (int k = 0; k < 3; k++) {
+        lo[k] = std::min(lo[k], o.V[3 * v + k]);
+        hi[k] = std::max(hi[k], o.V[3 * v + k]);
+      }
+    for (int v = 0; v < o.nv; v++) {
+      double d2 = 0.0;
+      for (int k = 0; k < 3; k++) {
+        const double x = o.V[3 * v + k] - 0.5 * (lo[k] + hi[k]);
+        d2 += x * x;
+      }
+      far2 = std::max(far2, d2);
+    }
+    g->obj_diam = std::max(g->obj_diam, 2.0 * std::sqrt(far2));
     mats.push_back(o.mat);
     for (int k = 0; k < 3; k++) origin.push_back(o.origin[k]);
   }

@@ -223,6 +223,8 @@ struct bg_geometry {
   bool uploaded = false, precomputed = false;
   bool dispersive = false;      // some object's eps comes from a MATERIAL section
   double rule_rmax = 0.0;       // largest distance of a 4-point rule point from its tetrahedron's centroid
+  double bf_rmax = 0.0;         // largest basis-function radius
+  double obj_diam = 0.0;        // bound on the distance of two points of one object
   bg::NearGraph graph;
   double *d_scratch = nullptr;  // general scratch (PFT partial sums etc.)
   double *d_fieldTet = nullptr, *d_fieldFace = nullptr;  // GetFields tables, 16 doubles per tet each

@@ -1283,6 +1283,8 @@ __global__ void k_pft_ext(PftArgs P, PWave pw, double *part) {
   }
 }
 
+#include "emt_pairs.cuh"
+
 // OPFT absorbed power (OPFT.cc:62-119, OverlapIntegrand_PFT PAbs term,
 // OverlapIntegrals.cc:79-170,242-298): sum Re(conj(Ja) Jb ME_ab),
 // ME_ab = 1/2 int b_a . (i Z0/w)(eps-1)^-1 . b_b on the shared tetrahedron.
@@ -1411,9 +1413,94 @@ int pft(bg_geometry *g, double wr, double wi, const void *dJ, const double *E0, 
   return BG_OK;
 }
 
+// Taylor coefficients of Im(phi), Im(psi) in r^2 (emt_pairs.cuh)
+static EmtKernel emt_kernel(double k) {
+  EmtKernel K{};
+  K.k = k;
+  K.k2 = k * k;
+  K.tiny2 = (2.0e-2 / k) * (2.0e-2 / k);
+  double f = 1.0, p = 1.0;   // (2n + 1)!, (-k^2)^n
+  for (int n = 0; n < EMT_MAXT; n++) {
+    if (n) { f *= (2.0 * n) * (2.0 * n + 1.0); p *= -K.k2; }
+    K.c[n] = p / f;
+    K.d[n] = -p * (2.0 * n + 2.0) / (f * (2.0 * n + 2.0) * (2.0 * n + 3.0));
+  }
+  return K;
+}
+// terms that reach 2e-17 of the value at r = 0 up to |k| r = x; 0: no polynomial
+static int emt_terms(double x) { return x <= 1.0 ? 9 : (x <= 2.0 ? 12 : (x <= 4.0 ? 16 : 0)); }
+
+static int emt_add_job(EmtReduce &R, const double *src, long long rows, int width, double *dst) {
+  if (rows > 0) {
+    R.src[R.n] = src; R.rows[R.n] = rows; R.width[R.n] = width; R.dst[R.n] = dst;
+    R.wmax = std::max(R.wmax, width);
+    R.n++;
+  }
+  return 0;
+}
+
+// pair sums through tetrahedra: far (job per object pair), near and self
+// partials into the scratch from `s` on; the sums' places are sums[0..]:
+// NO*NO*NPQ far, NO*NPQ near, NO self
+static int emt_tet_sums(bg_geometry *g, const PftArgs &P, double *s, double *sums, EmtReduce &R,
+                        const EmtBlockMap &bm, int nfar, int near_blocks, int near_per, int self_blocks) {
+  const int NO = P.nobj;
+  const EmtKernel K = emt_kernel(P.w);
+  const bool dr = P.DR != nullptr;
+  const int nt_far = emt_terms(std::fabs(P.w) * g->obj_diam);
+  const int nt_near = emt_terms(std::fabs(P.w) * std::min(g->obj_diam, 4.01 * g->bf_rmax));
+  // the points first: they are read as 16-byte pairs (s is 16-byte aligned)
+  double *pts = s, *pfar = pts + (dr ? 0 : (size_t)4 * g->NT * EMT_PT), *pnear = pfar + (size_t)nfar * NPQ,
+         *pself = pnear + (size_t)near_blocks * NO * NPQ;
+  if (!dr) {
+    k_emt_points<<<(4 * g->NT + 127) / 128, 128, 0, stream()>>>(g->dev, P.J, 1.0 / P.w, pts);
+    BG_LAUNCHED();
+    switch (nt_far) {
+      case 9: k_emt_far<9><<<nfar, EMT_JT, 0, stream()>>>(g->dev, K, bm, pts, pfar); break;
+      case 12: k_emt_far<12><<<nfar, EMT_JT, 0, stream()>>>(g->dev, K, bm, pts, pfar); break;
+      case 16: k_emt_far<16><<<nfar, EMT_JT, 0, stream()>>>(g->dev, K, bm, pts, pfar); break;
+      default: k_emt_far<0><<<nfar, EMT_JT, 0, stream()>>>(g->dev, K, bm, pts, pfar); break;
+    }
+  } else {
+    switch (nt_far) {
+      case 9: k_emt_far_dr<9><<<nfar, EMT_DJ, 0, stream()>>>(P, K, bm, pfar); break;
+      case 12: k_emt_far_dr<12><<<nfar, EMT_DJ, 0, stream()>>>(P, K, bm, pfar); break;
+      case 16: k_emt_far_dr<16><<<nfar, EMT_DJ, 0, stream()>>>(P, K, bm, pfar); break;
+      default: k_emt_far_dr<0><<<nfar, EMT_DJ, 0, stream()>>>(P, K, bm, pfar); break;
+    }
+  }
+  BG_LAUNCHED();
+  for (int m = 0; m < bm.nmap; m++)
+    emt_add_job(R, pfar + (size_t)bm.first[m] * NPQ, (m + 1 < bm.nmap ? bm.first[m + 1] : nfar) - bm.first[m], NPQ,
+                sums + (size_t)(bm.oa[m] * NO + bm.ob[m]) * NPQ);
+  if (near_blocks > 0) {
+    const int T = EMT_NG * 16;
+#define EMT_NEAR(n)                                                                                              \
+  case n:                                                                                                        \
+    if (dr) k_emt_near<n, true><<<near_blocks, T, 0, stream()>>>(P, g->near, K, near_per, pnear);                \
+    else k_emt_near<n, false><<<near_blocks, T, 0, stream()>>>(P, g->near, K, near_per, pnear);                  \
+    break;
+    switch (nt_near) { EMT_NEAR(9) EMT_NEAR(12) EMT_NEAR(16) EMT_NEAR(0) }
+#undef EMT_NEAR
+    BG_LAUNCHED();
+    emt_add_job(R, pnear, near_blocks, NO * NPQ, sums + (size_t)NO * NO * NPQ);
+  }
+  if (self_blocks > 0) {
+    k_emt_self<<<self_blocks, 256, 0, stream()>>>(P, pself);
+    BG_LAUNCHED();
+    emt_add_job(R, pself, self_blocks, NO, sums + (size_t)(NO * NO + NO) * NPQ);
+  }
+  return BG_OK;
+}
+
 // GetPFTMatrix with EMT (GetPFT.cc:133-189, EMTPFT.cc:324-493): out[8*no + c],
 // c = PAbs, PScat, Fx, Fy, Fz, Tx, Ty, Tz (force and torque in the
-// reference's units, TENTHIRDS = 10/3), plane-wave incident field
+// reference's units, TENTHIRDS = 10/3), plane-wave incident field.
+// The pair sums go through tetrahedra (emt_pairs.cuh) while every basis
+// function stays below the rule switch |omega| R = 5; above it pairs of one
+// tetrahedron pair ask for different rules and are taken one by one.  All
+// partial sums are added on the device in a fixed order; one small copy
+// returns them.
 static int pft_emt_impl(bg_geometry *g, double wr, double wi, const void *dJ, const void *dDR, size_t ldr,
                         const double *E0, const double *nhat, double *out) {
   int st = init_tables();
@@ -1423,45 +1510,89 @@ static int pft_emt_impl(bg_geometry *g, double wr, double wi, const void *dJ, co
   PftArgs P{g->dev, (const cd *)dJ, wr, std::sqrt(wr * wr + wi * wi), NO, (const cd *)dDR, ldr};
   int nrow = (g->N + 127) / 128;
   if ((st = build_near_lists(g))) return st;
-  int nb = (g->N + FT - 1) / FT;
-  size_t nfar = (size_t)nb * nb * NO * NO * NPQ;
-  int nnear_blocks = (g->near.npairs * 32 + 255) / 256;
-  size_t nnear = (size_t)std::max(nnear_blocks, 1) * NO * NPQ;
-  size_t next = (size_t)nrow * NO * NPQ;
-  if ((st = ensure_scratch(g, sizeof(double) * (nfar + nnear + next)))) return st;
-  double *pfar = g->d_scratch, *pnear = pfar + nfar, *pext = pnear + nnear;
-  k_pft_far<<<dim3(nb, nb), dim3(FT, FT), 0, stream()>>>(P, pfar);
-  BG_LAUNCHED();
-  if (g->near.npairs > 0) {
-    k_pft_near<<<nnear_blocks, 256, 0, stream()>>>(P, g->near, pnear);
+  const bool tets = P.absw * g->bf_rmax <= 5.0;
+  const int NP2 = NO * NO * NPQ;
+  // block partials of the far, near and self sums
+  size_t nfar = 0, nnear = 0, nself = 0, npts = 0;
+  EmtBlockMap bm{};
+  int far_blocks = 0, near_blocks = 0, near_per = 1, self_blocks = 0;
+  const int nb = (g->N + FT - 1) / FT;
+  if (tets) {
+    const int q = dDR ? 1 : 4, jt = dDR ? EMT_DJ : EMT_JT;
+    // short chunks while there are few points, so that every SM has blocks
+    bm.ic = dDR ? EMT_DI : (4 * g->NT <= 8192 ? EMT_JT : 4 * EMT_JT);
+    for (int oa = 0; oa < NO; oa++)
+      for (int ob = oa; ob < NO; ob++) {
+        const int m = bm.nmap;
+        bm.first[m] = far_blocks;
+        bm.oa[m] = oa; bm.ob[m] = ob;
+        bm.i0[m] = q * g->tOffset[oa]; bm.i1[m] = q * (g->tOffset[oa] + g->objs[oa].nt);
+        bm.j0[m] = q * g->tOffset[ob]; bm.j1[m] = q * (g->tOffset[ob] + g->objs[ob].nt);
+        bm.nj[m] = (bm.j1[m] - bm.j0[m] + jt - 1) / jt;
+        const long long nblk = (long long)bm.nj[m] * ((bm.i1[m] - bm.i0[m] + bm.ic - 1) / bm.ic);
+        if (nblk == 0) continue;
+        if (far_blocks + nblk > 0x7fffffffLL) { set_error("PFT: geometry too large"); return BG_ERR_ARG; }
+        far_blocks += (int)nblk;
+        bm.nmap++;
+      }
+    if (g->near.ntp > 0) {
+      near_blocks = std::min(148 * 8, (g->near.ntp + 4 * EMT_NG - 1) / (4 * EMT_NG));
+      near_per = (g->near.ntp + near_blocks * EMT_NG - 1) / (near_blocks * EMT_NG);
+    }
+    self_blocks = (g->N + 15) / 16;
+    nfar = (size_t)far_blocks * NPQ;
+    nnear = (size_t)near_blocks * NO * NPQ;
+    nself = (size_t)self_blocks * NO;
+    npts = dDR ? 0 : (size_t)4 * g->NT * EMT_PT;
+  } else {
+    near_blocks = (g->near.npairs * 32 + 255) / 256;
+    nfar = (size_t)nb * nb * NP2;
+    nnear = (size_t)near_blocks * NO * NPQ;
+  }
+  const size_t next = (size_t)nrow * NO * NPQ;
+  // sums first: far [NO][NO][NPQ], near [NO][NPQ], self [NO], extinction [NO][NPQ]
+  const size_t nsum = (size_t)NP2 + (size_t)NO * NPQ + NO + (size_t)NO * NPQ;
+  const size_t nsum_pad = (nsum + 1) / 2 * 2;     // the points are read as pairs
+  const size_t nparts = nfar + nnear + nself;
+  if ((st = ensure_scratch(g, sizeof(double) * (nsum_pad + nparts + npts + next)))) return st;
+  double *sums = g->d_scratch, *part = sums + nsum_pad, *pext = part + nparts + npts;
+  double *sext = sums + (size_t)NP2 + (size_t)NO * NPQ + NO;
+  BG_CUDA_TRY(cudaMemsetAsync(sums, 0, sizeof(double) * nsum, stream()));
+  EmtReduce R{};
+  if (tets) {
+    if ((st = emt_tet_sums(g, P, part, sums, R, bm, far_blocks, near_blocks, near_per, self_blocks))) return st;
+  } else {
+    k_pft_far<<<dim3(nb, nb), dim3(FT, FT), 0, stream()>>>(P, part);
     BG_LAUNCHED();
+    emt_add_job(R, part, (long long)nb * nb, NP2, sums);
+    if (g->near.npairs > 0) {
+      k_pft_near<<<near_blocks, 256, 0, stream()>>>(P, g->near, part + nfar);
+      BG_LAUNCHED();
+      emt_add_job(R, part + nfar, near_blocks, NO * NPQ, sums + NP2);
+    }
   }
   if (E0) {
     PWave pw = make_pw(wr, wi, E0, nhat);
     k_pft_ext<<<nrow, 128, 0, stream()>>>(P, pw, pext);
     BG_LAUNCHED();
-  } else {
-    BG_CUDA_TRY(cudaMemsetAsync(pext, 0, sizeof(double) * next, stream()));
+    emt_add_job(R, pext, nrow, NO * NPQ, sext);
   }
-  std::vector<double> h(nfar + nnear + next);
-  BG_CUDA_TRY(cudaMemcpyAsync(h.data(), g->d_scratch, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream()));
+  if (R.n) {
+    k_emt_reduce<<<dim3(R.n, R.wmax), 256, 0, stream()>>>(R);
+    BG_LAUNCHED();
+  }
+  std::vector<double> h(nsum);
+  BG_CUDA_TRY(cudaMemcpyAsync(h.data(), sums, sizeof(double) * nsum, cudaMemcpyDeviceToHost, stream()));
   BG_CUDA_TRY(cudaStreamSynchronize(stream()));
-  // scat[noa][nob][n]: pair sums; ext[no][n]
-  std::vector<double> scat((size_t)NO * NO * NPQ, 0.0), ext((size_t)NO * NPQ, 0.0);
-  for (size_t blk = 0; blk < (size_t)nb * nb; blk++)
-    for (size_t e = 0; e < (size_t)NO * NO * NPQ; e++) scat[e] += h[blk * NO * NO * NPQ + e];
-  if (g->near.npairs > 0)
-    for (int blk = 0; blk < nnear_blocks; blk++)
-      for (int o = 0; o < NO; o++)
-        for (int n = 0; n < NPQ; n++) scat[((size_t)o * NO + o) * NPQ + n] += h[nfar + ((size_t)blk * NO + o) * NPQ + n];
-  for (int blk = 0; blk < nrow; blk++)
-    for (size_t e = 0; e < (size_t)NO * NPQ; e++) ext[e] += h[nfar + nnear + (size_t)blk * NO * NPQ + e];
+  const double *scat = h.data(), *near = scat + NP2, *self = near + NO * NPQ, *ext = self + NO;
   double ftf = 0.5 * TEN_THIRDS / wr;
   for (int o = 0; o < NO; o++) {
     double s[NPQ] = {0};
     for (int ob = 0; ob < NO; ob++)
       for (int n = 0; n < NPQ; n++) s[n] += scat[((size_t)o * NO + ob) * NPQ + n];
-    const double *e = ext.data() + (size_t)o * NPQ;
+    for (int n = 0; n < NPQ; n++) s[n] += near[o * NPQ + n];
+    s[0] += self[o];
+    const double *e = ext + (size_t)o * NPQ;
     double *r = out + 8 * o;
     r[0] = 0.5 * e[0] - s[0];
     r[1] = s[0];
