@@ -93,7 +93,7 @@ static int slot_init(bg_geometry *g, Slot &S, const double *E0, const double *nh
   BG_CUDA_TRY(cudaMalloc(&S.rhs, 16 * (size_t)N));
   BG_CUDA_TRY(cudaMalloc(&S.T, 16 * (size_t)N));
   BG_CUDA_TRY(cudaMalloc(&S.fq, 4 * sizeof(double)));
-  BG_CUDA_TRY(cudaMalloc(&S.part, sizeof(double) * (size_t)((N + 127) / 128) * NO));
+  BG_CUDA_TRY(cudaMalloc(&S.part, sizeof(double) * (size_t)pft_point_blocks(g) * NO));
   BG_CUDA_TRY(cudaMalloc(&S.out, sizeof(double) * BATCH_MAXOBJ));
   BG_CUDA_TRY(cudaMalloc(&S.status, 2 * sizeof(int)));
   BG_CUDA_TRY(cudaMemset(S.status, 0, 2 * sizeof(int)));

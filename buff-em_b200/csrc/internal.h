@@ -276,6 +276,8 @@ int assemble_gram(bg_geometry *g, double wr, double wi, void *M, size_t ld, cons
 int refresh_materials(bg_geometry *g, double wr, double wi);
 int rhs_planewave(bg_geometry *g, double wr, double wi, const double *E0, const double *nhat, void *out,
                   const double *fq = nullptr);
+// part: pft_point_blocks(g) rows of one double per object
+int pft_point_blocks(const bg_geometry *g);
 int opft_enqueue(bg_geometry *g, double wr, double wi, const void *dJ, const double *fq, double *part,
                  double *out_dev);
 int pft(bg_geometry *g, double wr, double wi, const void *dJ, const double *E0, const double *nhat, int method,

@@ -280,29 +280,43 @@ __device__ cd expr_eval(const DevExpr &e, int comp, const double *x) {
 
 // permittivity functor (SVTensor::Evaluate semantics, SVTensor.cc:306-373);
 // ex: the object's compiled program when m.kind == BG_MAT_EXPR
-__device__ void mat_eval(const bg_material &m, const DevExpr *ex, const double *x, cd E[3][3]) {
+__device__ __noinline__ void mat_eval_expr(const DevExpr *ex, const double *x, cd E[3][3]) {
+  // components not given keep the identity, off-diagonal pairs are
+  // averaged, yy and zz follow xx when only xx is given (SVTensor.cc:344-372)
   for (int i = 0; i < 3; i++)
-    for (int j = 0; j < 3; j++) E[i][j] = cmk(0, 0);
+    for (int j = 0; j < 3; j++)
+      E[i][j] = ex->len[3 * i + j] ? expr_eval(*ex, 3 * i + j, x) : cmk(i == j ? 1.0 : 0.0, 0.0);
+  for (int mu = 0; mu < 3; mu++) {
+    int nu = (mu + 1) % 3;
+    cd a = cscale(cadd(E[mu][nu], E[nu][mu]), 0.5);
+    E[mu][nu] = E[nu][mu] = a;
+  }
+  if (ex->len[0]) {
+    if (!ex->len[4]) E[1][1] = E[0][0];
+    if (!ex->len[8]) E[2][2] = E[0][0];
+  }
+}
+// the fixed functors inline: a kernel calls out for compiled programs only
+__device__ __forceinline__ void mat_eval(const bg_material &m, const DevExpr *ex, const double *x, cd E[3][3]) {
   if (m.kind == BG_MAT_EXPR) {
-    // components not given keep the identity, off-diagonal pairs are
-    // averaged, yy and zz follow xx when only xx is given (SVTensor.cc:344-372)
+    cd T[3][3];
+    mat_eval_expr(ex, x, T);
+#pragma unroll
     for (int i = 0; i < 3; i++)
-      for (int j = 0; j < 3; j++)
-        E[i][j] = ex->len[3 * i + j] ? expr_eval(*ex, 3 * i + j, x) : cmk(i == j ? 1.0 : 0.0, 0.0);
-    for (int mu = 0; mu < 3; mu++) {
-      int nu = (mu + 1) % 3;
-      cd a = cscale(cadd(E[mu][nu], E[nu][mu]), 0.5);
-      E[mu][nu] = E[nu][mu] = a;
-    }
-    if (ex->len[0]) {
-      if (!ex->len[4]) E[1][1] = E[0][0];
-      if (!ex->len[8]) E[2][2] = E[0][0];
-    }
+#pragma unroll
+      for (int j = 0; j < 3; j++) E[i][j] = T[i][j];
     return;
   }
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) E[i][j] = cmk(0, 0);
   if (m.kind == BG_MAT_CONST_TENSOR) {
+#pragma unroll
     for (int i = 0; i < 3; i++)
+#pragma unroll
       for (int j = 0; j < 3; j++) E[i][j] = cmk(m.eps[2 * (3 * i + j)], m.eps[2 * (3 * i + j) + 1]);
+#pragma unroll
     for (int mu = 0; mu < 3; mu++) {
       int nu = (mu + 1) % 3;
       cd a = cscale(cadd(E[mu][nu], E[nu][mu]), 0.5);
@@ -323,7 +337,7 @@ __device__ void mat_eval(const bg_material &m, const DevExpr *ex, const double *
 }
 
 // Invert3x3Matrix, VIEMatrix.cc:51-72
-__device__ void inv3(cd M[3][3], cd W[3][3]) {
+__device__ __forceinline__ void inv3(cd M[3][3], cd W[3][3]) {
   cd M11 = M[0][0], M12 = M[0][1], M13 = M[0][2];
   cd M21 = M[1][0], M22 = M[1][1], M23 = M[1][2];
   cd M31 = M[2][0], M32 = M[2][1], M33 = M[2][2];
@@ -757,52 +771,58 @@ __global__ void k_near(DevGeom g, NearData nd, cd k, cd invk2, cd *M, size_t ld,
     k = cd{fq[0], fq[1]};
     invk2 = dev_invk2(fq[0], fq[1]);
   }
-  int kk = blockIdx.x * blockDim.x + threadIdx.x;
-  if (kk >= nd.npairs) return;
-  int2 ab = nd.pairs[kk];
-  int a = ab.x, b = ab.y;
-  int2 ta = g.bfTet[a], tb = g.bfTet[b], qa = g.bfQ[a], qb = g.bfQ[b];
-  double Aa = g.bfArea[a], Ab = g.bfArea[b];
+  // four lanes per pair, one per tetrahedron pair (PP, PM, MP, MM); the sum
+  // keeps that order (88 -> 26 us at N = 72, where 2,600 threads did not fill
+  // the SMs; 398 -> 375 us at N = 4,494)
+  const int id = blockIdx.x * blockDim.x + threadIdx.x, kk = id >> 2;
+  const bool live = kk < nd.npairs;
+  const int2 ab = nd.pairs[live ? kk : 0];
+  const int a = ab.x, b = ab.y, sa = (id >> 1) & 1, sb = id & 1;
+  const int2 ta = g.bfTet[a], tb = g.bfTet[b], qa = g.bfQ[a], qb = g.bfQ[b];
+  const double Aa = g.bfArea[a], Ab = g.bfArea[b];
   const double inv4pi = 0.25 / M_PI;
-  cd ik = cmk(-k.i, k.r);
-  cd acc = cmk(0, 0);
-  for (int sa = 0; sa < 2; sa++) {
-    int t1 = sa == 0 ? ta.x : ta.y;
-    double Q[3];
+  const cd ik = cmk(-k.i, k.r);
+  cd part = cmk(0, 0);
+  if (live) {
+    const int t1 = sa == 0 ? ta.x : ta.y, t2 = sb == 0 ? tb.x : tb.y;
+    double Q[3], QP[3];
     load3(g.V4, sa == 0 ? qa.x : qa.y, Q);
-    for (int sb = 0; sb < 2; sb++) {
-      int t2 = sb == 0 ? tb.x : tb.y;
-      double QP[3];
-      load3(g.V4, sb == 0 ? qb.x : qb.y, QP);
-      double cc = (sa == 0 ? 1.0 : -1.0) * (sb == 0 ? 1.0 : -1.0) * Aa * Ab;
-      cd part = cmk(0, 0);
-      for (int i = 0; i < 4; i++) {
-        const double *x = g.tetP4 + 16 * (size_t)t1 + 4 * i;
-        for (int j = 0; j < 4; j++) {
-          const double *y = g.tetP4 + 16 * (size_t)t2 + 4 * j;
-          double R0 = x[0] - y[0], R1 = x[1] - y[1], R2 = x[2] - y[2];
-          double r = sqrt(R0 * R0 + R1 * R1 + R2 * R2);
-          if (r < 1.0e-12) continue;
-          double dot = (x[0] - Q[0]) * (y[0] - QP[0]) + (x[1] - Q[1]) * (y[1] - QP[1]) + (x[2] - Q[2]) * (y[2] - QP[2]);
-          cd phi = cscale(exprel3(cscale(ik, r)), inv4pi / r);
-          cd pe = cmk(dot * (1.0 / 144.0) - invk2.r * (1.0 / 16.0), -invk2.i * (1.0 / 16.0));
-          part = cadd(part, cmul(pe, phi));
-        }
+    load3(g.V4, sb == 0 ? qb.x : qb.y, QP);
+    const double cc = (sa == sb ? 1.0 : -1.0) * Aa * Ab;
+    for (int i = 0; i < 4; i++) {
+      const double *x = g.tetP4 + 16 * (size_t)t1 + 4 * i;
+      for (int j = 0; j < 4; j++) {
+        const double *y = g.tetP4 + 16 * (size_t)t2 + 4 * j;
+        double R0 = x[0] - y[0], R1 = x[1] - y[1], R2 = x[2] - y[2];
+        double r = sqrt(R0 * R0 + R1 * R1 + R2 * R2);
+        if (r < 1.0e-12) continue;
+        double dot = (x[0] - Q[0]) * (y[0] - QP[0]) + (x[1] - Q[1]) * (y[1] - QP[1]) + (x[2] - Q[2]) * (y[2] - QP[2]);
+        cd phi = cscale(exprel3(cscale(ik, r)), inv4pi / r);
+        cd pe = cmk(dot * (1.0 / 144.0) - invk2.r * (1.0 / 16.0), -invk2.i * (1.0 / 16.0));
+        part = cadd(part, cmul(pe, phi));
       }
-      acc = cadd(acc, cscale(part, cc));
     }
+    part = cscale(part, cc);
   }
+  const int l0 = threadIdx.x & 28;
+  cd acc = cmk(0, 0);
+#pragma unroll
+  for (int q = 0; q < 4; q++)
+    acc = cadd(acc, cmk(__shfl_sync(0xffffffffu, part.r, l0 + q), __shfl_sync(0xffffffffu, part.i, l0 + q)));
+  if (!live) return;
   const double *F = nd.fibbi + 6 * (size_t)kk;
   cd t0 = cadd(cmk(F[0], 0), cscale(invk2, -F[1]));
   cd t1 = cmul(ik, cadd(cmk(F[2], 0), cscale(invk2, -F[3])));
   cd t2 = cmul(cmul(ik, ik), cadd(cmk(F[4], 0), cscale(invk2, -F[5])));
   acc = cadd(acc, cadd(t0, cadd(t1, t2)));
-  M[(size_t)a + (size_t)b * ld] = acc;
-  if (a != b) M[(size_t)b + (size_t)a * ld] = acc;
-  if (Fc) {   // the complex64 copy
+  // the four lanes write the entry, its mirror and their complex64 copies
+  const int w = id & 3;
+  if (w == 0) M[(size_t)a + (size_t)b * ld] = acc;
+  if (w == 1 && a != b) M[(size_t)b + (size_t)a * ld] = acc;
+  if (Fc) {
     const float2 f = make_float2((float)acc.r, (float)acc.i);
-    Fc[(size_t)a + (size_t)b * ldf] = f;
-    if (a != b) Fc[(size_t)b + (size_t)a * ldf] = f;
+    if (w == 2) Fc[(size_t)a + (size_t)b * ldf] = f;
+    if (w == 3 && a != b) Fc[(size_t)b + (size_t)a * ldf] = f;
   }
 }
 
@@ -811,7 +831,7 @@ int assemble_near(bg_geometry *g, double wr, double wi, void *M, size_t ld, cons
   if (nd.npairs == 0) return BG_OK;
   double d = (wr * wr - wi * wi) * (wr * wr - wi * wi) + 4 * wr * wr * wi * wi;
   cd invk2{(wr * wr - wi * wi) / d, -2 * wr * wi / d};
-  k_near<<<(nd.npairs + 127) / 128, 128, 0, stream()>>>(g->dev, nd, cd{wr, wi}, invk2, (cd *)M, ld, fq,
+  k_near<<<(int)((4LL * nd.npairs + 127) / 128), 128, 0, stream()>>>(g->dev, nd, cd{wr, wi}, invk2, (cd *)M, ld, fq,
                                                        (float2 *)F, ldf);
   BG_LAUNCHED();
   return BG_OK;
@@ -824,82 +844,89 @@ int assemble_near(bg_geometry *g, double wr, double wi, void *M, size_t ld, cons
 // Added to M(a,b) and M(b,a) for b >= a (the reference adds the full row and
 // its symmetric fill then overwrites the lower triangle with the upper).
 // =========================================================================
-__global__ void k_gram(DevGeom g, double w, cd *M, size_t ld, const double *fq, float2 *F, size_t ldf) {
+//
+// A half warp per tetrahedron of the row (lanes 0-15 the plus side, 16-31 the
+// minus side), its lanes over the 33 points: eps(x) and its 3 x 3 inverse are
+// formed once per point and serve the four faces, and the four sums come out
+// of a 16-lane shuffle tree.  One thread per row walked 2 x 4 x 33 points in
+// series, inverse included: 0.58-0.66 ms whatever N; now 20 us at N = 72 and
+// 50 us at N = 4,494.
+__global__ void __launch_bounds__(128) k_gram(DevGeom g, double w, cd *M, size_t ld, const double *fq, float2 *F,
+                                              size_t ldf) {
   if (fq) w = fq[0];
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (a >= g.N) return;
-  int2 tt = g.bfTet[a], qq = g.bfQ[a];
-  double Aa = g.bfArea[a];
-  int nnz = 1;
-  int idx[8];
-  cd val[8];
-  idx[0] = a;
-  val[0] = cmk(0, 0);
+  const int side = lane >> 4, l = lane & 15;
+  const int2 tt = g.bfTet[a], qq = g.bfQ[a];
   const double pre = -1.0 / (w * w);
-  for (int side = 0; side < 2; side++) {
-    int t = side == 0 ? tt.x : tt.y;
-    int obj = g.tetObj[t];
-    const bg_material &mat = g.mats[obj];
-    const DevExpr *mex = g.expr ? g.expr + obj : nullptr;
-    double vol = g.tetVol[t];
-    double QA[3];
-    load3(g.V4, side == 0 ? qq.x : qq.y, QA);
-    double pa = (side == 0 ? 1.0 : -1.0) * Aa / (3.0 * vol);
-    int4 vi = g.tetVI[t];
-    double V0[3], L[3][3];
-    load3(g.V4, vi.x, V0);
-    int vv[3] = {vi.y, vi.z, vi.w};
-    for (int i = 0; i < 3; i++) {
-      double tmp[3];
-      load3(g.V4, vv[i], tmp);
-      for (int c = 0; c < 3; c++) L[i][c] = tmp[c] - V0[c];
-    }
-    int4 fi = g.tetFI[t];
-    int fl[4] = {fi.x, fi.y, fi.z, fi.w};
-    for (int ifb = 0; ifb < 4; ifb++) {
-      int b = fl[ifb];
-      if (b < 0) continue;
-      int2 tb = g.bfTet[b], qb = g.bfQ[b];
-      double QB[3], pb;
-      if (tb.x == t) { load3(g.V4, qb.x, QB); pb = g.bfArea[b] / (3.0 * vol); }
-      else { load3(g.V4, qb.y, QB); pb = -g.bfArea[b] / (3.0 * vol); }
-      cd accv = cmk(0, 0);
-      for (int i = 0; i < 33; i++) {
-        const double *u = c_tcr33 + 4 * i;
-        double wt = 6.0 * vol * u[3], x[3];
-        for (int c = 0; c < 3; c++) x[c] = V0[c] + u[0] * L[0][c] + u[1] * L[1][c] + u[2] * L[2][c];
-        cd E[3][3], Ei[3][3];
-        mat_eval(mat, mex, x, E);
-        E[0][0].r -= 1.0; E[1][1].r -= 1.0; E[2][2].r -= 1.0;
-        inv3(E, Ei);
-        double FA[3], FB[3];
-        for (int c = 0; c < 3; c++) { FA[c] = pa * (x[c] - QA[c]); FB[c] = pb * (x[c] - QB[c]); }
-        cd v = cmk(0, 0);
-        for (int mu = 0; mu < 3; mu++)
-          for (int nu = 0; nu < 3; nu++) v = cadd(v, cscale(Ei[mu][nu], FA[mu] * FB[nu]));
-        accv = cadd(accv, cscale(v, pre * wt));
-      }
-      if (b == a) val[0] = cadd(val[0], accv);
-      else { idx[nnz] = b; val[nnz] = accv; nnz++; }
-    }
+  const int t = side == 0 ? tt.x : tt.y;
+  const int obj = g.tetObj[t];
+  const bg_material &mat = g.mats[obj];
+  const DevExpr *mex = g.expr ? g.expr + obj : nullptr;
+  const double vol = g.tetVol[t];
+  const double pa = (side == 0 ? 1.0 : -1.0) * g.bfArea[a] / (3.0 * vol);
+  double QA[3], V[4][3];
+  load3(g.V4, side == 0 ? qq.x : qq.y, QA);
+  const int4 vi = g.tetVI[t], fi = g.tetFI[t];
+  const int vv[4] = {vi.x, vi.y, vi.z, vi.w}, fl[4] = {fi.x, fi.y, fi.z, fi.w};
+  double pb[4];
+#pragma unroll
+  for (int f = 0; f < 4; f++) {
+    load3(g.V4, vv[f], V[f]);     // the vertex opposite face f is its Q
+    pb[f] = fl[f] < 0 ? 0.0 : (g.bfTet[fl[f]].x == t ? 1.0 : -1.0) * g.bfArea[fl[f]] / (3.0 * vol);
   }
-  for (int i = 0; i < nnz; i++) {
-    int b = idx[i];
-    if (b < a) continue;
-    cd *p = M + (size_t)a + (size_t)b * ld;
-    const cd v = cadd(*p, val[i]);
-    *p = v;
-    if (b != a) {
-      cd *q = M + (size_t)b + (size_t)a * ld;
-      *q = cadd(*q, val[i]);
+  cd acc[4] = {cmk(0, 0), cmk(0, 0), cmk(0, 0), cmk(0, 0)};
+  for (int i = l; i < 33; i += 16) {
+    const double *u = c_tcr33 + 4 * i;
+    const double wt = pre * (6.0 * vol * u[3]);
+    double x[3], FA[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      x[c] = V[0][c] + u[0] * (V[1][c] - V[0][c]) + u[1] * (V[2][c] - V[0][c]) + u[2] * (V[3][c] - V[0][c]);
+      FA[c] = pa * (x[c] - QA[c]);
     }
-    if (F) {   // the final value of these entries: the complex64 copy
-      F[(size_t)a + (size_t)b * ldf] = make_float2((float)v.r, (float)v.i);
-      if (b != a) {
-        const cd *q = M + (size_t)b + (size_t)a * ld;
-        F[(size_t)b + (size_t)a * ldf] = make_float2((float)q->r, (float)q->i);
-      }
+    cd E[3][3], Ei[3][3], r[3];
+    mat_eval(mat, mex, x, E);
+    E[0][0].r -= 1.0; E[1][1].r -= 1.0; E[2][2].r -= 1.0;
+    inv3(E, Ei);
+#pragma unroll
+    for (int nu = 0; nu < 3; nu++)
+      r[nu] = cscale(cadd(cadd(cscale(Ei[0][nu], FA[0]), cscale(Ei[1][nu], FA[1])), cscale(Ei[2][nu], FA[2])), wt);
+#pragma unroll
+    for (int f = 0; f < 4; f++)
+#pragma unroll
+      for (int nu = 0; nu < 3; nu++) acc[f] = cadd(acc[f], cscale(r[nu], pb[f] * (x[nu] - V[f][nu])));
+  }
+#pragma unroll
+  for (int f = 0; f < 4; f++)
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      acc[f].r += __shfl_xor_sync(0xffffffffu, acc[f].r, o);
+      acc[f].i += __shfl_xor_sync(0xffffffffu, acc[f].i, o);
     }
+  // the diagonal sums both sides; every other face belongs to one side
+  cd diag = cmk(0, 0);
+#pragma unroll
+  for (int f = 0; f < 4; f++)
+    if (fl[f] == a) diag = acc[f];
+  const cd other = cmk(__shfl_xor_sync(0xffffffffu, diag.r, 16), __shfl_xor_sync(0xffffffffu, diag.i, 16));
+  if (l >= 4) return;
+  const int b = l == 0 ? fl[0] : l == 1 ? fl[1] : l == 2 ? fl[2] : fl[3];
+  cd val = l == 0 ? acc[0] : l == 1 ? acc[1] : l == 2 ? acc[2] : acc[3];
+  if (b < a || (b == a && side == 1)) return;   // also faces of the surface, b = -1
+  if (b == a) val = cadd(diag, other);
+  cd *p = M + (size_t)a + (size_t)b * ld;
+  const cd v = cadd(*p, val);
+  *p = v;
+  cd vt = v;
+  if (b != a) {
+    cd *q = M + (size_t)b + (size_t)a * ld;
+    vt = cadd(*q, val);
+    *q = vt;
+  }
+  if (F) {   // the final value of these entries: the complex64 copy
+    F[(size_t)a + (size_t)b * ldf] = make_float2((float)v.r, (float)v.i);
+    if (b != a) F[(size_t)b + (size_t)a * ldf] = make_float2((float)vt.r, (float)vt.i);
   }
 }
 
@@ -907,7 +934,7 @@ int assemble_gram(bg_geometry *g, double wr, double wi, void *M, size_t ld, cons
   if (g->dispersive && fq) { set_error("frequency-dependent materials need a host frequency"); return BG_ERR_ARG; }
   int st = refresh_materials(g, wr, wi);
   if (st) return st;
-  k_gram<<<(g->N + 127) / 128, 128, 0, stream()>>>(g->dev, wr, (cd *)M, ld, fq, (float2 *)F, ldf);
+  k_gram<<<(g->N + 3) / 4, 128, 0, stream()>>>(g->dev, wr, (cd *)M, ld, fq, (float2 *)F, ldf);
   BG_LAUNCHED();
   return BG_OK;
 }
@@ -918,42 +945,8 @@ int assemble_gram(bg_geometry *g, double wr, double wi, void *M, size_t ld, cons
 // =========================================================================
 struct PWave { cd E0[3]; double nh[3]; cd k; };
 
-__device__ __forceinline__ cd bf_dot_field(const DevGeom &g, int a, const PWave &pw) {
-  int2 tt = g.bfTet[a], loc = g.bfLoc[a];
-  double Aa = g.bfArea[a];
-  cd tot = cmk(0, 0);
-  for (int side = 0; side < 2; side++) {
-    int t = side == 0 ? tt.x : tt.y, iq = side == 0 ? loc.x : loc.y;
-    int4 vi = g.tetVI[t];
-    int v[4] = {vi.x, vi.y, vi.z, vi.w};
-    double Q[3], L[3][3];
-    load3(g.V4, v[iq], Q);
-    for (int i = 0; i < 3; i++) {
-      double tmp[3];
-      load3(g.V4, v[(iq + 1 + i) % 4], tmp);
-      for (int c = 0; c < 3; c++) L[i][c] = tmp[c] - Q[c];
-    }
-    double vol = g.tetVol[t];
-    double pf = (side == 0 ? 1.0 : -1.0) * Aa / (3.0 * vol);
-    cd acc = cmk(0, 0);
-    for (int i = 0; i < 33; i++) {
-      const double *u = c_tcr33 + 4 * i;
-      double wt = 6.0 * vol * u[3], x[3], b[3];
-      for (int c = 0; c < 3; c++) {
-        b[c] = u[0] * L[0][c] + u[1] * L[1][c] + u[2] * L[2][c];
-        x[c] = Q[c] + b[c];
-        b[c] *= pf;
-      }
-      double ph = pw.nh[0] * x[0] + pw.nh[1] * x[1] + pw.nh[2] * x[2];
-      cd e = expikr(pw.k, ph);
-      cd be = cadd(cadd(cscale(pw.E0[0], b[0]), cscale(pw.E0[1], b[1])), cscale(pw.E0[2], b[2]));
-      acc = cadd(acc, cscale(cmul(be, e), wt));
-    }
-    tot = cadd(tot, acc);
-  }
-  return tot;
-}
-
+// 16 lanes per basis function, over the 2 x 33 points (one thread per basis
+// function evaluated them in series: 19-24 us; now 8-11 us)
 __global__ void k_rhs(DevGeom g, PWave pw, cd pre, cd *out, const double *fq) {
   if (fq) {
     // -1/(i w Z0) = i/(w Z0)
@@ -961,9 +954,39 @@ __global__ void k_rhs(DevGeom g, PWave pw, cd pre, cd *out, const double *fq) {
     pw.k = cd{wr, wi};
     pre = cd{wi / d, wr / d};
   }
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= g.N) return;
-  out[a] = cmul(pre, bf_dot_field(g, a, pw));
+  const int a = (blockIdx.x * blockDim.x + threadIdx.x) >> 4, l = threadIdx.x & 15;
+  const bool live = a < g.N;
+  cd tot = cmk(0, 0);
+  if (live) {
+    const int2 tt = g.bfTet[a], qq = g.bfQ[a];
+    const double Aa = g.bfArea[a];
+#pragma unroll 1
+    for (int side = 0; side < 2; side++) {
+      const int t = side == 0 ? tt.x : tt.y;
+      const int4 vi = g.tetVI[t];
+      double Q[3], V[4][3];
+      load3(g.V4, side == 0 ? qq.x : qq.y, Q);
+      load3(g.V4, vi.x, V[0]); load3(g.V4, vi.y, V[1]); load3(g.V4, vi.z, V[2]); load3(g.V4, vi.w, V[3]);
+      const double vol = g.tetVol[t], pf = (side == 0 ? 1.0 : -1.0) * Aa / (3.0 * vol);
+      for (int i = l; i < 33; i += 16) {
+        const double *u = c_tcr33 + 4 * i;
+        const double wt = 6.0 * vol * u[3] * pf;
+        double x[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+          x[c] = V[0][c] + u[0] * (V[1][c] - V[0][c]) + u[1] * (V[2][c] - V[0][c]) + u[2] * (V[3][c] - V[0][c]);
+        const cd e = expikr(pw.k, pw.nh[0] * x[0] + pw.nh[1] * x[1] + pw.nh[2] * x[2]);
+        const cd be = cadd(cadd(cscale(pw.E0[0], x[0] - Q[0]), cscale(pw.E0[1], x[1] - Q[1])), cscale(pw.E0[2], x[2] - Q[2]));
+        tot = cadd(tot, cscale(cmul(be, e), wt));
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) {
+    tot.r += __shfl_xor_sync(0xffffffffu, tot.r, o);
+    tot.i += __shfl_xor_sync(0xffffffffu, tot.i, o);
+  }
+  if (live && l == 0) out[a] = cmul(pre, tot);
 }
 
 static PWave make_pw(double wr, double wi, const double *E0, const double *nhat) {
@@ -982,7 +1005,7 @@ int rhs_planewave(bg_geometry *g, double wr, double wi, const double *E0, const 
   const double Z0 = 376.73031346177;
   double d = (wr * wr + wi * wi) * Z0;
   cd pre{wi / d, wr / d};
-  k_rhs<<<(g->N + 127) / 128, 128, 0, stream()>>>(g->dev, pw, pre, (cd *)out, fq);
+  k_rhs<<<(g->N + 7) / 8, 128, 0, stream()>>>(g->dev, pw, pre, (cd *)out, fq);
   BG_LAUNCHED();
   return BG_OK;
 }
@@ -1208,63 +1231,64 @@ __global__ void k_pft_near(PftArgs P, NearData nd, double *part) {
   }
 }
 
-// extinction (EMTPFT.cc:85-127, 151-211) for a plane wave (grad E = ik nhat E):
-// per basis function q0 = int b.E, qx = int (x - c) b.E, t1 = int b x E;
-// e[0] = Re(J* q0), e[1+i] = Im(J* ik nhat_i q0), e[4+i] = Im(J* t1_i),
-// e[7+i] = Im(J* ik (qx x nhat)_i); partial sums per block and object
-__global__ void k_pft_ext(PftArgs P, PWave pw, double *part) {
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
+// total current sum J_a b_a(x) of tetrahedron t (its up to four basis functions)
+__device__ __forceinline__ void tet_current(const DevGeom &g, const cd *J, int t, const double (*V)[3],
+                                            const double *x, cd j[3]) {
+  const int4 fi = g.tetFI[t];
+  const int f[4] = {fi.x, fi.y, fi.z, fi.w};
+  const double iv = 1.0 / (3.0 * g.tetVol[t]);
+  j[0] = j[1] = j[2] = cmk(0, 0);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const int a = f[q];
+    if (a < 0) continue;
+    const cd Ja = cscale(J[a], (g.bfTet[a].x == t ? 1.0 : -1.0) * g.bfArea[a] * iv);
+#pragma unroll
+    for (int c = 0; c < 3; c++) j[c] = cadd(j[c], cscale(Ja, x[c] - V[q][c]));
+  }
+}
+__device__ __forceinline__ void tet_point33(const DevGeom &g, int t, int i, double (*V)[3], double *x, double &wt) {
+  const int4 vi = g.tetVI[t];
+  load3(g.V4, vi.x, V[0]); load3(g.V4, vi.y, V[1]); load3(g.V4, vi.z, V[2]); load3(g.V4, vi.w, V[3]);
+  const double *u = c_tcr33 + 4 * i;
+#pragma unroll
+  for (int c = 0; c < 3; c++)
+    x[c] = V[0][c] + u[0] * (V[1][c] - V[0][c]) + u[1] * (V[2][c] - V[0][c]) + u[2] * (V[3][c] - V[0][c]);
+  wt = 6.0 * g.tetVol[t] * u[3];
+}
+
+// extinction (EMTPFT.cc:85-127, 151-211) for a plane wave (grad E = ik nhat E).
+// Linear in conj(J_a), so one thread per point of the 33-point rule takes the
+// tetrahedron's total current j: with be = conj(j).E and xt = x - c
+// (torque centre), e[0] = Re be, e[1+i] = Im(ik nhat_i be),
+// e[4+i] = Im(conj(j) x E)_i, e[7+i] = Im(ik be (xt x nhat)_i); partial sums
+// per block and object.  33 NT independent threads in place of N threads of
+// 66 points each (24-28 us at N = 72 and 4,494; now 6-10 us).
+__global__ void __launch_bounds__(128) k_pft_ext(PftArgs P, PWave pw, double *part) {
+  const DevGeom &g = P.g;
+  const int id = blockIdx.x * blockDim.x + threadIdx.x, t = id / 33;
   double e[NPQ];
   for (int n = 0; n < NPQ; n++) e[n] = 0.0;
   int obj = 0;
-  if (a < P.g.N) {
-    const DevGeom &g = P.g;
-    obj = g.bfV[a].w;
+  if (t < g.NT) {
+    obj = g.tetObj[t];
     const double *tc = g.objOrigin + 3 * obj;
-    int2 tt = g.bfTet[a], loc = g.bfLoc[a];
-    double Aa = g.bfArea[a];
-    cd q0 = cmk(0, 0), qx[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)}, t1[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)};
-    for (int side = 0; side < 2; side++) {
-      int t = side == 0 ? tt.x : tt.y, iq = side == 0 ? loc.x : loc.y;
-      int4 vi = g.tetVI[t];
-      int v[4] = {vi.x, vi.y, vi.z, vi.w};
-      double Q[3], L[3][3];
-      load3(g.V4, v[iq], Q);
-      for (int i = 0; i < 3; i++) {
-        double tmp[3];
-        load3(g.V4, v[(iq + 1 + i) % 4], tmp);
-        for (int c = 0; c < 3; c++) L[i][c] = tmp[c] - Q[c];
-      }
-      double vol = g.tetVol[t];
-      double pf = (side == 0 ? 1.0 : -1.0) * Aa / (3.0 * vol);
-      for (int i = 0; i < 33; i++) {
-        const double *u = c_tcr33 + 4 * i;
-        double wt = 6.0 * vol * u[3], x[3], bv[3];
-        for (int c = 0; c < 3; c++) {
-          bv[c] = u[0] * L[0][c] + u[1] * L[1][c] + u[2] * L[2][c];
-          x[c] = Q[c] + bv[c];
-          bv[c] *= pf;
-        }
-        cd ph = expikr(pw.k, pw.nh[0] * x[0] + pw.nh[1] * x[1] + pw.nh[2] * x[2]);
-        cd E[3];
-        for (int c = 0; c < 3; c++) E[c] = cscale(cmul(pw.E0[c], ph), wt);
-        cd be = cadd(cadd(cscale(E[0], bv[0]), cscale(E[1], bv[1])), cscale(E[2], bv[2]));
-        q0 = cadd(q0, be);
-        for (int c = 0; c < 3; c++) qx[c] = cadd(qx[c], cscale(be, x[c] - tc[c]));
-        t1[0] = cadd(t1[0], csub(cscale(E[2], bv[1]), cscale(E[1], bv[2])));
-        t1[1] = cadd(t1[1], csub(cscale(E[0], bv[2]), cscale(E[2], bv[0])));
-        t1[2] = cadd(t1[2], csub(cscale(E[1], bv[0]), cscale(E[0], bv[1])));
-      }
-    }
-    cd Jc = cmk(P.J[a].r, -P.J[a].i);
-    cd ik = cmk(-pw.k.i, pw.k.r);
-    e[0] = cmul(Jc, q0).r;
+    double V[4][3], x[3], wt;
+    tet_point33(g, t, id - 33 * t, V, x, wt);
+    cd j[3], E[3];
+    tet_current(g, P.J, t, V, x, j);
+    const cd ph = cscale(expikr(pw.k, pw.nh[0] * x[0] + pw.nh[1] * x[1] + pw.nh[2] * x[2]), wt);
+#pragma unroll
+    for (int c = 0; c < 3; c++) { E[c] = cmul(pw.E0[c], ph); j[c].i = -j[c].i; }
+    const cd be = cadd(cadd(cmul(j[0], E[0]), cmul(j[1], E[1])), cmul(j[2], E[2]));
+    const cd ikbe = cmul(cmk(-pw.k.i, pw.k.r), be);
+    e[0] = be.r;
+#pragma unroll
     for (int i = 0; i < 3; i++) {
-      int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
-      e[1 + i] = cmul(Jc, cscale(cmul(ik, q0), pw.nh[i])).i;
-      e[4 + i] = cmul(Jc, t1[i]).i;
-      cd qxn = csub(cscale(qx[i1], pw.nh[i2]), cscale(qx[i2], pw.nh[i1]));
-      e[7 + i] = cmul(Jc, cmul(ik, qxn)).i;
+      const int i1 = (i + 1) % 3, i2 = (i + 2) % 3;
+      e[1 + i] = ikbe.i * pw.nh[i];
+      e[4 + i] = csub(cmul(j[i1], E[i2]), cmul(j[i2], E[i1])).i;
+      e[7 + i] = ikbe.i * ((x[i1] - tc[i1]) * pw.nh[i2] - (x[i2] - tc[i2]) * pw.nh[i1]);
     }
   }
   __shared__ double red[4][PMAXOBJ][NPQ];
@@ -1283,78 +1307,36 @@ __global__ void k_pft_ext(PftArgs P, PWave pw, double *part) {
   }
 }
 
-#include "emt_pairs.cuh"
-
 // OPFT absorbed power (OPFT.cc:62-119, OverlapIntegrand_PFT PAbs term,
 // OverlapIntegrals.cc:79-170,242-298): sum Re(conj(Ja) Jb ME_ab),
 // ME_ab = 1/2 int b_a . (i Z0/w)(eps-1)^-1 . b_b on the shared tetrahedron.
-__global__ void k_opft(PftArgs P, cd omega, double *part, const double *fq) {
-  if (fq) {
-    omega = cd{fq[0], fq[1]};
-    P.w = fq[0];
-    P.absw = sqrt(fq[0] * fq[0] + fq[1] * fq[1]);
-  }
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
+// The sum over the faces of a tetrahedron is 1/2 int conj(j).(i Z0/w)
+// (eps-1)^-1.j of its total current, so one thread takes one of its 33 points
+// (one eps(x) and one inverse).  One thread per row walked 2 x 4 x 33 points
+// with an inverse each: 0.55-0.62 ms at any N; now 11 us at N = 72 and 20 us at 4,494.
+__global__ void __launch_bounds__(128) k_opft(PftArgs P, cd omega, double *part, const double *fq) {
+  if (fq) omega = cd{fq[0], fq[1]};
   const DevGeom &g = P.g;
+  const int id = blockIdx.x * blockDim.x + threadIdx.x, t = id / 33;
   double contrib = 0.0;
   int obj = 0;
-  if (a < g.N) {
-    obj = g.bfV[a].w;
-    const bg_material &mat = g.mats[obj];
-    const DevExpr *mex = g.expr ? g.expr + obj : nullptr;
-    int2 tt = g.bfTet[a], loc = g.bfLoc[a];
-    cd Ja = P.J[a];
-    const double Z0 = 376.73031346177;
-    cd pre = cdiv(cmk(0, Z0), omega);
-    for (int side = 0; side < 2; side++) {
-      int t = side == 0 ? tt.x : tt.y, iq = side == 0 ? loc.x : loc.y;
-      double vol = g.tetVol[t];
-      double pa = (side == 0 ? 1.0 : -1.0) * g.bfArea[a] / (3.0 * vol);
-      int4 vi = g.tetVI[t];
-      int v[4] = {vi.x, vi.y, vi.z, vi.w};
-      double QA[3], L[3][3];
-      load3(g.V4, v[iq], QA);
-      for (int i = 0; i < 3; i++) {
-        double tmp[3];
-        load3(g.V4, v[(iq + 1 + i) % 4], tmp);
-        for (int c = 0; c < 3; c++) L[i][c] = tmp[c] - QA[c];
-      }
-      int4 fi = g.tetFI[t];
-      int fl[4] = {fi.x, fi.y, fi.z, fi.w};
-      for (int ifb = 0; ifb < 4; ifb++) {
-        int b = fl[ifb];
-        if (b < 0) continue;
-        int2 tb = g.bfTet[b], qb = g.bfQ[b];
-        double QB[3], pb;
-        if (tb.x == t) { load3(g.V4, qb.x, QB); pb = g.bfArea[b] / (3.0 * vol); }
-        else { load3(g.V4, qb.y, QB); pb = -g.bfArea[b] / (3.0 * vol); }
-        cd me = cmk(0, 0);
-        for (int i = 0; i < 33; i++) {
-          const double *u = c_tcr33 + 4 * i;
-          double wt = 6.0 * vol * u[3], x[3], bA[3], bB[3];
-          for (int c = 0; c < 3; c++) {
-            bA[c] = u[0] * L[0][c] + u[1] * L[1][c] + u[2] * L[2][c];
-            x[c] = bA[c] + QA[c];
-            bB[c] = pb * (x[c] - QB[c]);
-            bA[c] *= pa;
-          }
-          cd E[3][3], Ei[3][3];
-          mat_eval(mat, mex, x, E);
-          E[0][0].r -= 1.0; E[1][1].r -= 1.0; E[2][2].r -= 1.0;
-          inv3(E, Ei);
-          cd vsum = cmk(0, 0);
-          for (int mu = 0; mu < 3; mu++) {
-            cd e = cmk(0, 0);
-            for (int nu = 0; nu < 3; nu++) e = cadd(e, cscale(cmul(pre, Ei[mu][nu]), bB[nu]));
-            vsum = cadd(vsum, cscale(e, 0.5 * bA[mu]));
-          }
-          me = cadd(me, cscale(vsum, wt));
-        }
-        cd Jb = P.J[b];
-        cd jj = cmk(Ja.r * Jb.r + Ja.i * Jb.i, Ja.r * Jb.i - Ja.i * Jb.r);
-        contrib += cmul(jj, me).r;
-      }
+  if (t < g.NT) {
+    obj = g.tetObj[t];
+    double V[4][3], x[3], wt;
+    tet_point33(g, t, id - 33 * t, V, x, wt);
+    cd j[3];
+    tet_current(g, P.J, t, V, x, j);
+    const cd pre = cscale(cdiv(cmk(0, 376.73031346177), omega), 0.5 * wt);
+    cd E[3][3], Ei[3][3], s = cmk(0, 0);
+    mat_eval(g.mats[obj], g.expr ? g.expr + obj : nullptr, x, E);
+    E[0][0].r -= 1.0; E[1][1].r -= 1.0; E[2][2].r -= 1.0;
+    inv3(E, Ei);
+#pragma unroll
+    for (int mu = 0; mu < 3; mu++) {
+      const cd r = cadd(cadd(cmul(Ei[mu][0], j[0]), cmul(Ei[mu][1], j[1])), cmul(Ei[mu][2], j[2]));
+      s = cadd(s, cmul(cmk(j[mu].r, -j[mu].i), r));
     }
+    contrib = cmul(pre, s).r;
   }
   __shared__ double red[4][PMAXOBJ];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1370,6 +1352,11 @@ __global__ void k_opft(PftArgs P, cd omega, double *part, const double *fq) {
   }
 }
 
+// blocks (and rows of partial sums) of k_opft and k_pft_ext
+int pft_point_blocks(const bg_geometry *g) { return (int)((33LL * g->NT + 127) / 128); }
+
+#include "emt_pairs.cuh"
+
 static int ensure_scratch(bg_geometry *g, size_t bytes) {
   if (g->scratch_bytes >= bytes) return BG_OK;
   if (g->d_scratch) cudaFree(g->d_scratch);
@@ -1380,26 +1367,37 @@ static int ensure_scratch(bg_geometry *g, size_t bytes) {
   return BG_OK;
 }
 
+__global__ void k_opft_reduce(int nrow, int nobj, const double *part, double *out) {
+  int o = blockIdx.x;
+  double s = 0;
+  for (int b = threadIdx.x; b < nrow; b += blockDim.x) s += part[(size_t)b * nobj + o];
+  s = warp_sum(s);
+  __shared__ double red[8];
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
+    out[o] = t;
+  }
+}
+
 int pft(bg_geometry *g, double wr, double wi, const void *dJ, const double *E0, const double *nhat, int method,
         double *out) {
   int st = init_tables();
   if (st) return st;
   int NO = (int)g->objs.size();
   if (NO > PMAXOBJ) { set_error("PFT supports at most %d objects", PMAXOBJ); return BG_ERR_ARG; }
-  PftArgs P{g->dev, (const cd *)dJ, wr, std::sqrt(wr * wr + wi * wi), NO};
-  int nrow = (g->N + 127) / 128;
   if (method == BG_PFT_OVERLAP) {
-    if ((st = ensure_scratch(g, sizeof(double) * nrow * NO))) return st;
     if ((st = refresh_materials(g, wr, wi))) return st;
-    k_opft<<<nrow, 128, 0, stream()>>>(P, cd{wr, wi}, g->d_scratch, nullptr);
-    BG_LAUNCHED();
-    std::vector<double> h((size_t)nrow * NO);
-    BG_CUDA_TRY(cudaMemcpyAsync(h.data(), g->d_scratch, sizeof(double) * h.size(), cudaMemcpyDeviceToHost, stream()));
+    const int nblk = pft_point_blocks(g);
+    if ((st = ensure_scratch(g, sizeof(double) * ((size_t)nblk + 1) * NO))) return st;
+    double *sum = g->d_scratch, h[PMAXOBJ];
+    if ((st = opft_enqueue(g, wr, wi, dJ, nullptr, sum + NO, sum))) return st;
+    BG_CUDA_TRY(cudaMemcpyAsync(h, sum, sizeof(double) * NO, cudaMemcpyDeviceToHost, stream()));
     BG_CUDA_TRY(cudaStreamSynchronize(stream()));
     for (int o = 0; o < NO; o++) {
-      double s = 0;
-      for (int b = 0; b < nrow; b++) s += h[(size_t)b * NO + o];
-      out[2 * o] = s;
+      out[2 * o] = h[o];
       out[2 * o + 1] = 0.0;
     }
     return BG_OK;
@@ -1508,7 +1506,7 @@ static int pft_emt_impl(bg_geometry *g, double wr, double wi, const void *dJ, co
   int NO = (int)g->objs.size();
   if (NO > PMAXOBJ) { set_error("PFT supports at most %d objects", PMAXOBJ); return BG_ERR_ARG; }
   PftArgs P{g->dev, (const cd *)dJ, wr, std::sqrt(wr * wr + wi * wi), NO, (const cd *)dDR, ldr};
-  int nrow = (g->N + 127) / 128;
+  const int nrow = pft_point_blocks(g);
   if ((st = build_near_lists(g))) return st;
   const bool tets = P.absw * g->bf_rmax <= 5.0;
   const int NP2 = NO * NO * NPQ;
@@ -1733,31 +1731,16 @@ int neq_overlaps(bg_geometry *g, double w, int *idx, double *S, void *V, double 
 // Absorbed power per object by the overlap method with every number kept on
 // the device (for captured graphs): partial sums into part (ceil(N/128) x NO
 // doubles), then out[o] = sum over blocks, o < NO.
-__global__ void k_opft_reduce(int nrow, int nobj, const double *part, double *out) {
-  int o = blockIdx.x;
-  double s = 0;
-  for (int b = threadIdx.x; b < nrow; b += blockDim.x) s += part[(size_t)b * nobj + o];
-  s = warp_sum(s);
-  __shared__ double red[8];
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-    out[o] = t;
-  }
-}
-
 int opft_enqueue(bg_geometry *g, double wr, double wi, const void *dJ, const double *fq, double *part,
                  double *out_dev) {
   if (g->dispersive && fq) { set_error("frequency-dependent materials need a host frequency"); return BG_ERR_ARG; }
   int NO = (int)g->objs.size();
   if (NO > PMAXOBJ) { set_error("PFT supports at most %d objects", PMAXOBJ); return BG_ERR_ARG; }
   PftArgs P{g->dev, (const cd *)dJ, wr, std::sqrt(wr * wr + wi * wi), NO};
-  int nrow = (g->N + 127) / 128;
-  k_opft<<<nrow, 128, 0, stream()>>>(P, cd{wr, wi}, part, fq);
+  const int nblk = pft_point_blocks(g);
+  k_opft<<<nblk, 128, 0, stream()>>>(P, cd{wr, wi}, part, fq);
   BG_LAUNCHED();
-  k_opft_reduce<<<NO, 256, 0, stream()>>>(nrow, NO, part, out_dev);
+  k_opft_reduce<<<NO, 256, 0, stream()>>>(nblk, NO, part, out_dev);
   BG_LAUNCHED();
   return BG_OK;
 }
