@@ -693,20 +693,282 @@ __global__ void __launch_bounds__(PCL_THREADS) k_panel_cl(PanelArgs<C> P) {
   cl.sync();   // no CTA leaves while another may still read its shared memory
 }
 
-// apply the interchanges ipiv[k0..k0+w) to columns [c0, c1) of A
+// -------------------------------------------------------------------------
+// The panel with its rows in registers, on one cluster.  A thread owns one row
+// of the panel; the active columns sit in its registers and move down by one
+// place per step (column j is always a[0]), so the rank-1 update reads and
+// writes registers only, and the finished columns go to shared memory
+// (Ls[c][row]), from where the whole slice is written out once.  The
+// shared-memory form above moves 32 bytes of shared memory per updated entry
+// and is bound by that and by its barriers: 3.3-3.9 us a column.
+//
+// One column costs two block barriers and one exchange.  Every warp finds its
+// pivot candidate with redux on the bits of |re| + |im| (non-negative, so they
+// order as integers) and the candidate's thread copies its row to shared
+// memory; after the barrier every warp knows the CTA's candidate, and warp q
+// pushes the candidate's row to CTAs q, q + warps, ... with st.async, which
+// counts its bytes on the receiver's mbarrier.  The CTA of rank 0, which owns
+// the rows k0 .. k0 + w - 1, pushes row k0 + j as well.  When its mbarrier
+// completes, a CTA has every candidate and both rows of the interchange in its
+// own shared memory: no remote loads, no cluster barrier.  Two buffers by
+// column parity: a CTA sends column j + 2 after it has received every
+// candidate of column j + 1, which each CTA sends only after all its warps
+// have finished with column j.  Waits are bounded; one that runs out is
+// reported through info, and the CTA goes on so that the cluster ends.
+//
+// Pivot choice (first index on ties), interchanges and arithmetic are those of
+// k_panel.  A NaN never wins; a column of NaNs takes its own row.
+// -------------------------------------------------------------------------
+#define PRF_MAXCL 16
+#define PRF_SPIN (1 << 17)
+template <class C> struct PrfCfg;
+template <> struct PrfCfg<cdl> { static constexpr int T = 256; };   // 32 columns = 128 registers a row
+template <> struct PrfCfg<cfl> { static constexpr int T = 512; };
+
 template <class C>
-__global__ void k_laswp(C *A, size_t ld, const int *ipiv, int k0, int w, int c0, int c1, int skip0, int skip1) {
-  int col = c0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (col >= c1 || (col >= skip0 && col < skip1)) return;
-  C *cp = A + (size_t)col * ld;
-  for (int i = 0; i < w; i++) {
-    int p = ipiv[k0 + i] - 1;
-    if (p != k0 + i) {
-      C t = cp[k0 + i];
-      cp[k0 + i] = cp[p];
-      cp[p] = t;
+struct PrfMsg {
+  C row[32];
+  unsigned long long key;
+  long long idx;
+};
+template <class C>
+struct PrfSmem {
+  PrfMsg<C> msg[2][PRF_MAXCL];
+  C jrow[2][32];                    // row k0 + j before the interchange
+  C wrow[2][PrfCfg<C>::T / 32][32]; // candidate rows of the warps (active part, wrow[c] = column j + c)
+  C myj[2][32];                     // rank 0: active part of row k0 + j
+  unsigned long long wkey[2][PrfCfg<C>::T / 32];
+  int widx[2][PrfCfg<C>::T / 32];
+  unsigned long long bar[2];
+};
+__device__ __forceinline__ unsigned long long pivot_key(cdl v) {
+  const double a = fabs(v.r) + fabs(v.i);
+  return a == a ? (unsigned long long)__double_as_longlong(a) : 0ull;
+}
+__device__ __forceinline__ unsigned long long pivot_key(cfl v) {
+  const float a = fabsf(v.r) + fabsf(v.i);
+  return a == a ? (unsigned long long)__float_as_uint(a) << 32 : 0ull;
+}
+// lane of the first maximum of key over the lanes with ok (-1: none); key of it
+template <class C>
+__device__ __forceinline__ int warp_first_max(unsigned long long &key, bool ok) {
+  const unsigned hi = ok ? (unsigned)(key >> 32) : 0u;
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  bool c = ok && hi == mh;
+  unsigned ml = 0;
+  if (sizeof(C) == 16) {
+    const unsigned lo = c ? (unsigned)key : 0u;
+    ml = __reduce_max_sync(0xffffffffu, lo);
+    c = c && lo == ml;
+  }
+  const unsigned b = __ballot_sync(0xffffffffu, c);
+  key = (unsigned long long)mh << 32 | ml;
+  return b ? __ffs(b) - 1 : -1;
+}
+__device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ unsigned map_cta(unsigned a, int rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_async16(unsigned dst, unsigned long long x, unsigned long long y, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+               "l"(x), "l"(y), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void st_async8(unsigned dst, unsigned long long x, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst), "l"(x), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void push_c(unsigned dst, cdl v, unsigned bar) {
+  st_async16(dst, (unsigned long long)__double_as_longlong(v.r), (unsigned long long)__double_as_longlong(v.i), bar);
+}
+__device__ __forceinline__ void push_c(unsigned dst, cfl v, unsigned bar) {
+  st_async8(dst, (unsigned long long)__float_as_uint(v.i) << 32 | __float_as_uint(v.r), bar);
+}
+
+template <class C>
+__global__ void __launch_bounds__(PrfCfg<C>::T) k_panel_rf(PanelArgs<C> P) {
+  typedef typename CxT<C>::R R;
+  constexpr int T = PrfCfg<C>::T, NW = T / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  PrfSmem<C> &S = *reinterpret_cast<PrfSmem<C> *>(smem_raw);
+  C *Ls = reinterpret_cast<C *>(smem_raw + sizeof(PrfSmem<C>));   // [w][T]
+  cg::cluster_group cl = cg::this_cluster();
+  const int w = P.w, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int rank = (int)cl.block_rank(), G = (int)cl.num_blocks();
+  const int r0 = P.k0 + rank * P.rows_per, nr = max(0, min(P.rows_per, P.Nr - r0));
+  const int row = r0 + tid;
+  const bool mine = tid < nr;
+  C a[32];
+#pragma unroll
+  for (int c = 0; c < 32; c++) a[c] = (mine && c < w) ? P.A[(size_t)(P.k0 + c) * P.ld + row] : C{0, 0};
+  const unsigned bar0 = smem_addr(&S.bar[0]);
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cl.sync();   // barriers of every CTA are ready
+  const unsigned bytes = (unsigned)(G * (32 * sizeof(C) + 16) + 32 * sizeof(C));
+  int limit = PRF_SPIN;
+  for (int j = 0; j < w; j++) {
+    const int gj = P.k0 + j, buf = j & 1;
+    const unsigned bar = bar0 + 8 * buf;
+    if (tid == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+    // 1. candidate of every warp; its row and rank 0's row gj to shared memory
+    {
+      unsigned long long key = pivot_key(a[0]);
+      const int src = warp_first_max<C>(key, mine && row >= gj);
+      if (lane == 0) {
+        S.wkey[buf][wid] = key;
+        S.widx[buf][wid] = src < 0 ? 0x7fffffff : r0 + wid * 32 + src;
+      }
+      if (lane == src)
+#pragma unroll
+        for (int c = 0; c < 32; c++) S.wrow[buf][wid][c] = a[c];
+      if (mine && row == gj)
+#pragma unroll
+        for (int c = 0; c < 32; c++) S.myj[buf][c] = a[c];
+    }
+    __syncthreads();
+    // 2. the CTA's candidate, pushed to every CTA (warp q: CTAs q, q + NW, ...)
+    {
+      unsigned long long key = lane < NW ? S.wkey[buf][lane] : 0ull;
+      const int idx = lane < NW ? S.widx[buf][lane] : 0x7fffffff;
+      const int bw = warp_first_max<C>(key, idx != 0x7fffffff);
+      const int bi = __shfl_sync(0xffffffffu, idx, bw < 0 ? 0 : bw);
+      C v = C{0, 0};
+      if (bw >= 0 && lane < w) v = lane < j ? Ls[lane * T + (bi - r0)] : S.wrow[buf][bw][lane - j];
+      C vj = C{0, 0};
+      if (rank == 0 && lane < w) vj = lane < j ? Ls[lane * T + j] : S.myj[buf][lane - j];
+      for (int q = wid; q < G; q += NW) {
+        const unsigned rb = map_cta(bar, q);
+        push_c(map_cta(smem_addr(&S.msg[buf][rank].row[lane]), q), v, rb);
+        if (lane == 0)
+          st_async16(map_cta(smem_addr(&S.msg[buf][rank].key), q), key, (unsigned long long)(bw < 0 ? -1ll : (long long)bi), rb);
+        if (rank == 0) push_c(map_cta(smem_addr(&S.jrow[buf][lane]), q), vj, rb);
+      }
+    }
+    // 3. everyone's candidates
+    {
+      unsigned done = 0;
+      for (int it = 0; it < limit && !done; it++)
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(bar), "r"((unsigned)((j >> 1) & 1))
+            : "memory");
+      if (!done) { limit = 1; atomicExch(P.info, 0x7fffffff); atomicExch(P.info + 1, 300); }
+    }
+    __syncthreads();   // every warp has read the rows it pushes (Ls changes below)
+    unsigned long long key = lane < G ? S.msg[buf][lane].key : 0ull;
+    const long long idx = lane < G ? S.msg[buf][lane].idx : -1;
+    int b = warp_first_max<C>(key, idx >= 0);
+    if (b < 0) b = 0;
+    const int piv = (int)__shfl_sync(0xffffffffu, (int)idx, b);
+    const C *prow = S.msg[buf][b].row;
+    if (rank == 0 && tid == 0) P.ipiv[gj] = piv + 1;
+    // 4. interchange: row gj's U part and L part are final and go to Ls (by
+    // the last warp of rank 0); the pivot's owner takes over the old row gj
+    if (rank == 0 && wid == NW - 1 && lane < w) Ls[lane * T + j] = prow[lane];
+    if (piv != gj && mine && row == piv) {
+#pragma unroll
+      for (int c = 0; c < 32; c++)
+        if (j + c < w) a[c] = S.jrow[buf][j + c];
+#pragma unroll 8
+      for (int c = 0; c < j; c++) Ls[c * T + tid] = S.jrow[buf][c];
+    }
+    // 5. scale and update; a[c] becomes column j + 1 + c
+    const C p = prow[j];
+    const R d = p.r * p.r + p.i * p.i;
+    const bool zero = d == (R)0;
+    if (zero && rank == 0 && tid == 0) atomicCAS(P.info, 0, gj + 1);
+    if (mine && row > gj) {
+      C l = a[0];
+      if (!zero) {
+        const C inv{p.r / d, -p.i / d};
+        l = C{a[0].r * inv.r - a[0].i * inv.i, a[0].r * inv.i + a[0].i * inv.r};
+      }
+      Ls[j * T + tid] = l;
+      if (zero) l = C{0, 0};
+      const int ncol = w - j - 1;
+#pragma unroll
+      for (int c0 = 0; c0 < 32; c0 += 8)
+        if (c0 < ncol)
+#pragma unroll
+          for (int c = c0; c < c0 + 8 && c < 31; c++) {
+            const C u = (c < ncol && !zero) ? prow[j + 1 + c] : C{0, 0};
+            a[c].r = a[c + 1].r - (l.r * u.r - l.i * u.i);
+            a[c].i = a[c + 1].i - (l.r * u.i + l.i * u.r);
+          }
     }
   }
+  __syncthreads();
+  // rows k0 .. k0 + w - 1 hold U (and the L of their interchanges), written
+  // to Ls by step 4; the others hold their L
+  if (mine)
+    for (int c = 0; c < w; c++) P.A[(size_t)(P.k0 + c) * P.ld + row] = Ls[c * T + tid];
+  cl.sync();   // no CTA leaves while messages for it may be in flight
+}
+
+// Row interchanges ipiv[k0..k0+w) on the columns [0, ncols) outside
+// [skip0, skip1), one warp per column.  The w interchanges are one
+// permutation of at most 2 w rows: the w top rows (lane l holds row k0 + l)
+// and the pivot rows below them (lane l holds the row that interchange l is
+// the first to name).  The source of each place is found once per block by
+// walking the w interchanges on row numbers; each lane then loads two
+// entries and stores two, independent of one another.  Walking the
+// interchanges on the data, one thread per column, was a chain of w dependent
+// round trips (27 us for scattered pivots at N = 4,092).
+#define LSW_WARPS 8
+template <class C>
+__global__ void __launch_bounds__(LSW_WARPS * 32) k_laswp(C *A, size_t ld, const int *ipiv, int k0, int w, int ncols,
+                                                           int skip0, int skip1) {
+  __shared__ int src[64], slot[32], rowof[64];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid < 32) {
+    const int p = lane < w ? ipiv[k0 + lane] - 1 : -1 - lane;
+    const unsigned same = __match_any_sync(0xffffffffu, p);
+    const bool below = p >= k0 + w;
+    slot[lane] = lane < w ? (below ? 32 + __ffs(same) - 1 : p - k0) : 0;
+    rowof[lane] = lane < w ? k0 + lane : -1;
+    rowof[32 + lane] = lane < w && below && __ffs(same) - 1 == lane ? p : -1;
+    src[lane] = lane;
+    src[32 + lane] = 32 + lane;
+    __syncwarp();
+    if (lane == 0)
+      for (int i = 0; i < w; i++) {
+        const int q = slot[i], x = src[i], y = src[q];
+        src[i] = y;
+        src[q] = x;
+      }
+  }
+  __syncthreads();
+  // place s takes the entry that was at place src[s]
+  const int d0 = rowof[lane], d1 = rowof[32 + lane];
+  const int s0 = d0 >= 0 ? rowof[src[lane]] : -1, s1 = d1 >= 0 ? rowof[src[32 + lane]] : -1;
+  const bool m0 = d0 >= 0 && s0 != d0, m1 = d1 >= 0 && s1 != d1;
+  for (int c = blockIdx.x * LSW_WARPS + (tid >> 5); c < ncols; c += gridDim.x * LSW_WARPS) {
+    if (c >= skip0 && c < skip1) continue;
+    C *cp = A + (size_t)c * ld;
+    const C v0 = m0 ? cp[s0] : C{0, 0}, v1 = m1 ? cp[s1] : C{0, 0};
+    __syncwarp();   // every load of the column before its stores
+    if (m0) cp[d0] = v0;
+    if (m1) cp[d1] = v1;
+  }
+}
+
+template <class C>
+static int laswp(bg_matrix *m, int k0, int w) {
+  const int blocks = std::min((m->N + LSW_WARPS - 1) / LSW_WARPS, 148 * 8);
+  prof_start(PROF_LASWP);
+  k_laswp<C><<<blocks, LSW_WARPS * 32, 0, stream()>>>((C *)m->d, m->ld, m->d_ipiv, k0, w, m->N, k0, k0 + w);
+  BG_LAUNCHED();
+  prof_stop(PROF_LASWP, 0.0);
+  return BG_OK;
 }
 
 struct LUWork {
@@ -761,10 +1023,68 @@ static int panel_cluster_size() {
   return cs;
 }
 
+// CTAs per cluster of k_panel_rf<C> that this device can place (16, 8 or 0)
+template <class C>
+static int panel_rf_cluster() {
+  static int cs = -1;
+  if (cs >= 0) return cs;
+  cs = 0;
+  const int smem = (int)sizeof(PrfSmem<C>) + 32 * PrfCfg<C>::T * (int)sizeof(C);
+  if (cudaFuncSetAttribute(k_panel_rf<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_panel_rf<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return cs;
+  }
+  for (int want = PRF_MAXCL; want >= 8 && !cs; want /= 2) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = dim3(want);
+    cfg.blockDim = dim3(PrfCfg<C>::T);
+    cfg.dynamicSmemBytes = smem;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = want;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, (void *)k_panel_rf<C>, &cfg) == cudaSuccess && n >= 1) cs = want;
+  }
+  cudaGetLastError();
+  return cs;
+}
+
 template <class C>
 static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w) {
   int N = m->N;
   int Mp = N - k0;
+  // rows in the registers of one cluster, while they fit (a row per thread:
+  // 4,096 rows of complex128, 8,192 of complex64)
+  const int RS = panel_rf_cluster<C>();
+  if (RS && Mp <= RS * PrfCfg<C>::T) {
+    // at least 64 rows per CTA: rank 0 owns the w rows of the diagonal block,
+    // and fewer CTAs exchange faster than 32-row slices update
+    const int G = std::min(RS, std::max(1, (Mp + 63) / 64));
+    const int rows = (Mp + G - 1) / G;
+    PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow};
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(G);
+    cfg.blockDim = dim3(PrfCfg<C>::T);
+    cfg.dynamicSmemBytes = sizeof(PrfSmem<C>) + (size_t)32 * PrfCfg<C>::T * sizeof(C);
+    cfg.stream = stream();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = G;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    prof_start(PROF_PANEL);
+    BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_rf<C>, P));
+    BG_LAUNCHED();
+    prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
+    return laswp<C>(m, k0, w);
+  }
   // the whole panel in one cluster's shared memory: cluster barriers and
   // distributed shared memory instead of a grid barrier per column
   const int CS = panel_cluster_size<C>();
@@ -792,11 +1112,7 @@ static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w) {
       BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_cl<C>, P));
       BG_LAUNCHED();
       prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
-      prof_start(PROF_LASWP);
-      k_laswp<C><<<(N + 255) / 256, 256, 0, stream()>>>((C *)m->d, m->ld, m->d_ipiv, k0, w, 0, N, k0, k0 + w);
-      BG_LAUNCHED();
-      prof_stop(PROF_LASWP, 0.0);
-      return BG_OK;
+      return laswp<C>(m, k0, w);
     }
   }
   int G = std::min(panel_grid, std::max(1, (Mp + panel_rows_target - 1) / panel_rows_target));
@@ -818,13 +1134,7 @@ static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w) {
   BG_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_panel<C>, dim3(G), dim3(256), args, smem, stream()));
   BG_LAUNCHED();
   prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
-  int threads = 256;
-  int blocks = (N + threads - 1) / threads;
-  prof_start(PROF_LASWP);
-  k_laswp<C><<<blocks, threads, 0, stream()>>>((C *)m->d, m->ld, m->d_ipiv, k0, w, 0, N, k0, k0 + w);
-  BG_LAUNCHED();
-  prof_stop(PROF_LASWP, 0.0);
-  return BG_OK;
+  return laswp<C>(m, k0, w);
 }
 
 // factor columns [k0, k0+n) (rows k0..N-1); interchanges applied to all columns
@@ -907,7 +1217,7 @@ int lu_factor(bg_matrix *m) {
   BG_CUDA_TRY(cudaMemcpyAsync(info, W.info, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream()));
   BG_CUDA_TRY(cudaStreamSynchronize(stream()));
   if (info[1]) {
-    set_error("tensor-core GEMM reported a pipeline timeout (code %d)", info[1]);
+    set_error("factorisation: a %s wait timed out (code %d)", info[1] == 300 ? "panel" : "tensor-core GEMM", info[1]);
     return BG_ERR_CUDA;
   }
   if ((st = build_perm(m))) return st;
