@@ -695,10 +695,11 @@ __global__ void __launch_bounds__(PCL_THREADS) k_panel_cl(PanelArgs<C> P) {
 
 // -------------------------------------------------------------------------
 // The panel with its rows in registers, on one cluster.  A thread owns one row
-// of the panel; the active columns sit in its registers and move down by one
-// place per step (column j is always a[0]), so the rank-1 update reads and
-// writes registers only, and the finished columns go to shared memory
-// (Ls[c][row]), from where the whole slice is written out once.  The
+// of the panel in registers, so the rank-1 update reads and writes registers
+// only; finished columns go to shared memory (Ls[c][row]), from where the whole
+// slice is written out once.  Columns are updated in fixed groups of eight
+// that end past column j: the finished columns among them compute on
+// leftovers that nothing reads.  The
 // shared-memory form above moves 32 bytes of shared memory per updated entry
 // and is bound by that and by its barriers: 3.3-3.9 us a column.
 //
@@ -706,14 +707,22 @@ __global__ void __launch_bounds__(PCL_THREADS) k_panel_cl(PanelArgs<C> P) {
 // pivot candidate with redux on the bits of |re| + |im| (non-negative, so they
 // order as integers) and the candidate's thread copies its row to shared
 // memory; after the barrier every warp knows the CTA's candidate, and warp q
-// pushes the candidate's row to CTAs q, q + warps, ... with st.async, which
-// counts its bytes on the receiver's mbarrier.  The CTA of rank 0, which owns
-// the rows k0 .. k0 + w - 1, pushes row k0 + j as well.  When its mbarrier
-// completes, a CTA has every candidate and both rows of the interchange in its
-// own shared memory: no remote loads, no cluster barrier.  Two buffers by
-// column parity: a CTA sends column j + 2 after it has received every
-// candidate of column j + 1, which each CTA sends only after all its warps
-// have finished with column j.  Waits are bounded; one that runs out is
+// pushes its row to CTAs q, q + warps, ... with st.async, which counts its
+// bytes on the receiver's mbarrier.  An extra warp pushes the candidate's key
+// and the reciprocal of its pivot.  When the mbarrier completes, a CTA has
+// every candidate in its own shared memory: no remote loads, no cluster
+// barrier.  The other row of the interchange, k0 + j, is in every CTA as
+// well: the extra warp keeps a copy of the w top rows and updates it like its
+// own.  The next column is updated first, so that the search for its pivot
+// runs while the other columns are updated.  What bounds a column is the
+// number of instructions a warp issues between two exchanges (8 cycles each
+// with two or three warps per scheduler): registers keep their columns (moving
+// them down by one place per step cost two moves per register), offsets are
+// constants of the unrolled code, column j + 1 is picked by a jump, and the
+// division is left to the extra warp.
+// Two buffers by column parity: a CTA sends column j + 2 after it has received
+// every candidate of column j + 1, which each CTA sends only after all its
+// warps have finished with column j.  Waits are bounded; one that runs out is
 // reported through info, and the CTA goes on so that the cluster ends.
 //
 // Pivot choice (first index on ties), interchanges and arithmetic are those of
@@ -721,24 +730,29 @@ __global__ void __launch_bounds__(PCL_THREADS) k_panel_cl(PanelArgs<C> P) {
 // -------------------------------------------------------------------------
 #define PRF_MAXCL 16
 #define PRF_SPIN (1 << 17)
+// Rows per CTA at most: T0 while that is enough (256 / 512 threads with the
+// extra warp, so that a thread may use 255 / 128 registers and the eight
+// loads of a group are in flight together), T1 for the tallest panels
 template <class C> struct PrfCfg;
-template <> struct PrfCfg<cdl> { static constexpr int T = 256; };   // 32 columns = 128 registers a row
-template <> struct PrfCfg<cfl> { static constexpr int T = 512; };
+template <> struct PrfCfg<cdl> { static constexpr int T0 = 224, T1 = 256; };   // 32 columns = 128 registers a row
+template <> struct PrfCfg<cfl> { static constexpr int T0 = 480, T1 = 512; };
 
 template <class C>
-struct PrfMsg {
+struct alignas(16) PrfMsg {        // st.async writes 16 bytes at a time
   C row[32];
   unsigned long long key;
   long long idx;
+  C inv;                            // reciprocal of the candidate
 };
 template <class C>
-struct PrfSmem {
+struct alignas(16) PrfSmem {
+  static constexpr int NW = PrfCfg<C>::T1 / 32;
   PrfMsg<C> msg[2][PRF_MAXCL];
-  C jrow[2][32];                    // row k0 + j before the interchange
-  C wrow[2][PrfCfg<C>::T / 32][32]; // candidate rows of the warps (active part, wrow[c] = column j + c)
-  C myj[2][32];                     // rank 0: active part of row k0 + j
-  unsigned long long wkey[2][PrfCfg<C>::T / 32];
-  int widx[2][PrfCfg<C>::T / 32];
+  alignas(16) C wrow[2][NW][32];    // candidate rows of the warps, columns >= j
+  alignas(16) C jrow[2][32];                    // row k0 + j before the interchange, columns >= j
+  alignas(16) C Lt[32][32];                // Lt[c][i]: finished columns of the copy of row k0 + i
+  unsigned long long wkey[2][NW];
+  int widx[2][NW];
   unsigned long long bar[2];
 };
 __device__ __forceinline__ unsigned long long pivot_key(cdl v) {
@@ -749,22 +763,34 @@ __device__ __forceinline__ unsigned long long pivot_key(cfl v) {
   const float a = fabsf(v.r) + fabsf(v.i);
   return a == a ? (unsigned long long)__float_as_uint(a) << 32 : 0ull;
 }
-// lane of the first maximum of key over the lanes with ok (-1: none); key of it
+// lane of the first maximum of key over the lanes with ok (-1: none), key of
+// it; mh: the warp's maximum of the high words (of the lanes with ok, else 0).
+// Equal high words are rare, so the low words are compared only then.
+__device__ __forceinline__ unsigned key_hi(unsigned long long key, bool ok) { return ok ? (unsigned)(key >> 32) : 0u; }
 template <class C>
-__device__ __forceinline__ int warp_first_max(unsigned long long &key, bool ok) {
-  const unsigned hi = ok ? (unsigned)(key >> 32) : 0u;
-  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-  bool c = ok && hi == mh;
-  unsigned ml = 0;
-  if (sizeof(C) == 16) {
-    const unsigned lo = c ? (unsigned)key : 0u;
-    ml = __reduce_max_sync(0xffffffffu, lo);
+__device__ __forceinline__ int warp_first_max(unsigned long long &key, bool ok, unsigned mh) {
+  bool c = ok && (unsigned)(key >> 32) == mh;
+  unsigned b = __ballot_sync(0xffffffffu, c);
+  if (sizeof(C) == 16 && (b & (b - 1))) {
+    const unsigned lo = c ? (unsigned)key : 0u, ml = __reduce_max_sync(0xffffffffu, lo);
     c = c && lo == ml;
+    b = __ballot_sync(0xffffffffu, c);
   }
-  const unsigned b = __ballot_sync(0xffffffffu, c);
-  key = (unsigned long long)mh << 32 | ml;
-  return b ? __ffs(b) - 1 : -1;
+  const int src = b ? __ffs(b) - 1 : -1;
+  key = __shfl_sync(0xffffffffu, key, src < 0 ? 0 : src);
+  return src;
 }
+// one access per entry of an aligned shared array
+__device__ __forceinline__ cdl lds_c(const cdl *p) {
+  const double2 v = *reinterpret_cast<const double2 *>(p);
+  return cdl{v.x, v.y};
+}
+__device__ __forceinline__ cfl lds_c(const cfl *p) {
+  const float2 v = *reinterpret_cast<const float2 *>(p);
+  return cfl{v.x, v.y};
+}
+__device__ __forceinline__ void sts_c(cdl *p, cdl v) { *reinterpret_cast<double2 *>(p) = make_double2(v.r, v.i); }
+__device__ __forceinline__ void sts_c(cfl *p, cfl v) { *reinterpret_cast<float2 *>(p) = make_float2(v.r, v.i); }
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned map_cta(unsigned a, int rank) {
   unsigned r;
@@ -787,22 +813,33 @@ __device__ __forceinline__ void push_c(unsigned dst, cfl v, unsigned bar) {
   st_async8(dst, (unsigned long long)__float_as_uint(v.i) << 32 | __float_as_uint(v.r), bar);
 }
 
+// a - l u
 template <class C>
-__global__ void __launch_bounds__(PrfCfg<C>::T) k_panel_rf(PanelArgs<C> P) {
+__device__ __forceinline__ C prf_upd(C a, C l, C u) {
+  return C{fma(-l.r, u.r, fma(l.i, u.i, a.r)), fma(-l.r, u.i, fma(-l.i, u.r, a.i))};
+}
+
+template <class C, int TMAX>
+__global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
   typedef typename CxT<C>::R R;
-  constexpr int T = PrfCfg<C>::T, NW = T / 32;
+  constexpr int T = TMAX + 1;      // column stride of Ls: a row's columns fall into different banks
   extern __shared__ __align__(16) unsigned char smem_raw[];
   PrfSmem<C> &S = *reinterpret_cast<PrfSmem<C> *>(smem_raw);
-  C *Ls = reinterpret_cast<C *>(smem_raw + sizeof(PrfSmem<C>));   // [w][T]
+  C *Ls = reinterpret_cast<C *>(smem_raw + sizeof(PrfSmem<C>));   // [32][T]
   cg::cluster_group cl = cg::this_cluster();
-  const int w = P.w, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int w = P.w, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = (int)(blockDim.x >> 5) - 1;
   const int rank = (int)cl.block_rank(), G = (int)cl.num_blocks();
   const int r0 = P.k0 + rank * P.rows_per, nr = max(0, min(P.rows_per, P.Nr - r0));
-  const int row = r0 + tid;
-  const bool mine = tid < nr;
+  const bool top = wid == nw;                      // the copy of the top rows
+  const int row = top ? P.k0 + lane : r0 + tid;
+  const bool mine = !top && tid < nr, held = mine || (top && lane < w);
+  // finished columns of this thread's row: column c at Lrow[c * Lstep]
+  C *Lrow = top ? &S.Lt[0][lane] : Ls + tid;
+  const int Lstep = top ? 32 : T;
   C a[32];
 #pragma unroll
-  for (int c = 0; c < 32; c++) a[c] = (mine && c < w) ? P.A[(size_t)(P.k0 + c) * P.ld + row] : C{0, 0};
+  for (int c = 0; c < 32; c++) a[c] = (held && c < w) ? P.A[(size_t)(P.k0 + c) * P.ld + row] : C{0, 0};
+  const unsigned base = smem_addr(&S);
   const unsigned bar0 = smem_addr(&S.bar[0]);
   if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
@@ -810,45 +847,65 @@ __global__ void __launch_bounds__(PrfCfg<C>::T) k_panel_rf(PanelArgs<C> P) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   cl.sync();   // barriers of every CTA are ready
-  const unsigned bytes = (unsigned)(G * (32 * sizeof(C) + 16) + 32 * sizeof(C));
+  const unsigned bytes = (unsigned)(G * (33 * sizeof(C) + 16));
   int limit = PRF_SPIN;
+  // search state of the coming column: this row's entry, its key, the warp's maximum
+  C cur = a[0];
+  unsigned long long key = pivot_key(cur);
+  unsigned mh = __reduce_max_sync(0xffffffffu, key_hi(key, mine));
   for (int j = 0; j < w; j++) {
     const int gj = P.k0 + j, buf = j & 1;
     const unsigned bar = bar0 + 8 * buf;
     if (tid == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-    // 1. candidate of every warp; its row and rank 0's row gj to shared memory
-    {
-      unsigned long long key = pivot_key(a[0]);
-      const int src = warp_first_max<C>(key, mine && row >= gj);
+    // 1. candidate of every warp; its row, and row gj from the top copy
+    int src = j;
+    C *keep = S.jrow[buf];
+    if (!top) {
+      src = warp_first_max<C>(key, mine && row >= gj, mh);
       if (lane == 0) {
         S.wkey[buf][wid] = key;
         S.widx[buf][wid] = src < 0 ? 0x7fffffff : r0 + wid * 32 + src;
       }
-      if (lane == src)
-#pragma unroll
-        for (int c = 0; c < 32; c++) S.wrow[buf][wid][c] = a[c];
-      if (mine && row == gj)
-#pragma unroll
-        for (int c = 0; c < 32; c++) S.myj[buf][c] = a[c];
+      keep = S.wrow[buf][wid];
     }
+    if (lane == src)
+#pragma unroll
+      for (int c0 = 0; c0 < 32; c0 += 8)
+        if (c0 + 7 >= j)
+#pragma unroll
+          for (int c = c0; c < c0 + 8; c++) sts_c(keep + c, a[c]);
     __syncthreads();
-    // 2. the CTA's candidate, pushed to every CTA (warp q: CTAs q, q + NW, ...)
+    // 2. the CTA's candidate, pushed to every CTA: its row by warp q to CTAs
+    // q, q + nw, ..., key and reciprocal by the extra warp, lane q to CTA q
     {
-      unsigned long long key = lane < NW ? S.wkey[buf][lane] : 0ull;
-      const int idx = lane < NW ? S.widx[buf][lane] : 0x7fffffff;
-      const int bw = warp_first_max<C>(key, idx != 0x7fffffff);
-      const int bi = __shfl_sync(0xffffffffu, idx, bw < 0 ? 0 : bw);
-      C v = C{0, 0};
-      if (bw >= 0 && lane < w) v = lane < j ? Ls[lane * T + (bi - r0)] : S.wrow[buf][bw][lane - j];
-      C vj = C{0, 0};
-      if (rank == 0 && lane < w) vj = lane < j ? Ls[lane * T + j] : S.myj[buf][lane - j];
-      for (int q = wid; q < G; q += NW) {
-        const unsigned rb = map_cta(bar, q);
-        push_c(map_cta(smem_addr(&S.msg[buf][rank].row[lane]), q), v, rb);
-        if (lane == 0)
-          st_async16(map_cta(smem_addr(&S.msg[buf][rank].key), q), key, (unsigned long long)(bw < 0 ? -1ll : (long long)bi), rb);
-        if (rank == 0) push_c(map_cta(smem_addr(&S.jrow[buf][lane]), q), vj, rb);
+      unsigned long long k2 = lane < nw ? S.wkey[buf][lane] : 0ull;
+      const int idx = lane < nw ? S.widx[buf][lane] : 0x7fffffff;
+      const bool ok = idx != 0x7fffffff;
+      const int bw = warp_first_max<C>(k2, ok, __reduce_max_sync(0xffffffffu, key_hi(k2, ok)));
+      const unsigned msg = smem_addr(&S.msg[buf][rank]) - base;
+      if (top) {
+        const int bi = __shfl_sync(0xffffffffu, idx, bw < 0 ? 0 : bw);
+        if (lane < G) {
+          const unsigned rbase = map_cta(base, lane), rb = rbase + (bar - base);
+          st_async16(rbase + msg + 32 * (unsigned)sizeof(C), k2, (unsigned long long)(bw < 0 ? -1ll : (long long)bi), rb);
+          C iv = C{0, 0};
+          if (bw >= 0) {
+            const C p = lds_c(&S.wrow[buf][bw][j]);
+            const R d = p.r * p.r + p.i * p.i;
+            iv = C{p.r / d, -p.i / d};
+          }
+          push_c(rbase + msg + 32 * (unsigned)sizeof(C) + 16, iv, rb);
+        }
+      } else {
+        const int bi = __shfl_sync(0xffffffffu, idx, bw < 0 ? 0 : bw);
+        C v = C{0, 0};
+        if (bw >= 0 && lane < w) v = lds_c(lane < j ? &Ls[lane * T + (bi - r0)] : &S.wrow[buf][bw][lane]);
+        const unsigned dst = msg + lane * (unsigned)sizeof(C);
+        for (int q = wid; q < G; q += nw) {
+          const unsigned rbase = map_cta(base, q);
+          push_c(rbase + dst, v, rbase + (bar - base));
+        }
       }
     }
     // 3. everyone's candidates
@@ -863,54 +920,67 @@ __global__ void __launch_bounds__(PrfCfg<C>::T) k_panel_rf(PanelArgs<C> P) {
             : "memory");
       if (!done) { limit = 1; atomicExch(P.info, 0x7fffffff); atomicExch(P.info + 1, 300); }
     }
-    __syncthreads();   // every warp has read the rows it pushes (Ls changes below)
-    unsigned long long key = lane < G ? S.msg[buf][lane].key : 0ull;
-    const long long idx = lane < G ? S.msg[buf][lane].idx : -1;
-    int b = warp_first_max<C>(key, idx >= 0);
+    const int ql = lane < G ? lane : 0;
+    unsigned long long k3 = S.msg[buf][ql].key;
+    const int idx = (int)S.msg[buf][ql].idx;
+    const bool ok = lane < G && idx >= 0;
+    int b = warp_first_max<C>(k3, ok, __reduce_max_sync(0xffffffffu, key_hi(k3, ok)));
     if (b < 0) b = 0;
-    const int piv = (int)__shfl_sync(0xffffffffu, (int)idx, b);
-    const C *prow = S.msg[buf][b].row;
-    if (rank == 0 && tid == 0) P.ipiv[gj] = piv + 1;
-    // 4. interchange: row gj's U part and L part are final and go to Ls (by
-    // the last warp of rank 0); the pivot's owner takes over the old row gj
-    if (rank == 0 && wid == NW - 1 && lane < w) Ls[lane * T + j] = prow[lane];
-    if (piv != gj && mine && row == piv) {
-#pragma unroll
-      for (int c = 0; c < 32; c++)
-        if (j + c < w) a[c] = S.jrow[buf][j + c];
-#pragma unroll 8
-      for (int c = 0; c < j; c++) Ls[c * T + tid] = S.jrow[buf][c];
+    const int piv = __shfl_sync(0xffffffffu, idx, b);
+    const PrfMsg<C> &W = S.msg[buf][b];
+    const C p = lds_c(&W.row[j]), pinv = lds_c(&W.inv);
+    __syncthreads();   // every warp has read the rows it pushes (Ls changes below)
+    // 4. interchange: row gj is final and goes to Ls (a warp of rank 0); the
+    // pivot's place takes over the old row gj
+    if (rank == 0) {
+      if (tid == 0) P.ipiv[gj] = piv + 1;
+      if (wid == nw - 1 && lane < w) sts_c(&Ls[lane * T + j], lds_c(&W.row[lane]));
     }
-    // 5. scale and update; a[c] becomes column j + 1 + c
-    const C p = prow[j];
-    const R d = p.r * p.r + p.i * p.i;
-    const bool zero = d == (R)0;
-    if (zero && rank == 0 && tid == 0) atomicCAS(P.info, 0, gj + 1);
-    if (mine && row > gj) {
-      C l = a[0];
-      if (!zero) {
-        const C inv{p.r / d, -p.i / d};
-        l = C{a[0].r * inv.r - a[0].i * inv.i, a[0].r * inv.i + a[0].i * inv.r};
-      }
-      Ls[j * T + tid] = l;
-      if (zero) l = C{0, 0};
-      const int ncol = w - j - 1;
+    if (piv != gj && held && row == piv) {
 #pragma unroll
       for (int c0 = 0; c0 < 32; c0 += 8)
-        if (c0 < ncol)
+        if (c0 + 7 >= j)
 #pragma unroll
-          for (int c = c0; c < c0 + 8 && c < 31; c++) {
-            const C u = (c < ncol && !zero) ? prow[j + 1 + c] : C{0, 0};
-            a[c].r = a[c + 1].r - (l.r * u.r - l.i * u.i);
-            a[c].i = a[c + 1].i - (l.r * u.i + l.i * u.r);
-          }
+          for (int c = c0; c < c0 + 8; c++) a[c] = lds_c(&S.jrow[buf][c]);
+      cur = lds_c(&S.jrow[buf][j]);
+#pragma unroll 8
+      for (int c = 0; c < j; c++) sts_c(&Lrow[c * Lstep], lds_c(&S.Lt[c][j]));
+    }
+    // 5. scale and update
+    const R d = p.r * p.r + p.i * p.i;
+    const bool zero = d == (R)0, below = held && row > gj;
+    C l = cur;
+    if (zero) {
+      if (rank == 0 && tid == 0) atomicCAS(P.info, 0, gj + 1);
+    } else {
+      l = C{cur.r * pinv.r - cur.i * pinv.i, cur.r * pinv.i + cur.i * pinv.r};
+    }
+    if (below) sts_c(&Lrow[j * Lstep], l);
+    if (j + 1 == w) break;
+    switch (j + 1) {
+#define PRF_PICK(c) case c: cur = a[c]; break;
+      PRF_PICK(1) PRF_PICK(2) PRF_PICK(3) PRF_PICK(4) PRF_PICK(5) PRF_PICK(6) PRF_PICK(7) PRF_PICK(8) PRF_PICK(9)
+      PRF_PICK(10) PRF_PICK(11) PRF_PICK(12) PRF_PICK(13) PRF_PICK(14) PRF_PICK(15) PRF_PICK(16) PRF_PICK(17)
+      PRF_PICK(18) PRF_PICK(19) PRF_PICK(20) PRF_PICK(21) PRF_PICK(22) PRF_PICK(23) PRF_PICK(24) PRF_PICK(25)
+      PRF_PICK(26) PRF_PICK(27) PRF_PICK(28) PRF_PICK(29) PRF_PICK(30) PRF_PICK(31)
+#undef PRF_PICK
+    }
+    if (!zero) cur = prf_upd(cur, l, lds_c(&W.row[j + 1]));
+    key = pivot_key(cur);
+    mh = __reduce_max_sync(0xffffffffu, key_hi(key, mine && row > gj));
+    if (!zero) {
+#pragma unroll
+      for (int c0 = 0; c0 < 32; c0 += 8)
+        if (c0 + 7 > j)
+#pragma unroll
+          for (int c = c0; c < c0 + 8; c++) a[c] = prf_upd(a[c], l, lds_c(&W.row[c]));
     }
   }
   __syncthreads();
   // rows k0 .. k0 + w - 1 hold U (and the L of their interchanges), written
   // to Ls by step 4; the others hold their L
   if (mine)
-    for (int c = 0; c < w; c++) P.A[(size_t)(P.k0 + c) * P.ld + row] = Ls[c * T + tid];
+    for (int c = 0; c < w; c++) P.A[(size_t)(P.k0 + c) * P.ld + row] = lds_c(&Ls[c * T + tid]);
   cl.sync();   // no CTA leaves while messages for it may be in flight
 }
 
@@ -1023,15 +1093,18 @@ static int panel_cluster_size() {
   return cs;
 }
 
-// CTAs per cluster of k_panel_rf<C> that this device can place (16, 8 or 0)
-template <class C>
+template <class C, int TMAX>
+constexpr int panel_rf_smem() { return (int)sizeof(PrfSmem<C>) + 32 * (TMAX + 1) * (int)sizeof(C); }
+
+// CTAs per cluster of k_panel_rf that this device can place (16, 8 or 0)
+template <class C, int TMAX>
 static int panel_rf_cluster() {
   static int cs = -1;
   if (cs >= 0) return cs;
   cs = 0;
-  const int smem = (int)sizeof(PrfSmem<C>) + 32 * PrfCfg<C>::T * (int)sizeof(C);
-  if (cudaFuncSetAttribute(k_panel_rf<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_panel_rf<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+  const int smem = panel_rf_smem<C, TMAX>();
+  if (cudaFuncSetAttribute(k_panel_rf<C, TMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_panel_rf<C, TMAX>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return cs;
   }
@@ -1039,7 +1112,7 @@ static int panel_rf_cluster() {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     cfg.gridDim = dim3(want);
-    cfg.blockDim = dim3(PrfCfg<C>::T);
+    cfg.blockDim = dim3(TMAX + 32);
     cfg.dynamicSmemBytes = smem;
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = want;
@@ -1048,10 +1121,40 @@ static int panel_rf_cluster() {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, (void *)k_panel_rf<C>, &cfg) == cudaSuccess && n >= 1) cs = want;
+    if (cudaOccupancyMaxActiveClusters(&n, (void *)k_panel_rf<C, TMAX>, &cfg) == cudaSuccess && n >= 1) cs = want;
   }
   cudaGetLastError();
   return cs;
+}
+
+// the panel on one cluster with its rows in registers; *done = false: too tall
+template <class C, int TMAX>
+static int panel_rf(bg_matrix *m, const LUWork &W, int k0, int w, bool *done) {
+  const int N = m->N, Mp = N - k0, RS = panel_rf_cluster<C, TMAX>();
+  *done = RS && Mp <= RS * TMAX;
+  if (!*done) return BG_OK;
+  // 128 rows per CTA, one warp per scheduler, until the cluster is full
+  // (rank 0 owns the w rows of the diagonal block)
+  const int G = std::min(RS, std::max(1, (Mp + 127) / 128));
+  const int rows = (Mp + G - 1) / G, threads = (rows + 31) / 32 * 32 + 32;
+  PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(G);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = panel_rf_smem<C, TMAX>();
+  cfg.stream = stream();
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = G;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  prof_start(PROF_PANEL);
+  BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_rf<C, TMAX>, P));
+  BG_LAUNCHED();
+  prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
+  return laswp<C>(m, k0, w);
 }
 
 template <class C>
@@ -1059,32 +1162,11 @@ static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w) {
   int N = m->N;
   int Mp = N - k0;
   // rows in the registers of one cluster, while they fit (a row per thread:
-  // 4,096 rows of complex128, 8,192 of complex64)
-  const int RS = panel_rf_cluster<C>();
-  if (RS && Mp <= RS * PrfCfg<C>::T) {
-    // at least 64 rows per CTA: rank 0 owns the w rows of the diagonal block,
-    // and fewer CTAs exchange faster than 32-row slices update
-    const int G = std::min(RS, std::max(1, (Mp + 63) / 64));
-    const int rows = (Mp + G - 1) / G;
-    PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow};
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(G);
-    cfg.blockDim = dim3(PrfCfg<C>::T);
-    cfg.dynamicSmemBytes = sizeof(PrfSmem<C>) + (size_t)32 * PrfCfg<C>::T * sizeof(C);
-    cfg.stream = stream();
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = G;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    prof_start(PROF_PANEL);
-    BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_rf<C>, P));
-    BG_LAUNCHED();
-    prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
-    return laswp<C>(m, k0, w);
-  }
+  // 4,096 rows of complex128, 8,192 of complex64 with 16 CTAs)
+  bool done = false;
+  int st = panel_rf<C, PrfCfg<C>::T0>(m, W, k0, w, &done);
+  if (!st && !done) st = panel_rf<C, PrfCfg<C>::T1>(m, W, k0, w, &done);
+  if (st || done) return st;
   // the whole panel in one cluster's shared memory: cluster barriers and
   // distributed shared memory instead of a grid barrier per column
   const int CS = panel_cluster_size<C>();
