@@ -60,10 +60,29 @@ __device__ __forceinline__ void dmma16(double (&d)[4], const double (&a)[8], con
         "d"(b[1]), "d"(b[2]), "d"(b[3]));
 }
 
+// one access per entry of an aligned shared array
+__device__ __forceinline__ cdl lds_c(const cdl *p) {
+  const double2 v = *reinterpret_cast<const double2 *>(p);
+  return cdl{v.x, v.y};
+}
+__device__ __forceinline__ cfl lds_c(const cfl *p) {
+  const float2 v = *reinterpret_cast<const float2 *>(p);
+  return cfl{v.x, v.y};
+}
+__device__ __forceinline__ void sts_c(cdl *p, cdl v) { *reinterpret_cast<double2 *>(p) = make_double2(v.r, v.i); }
+__device__ __forceinline__ void sts_c(cfl *p, cfl v) { *reinterpret_cast<float2 *>(p) = make_float2(v.r, v.i); }
+
 __device__ __forceinline__ void cp16(void *smem, const void *gmem, bool pred) {
   unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   int n = pred ? 16 : 0;
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
+}
+// one matrix entry, zero when !pred
+__device__ __forceinline__ void cp_entry(cdl *smem, const cdl *gmem, bool pred) { cp16(smem, gmem, pred); }
+__device__ __forceinline__ void cp_entry(cfl *smem, const cfl *gmem, bool pred) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  int n = pred ? 8 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(n));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -194,6 +213,134 @@ __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, STAGES>::THREADS)
   }
 }
 
+// The same product with 32 x 32 tiles and the K loop split over the four warps
+// of a CTA (warp q takes rows 8 q .. 8 q + 7 of every 32-deep chunk; the four
+// partial tiles are summed in shared memory in warp order).  A 64 x 64 tile
+// occupies its SM for 17 us at K = 128 whatever the grid; where a product has
+// too few of them for the 148 SMs this form has four times the tiles, a quarter
+// of the time each: 128 x 128 x 128 27.9 -> 10.5 us, 512^3 90 -> 43 us,
+// 256 x 2048 x 256 49 -> 45 us.  It reads twice the operand bytes per flop and
+// loses from about 230 tiles on (3840 x 256 x 256, 240 tiles: 83 against 87 us).
+__device__ __forceinline__ void dmma8(double (&d)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+d"(d[0]), "+d"(d[1]), "+d"(d[2]), "+d"(d[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+#define ZG_SMALL 220             // 64 x 64 tiles up to which the small tiles are taken
+#define ZS_ST 3
+#define ZS_AP 34                 // As[k][m] stride, = 2 mod 8
+#define ZS_BP 36                 // Bs[n][k] stride, = 4 mod 8
+#define ZS_STAGE (32 * ZS_AP + 32 * ZS_BP)
+#define ZS_SMEM (ZS_ST * ZS_STAGE * 16)
+__global__ void __launch_bounds__(128) k_zgemm_small(int M, int N, int K, const cdl *__restrict__ A, size_t lda,
+                                                      const cdl *__restrict__ B, size_t ldb, cdl *C, size_t ldc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cdl *sm = (cdl *)smem_raw;
+  const int m0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
+  const int tid = threadIdx.x, lane = tid & 31, wk = tid >> 5, t0 = lane & 3, t1 = lane >> 2;
+  double cr[2][4][4], ci[2][4][4];
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+#pragma unroll
+      for (int v = 0; v < 4; v++) cr[i][j][v] = ci[i][j][v] = 0.0;
+  const int nchunks = (K + 31) / 32;
+  auto load_chunk = [&](int chunk) {
+    const int k0 = chunk * 32;
+    cdl *as = sm + (chunk % ZS_ST) * ZS_STAGE, *bs = as + 32 * ZS_AP;
+#pragma unroll
+    for (int it = 0; it < 8; it++) {
+      const int kk = wk + 4 * it;
+      const bool oka = m0 + lane < M && k0 + kk < K, okb = k0 + lane < K && n0 + kk < N;
+      cp16(as + kk * ZS_AP + lane, oka ? A + (size_t)(k0 + kk) * lda + m0 + lane : A, oka);
+      cp16(bs + kk * ZS_BP + lane, okb ? B + (size_t)(n0 + kk) * ldb + k0 + lane : B, okb);
+    }
+  };
+#pragma unroll
+  for (int s = 0; s < ZS_ST - 1; s++) {
+    if (s < nchunks) load_chunk(s);
+    cp_commit();
+  }
+  // this thread's entries of C (the rows 8 wk .. of the tile), read early
+  cdl x[8];
+#pragma unroll
+  for (int e = 0; e < 8; e++) {
+    const int col = n0 + wk * 8 + e;
+    x[e] = (m0 + lane < M && col < N) ? C[(size_t)col * ldc + m0 + lane] : cdl{0.0, 0.0};
+  }
+  for (int chunk = 0; chunk < nchunks; chunk++) {
+    cp_wait<ZS_ST - 2>();
+    __syncthreads();
+    if (chunk + ZS_ST - 1 < nchunks) load_chunk(chunk + ZS_ST - 1);
+    cp_commit();
+    const cdl *as = sm + (chunk % ZS_ST) * ZS_STAGE + (8 * wk + t0) * ZS_AP + t1;
+    const cdl *bs = sm + (chunk % ZS_ST) * ZS_STAGE + 32 * ZS_AP + t1 * ZS_BP + 8 * wk + t0;
+    double ar[2][4], ai[2][4];
+#pragma unroll
+    for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+      for (int v = 0; v < 4; v++) {
+        const cdl z = lds_c(as + 4 * (v >> 1) * ZS_AP + mt * 16 + 8 * (v & 1));
+        ar[mt][v] = z.r;
+        ai[mt][v] = z.i;
+      }
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++) {
+      double br[2], bi[2], nbi[2];
+#pragma unroll
+      for (int v = 0; v < 2; v++) {
+        const cdl z = lds_c(bs + nt * 8 * ZS_BP + 4 * v);
+        br[v] = z.r;
+        bi[v] = z.i;
+        nbi[v] = -z.i;
+      }
+#pragma unroll
+      for (int mt = 0; mt < 2; mt++) {
+        dmma8(cr[mt][nt], ar[mt], br);
+        dmma8(cr[mt][nt], ai[mt], nbi);
+        dmma8(ci[mt][nt], ar[mt], bi);
+        dmma8(ci[mt][nt], ai[mt], br);
+      }
+    }
+  }
+  cp_wait<0>();
+  __syncthreads();
+  // partial tiles [warp][col][row], then C -= their sum
+#pragma unroll
+  for (int mt = 0; mt < 2; mt++)
+#pragma unroll
+    for (int nt = 0; nt < 4; nt++)
+#pragma unroll
+      for (int v = 0; v < 4; v++)
+        sts_c(sm + wk * 32 * 33 + (nt * 8 + 2 * t0 + (v & 1)) * 33 + mt * 16 + t1 + 8 * (v >> 1),
+              cdl{cr[mt][nt][v], ci[mt][nt][v]});
+  __syncthreads();
+#pragma unroll
+  for (int e = 0; e < 8; e++) {
+    const int c = wk * 8 + e, col = n0 + c;
+    cdl s{0.0, 0.0};
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const cdl z = lds_c(sm + q * 32 * 33 + c * 33 + lane);
+      s.r += z.r;
+      s.i += z.i;
+    }
+    if (m0 + lane < M && col < N) C[(size_t)col * ldc + m0 + lane] = cdl{x[e].r - s.r, x[e].i - s.i};
+  }
+}
+static int zgemm_small(int M, int N, int K, const cdl *A, size_t lda, const cdl *B, size_t ldb, cdl *C, size_t ldc) {
+  static bool attr = false;
+  if (!attr) {
+    BG_CUDA_TRY(cudaFuncSetAttribute(k_zgemm_small, cudaFuncAttributeMaxDynamicSharedMemorySize, ZS_SMEM));
+    attr = true;
+  }
+  k_zgemm_small<<<dim3((M + 31) / 32, (N + 31) / 32), 128, ZS_SMEM, stream()>>>(M, N, K, A, lda, B, ldb, C, ldc);
+  BG_LAUNCHED();
+  return BG_OK;
+}
+
 // CTA tile of the complex128 GEMM, chosen at run time (the batching form's
 // autotuner times them per size class): 0 = 64 x 64, 1 = 128 x 64,
 // 2 = 64 x 128 complex outputs; warps always own 32 x 32.
@@ -220,98 +367,158 @@ static int zgemm_launch(int M, int N, int K, const cdl *A, size_t lda, const cdl
 static int zgemm_sub(int M, int N, int K, const cdl *A, size_t lda, const cdl *B, size_t ldb, cdl *C, size_t ldc) {
   if (M <= 0 || N <= 0 || K <= 0) return BG_OK;
   prof_start(PROF_GEMM);
-  int st = zg_tile == 1 ? zgemm_launch<128, 64>(M, N, K, A, lda, B, ldb, C, ldc)
+  // few 64 x 64 tiles leave SMs without work (both sides measured, see k_zgemm_small)
+  const long tiles = (long)((M + 63) / 64) * ((N + 63) / 64);
+  int st = tiles <= ZG_SMALL ? zgemm_small(M, N, K, A, lda, B, ldb, C, ldc)
+         : zg_tile == 1 ? zgemm_launch<128, 64>(M, N, K, A, lda, B, ldb, C, ldc)
          : zg_tile == 2 ? zgemm_launch<64, 128>(M, N, K, A, lda, B, ldb, C, ldc)
                         : zgemm_launch<64, 64>(M, N, K, A, lda, B, ldb, C, ldc);
   prof_stop(PROF_GEMM, 8.0 * M * (double)N * K);
   return st;
 }
 
-// =========================================================================
-// leaf triangular solves (n <= 64 rows).  The triangle is staged in shared
-// memory once per CTA; each warp then solves TRS_CPW right-hand-side columns
-// together: lane l holds rows l and l+32 of each of its columns in registers,
-// the solved entries of step i are broadcast with warp shuffles, and every
-// lane updates its two rows of every column with the one triangle entry it
-// read -- TRS_CPW independent recurrences per step, no block barriers inside
-// the substitution.
-// =========================================================================
-#define TRS_WARPS 8
-#define TRS_CPW 4                         // columns per warp per CTA
-#define TRS_COLS (TRS_WARPS * TRS_CPW)
+// a - l u
+template <class C>
+__device__ __forceinline__ C cfms(C a, C l, C u) {
+  return C{fma(-l.r, u.r, fma(l.i, u.i, a.r)), fma(-l.r, u.i, fma(-l.i, u.r, a.i))};
+}
 template <class C>
 __device__ __forceinline__ C cshfl(C v, int src) {
   return C{__shfl_sync(0xffffffffu, v.r, src), __shfl_sync(0xffffffffu, v.i, src)};
 }
+
+// =========================================================================
+// leaf triangular solves (n <= 128 rows).  The triangle is staged in shared
+// memory once per CTA, as the 32 x 32 blocks on and below (above) the
+// diagonal, column-major; a warp solves CPW right-hand-side columns, lane l
+// holding rows l, l + 32, l + 64, l + 96 of each in registers.  Step i
+// broadcasts the solved entry of every column with shuffles and updates all
+// later rows, those of the following blocks included, so the off-diagonal
+// products need no further pass where a 64-row leaf left them to GEMM launches
+// of 64 rows.  TRSM class of one factorisation: 5.2 -> 1.5 ms at N = 4,092,
+// 41 -> 23 ms at N = 19,872 (complex64 32 -> 13 ms).  CPW is the largest of
+// 4, 2, 1 that still gives every SM a CTA.
+// =========================================================================
+#define TRS_WARPS 8
+#define TRS_MAX 128
 template <class C>
-__global__ void __launch_bounds__(TRS_WARPS * 32) k_trsm_leaf(int n, int m, const C *T, size_t ldt, C *B,
-                                                              size_t ldb, int upper) {
+constexpr int trsm_smem() { return 10 * 32 * 32 * (int)sizeof(C) + TRS_MAX * (int)sizeof(C); }
+// block (br, bc) of the staged triangle: lower br >= bc, upper br <= bc
+__device__ __forceinline__ int trs_block(int br, int bc, bool upper) {
+  const int hi = upper ? bc : br, lo = upper ? br : bc;
+  return (hi * (hi + 1) / 2 + lo) * 1024;
+}
+template <class C, int CPW, bool UPPER>
+__global__ void __launch_bounds__(TRS_WARPS * 32) k_trsm_leaf(int n, int m, const C *T, size_t ldt, C *B, size_t ldb) {
   typedef typename CxT<C>::R R;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C(*Ts)[65] = (C(*)[65])smem_raw;   // Ts[r][c]
+  C *Ts = (C *)smem_raw;
+  C *dinv = Ts + 10 * 1024;      // upper: conj(u) / |u|^2 of the diagonal
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  // staged eight loads per thread at a time (their latencies overlap)
-  for (int e0 = 0; e0 < n * n; e0 += 8 * TRS_WARPS * 32) {
-    C v[8];
+  const int nb = (n + 31) / 32;
+  const int cbase = (blockIdx.x * TRS_WARPS + warp) * CPW;
+  C b[4][CPW];
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int e = e0 + u * TRS_WARPS * 32 + tid;
-      v[u] = e < n * n ? T[(size_t)(e / n) * ldt + e % n] : C{0, 0};
-    }
+  for (int q = 0; q < 4; q++)
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int e = e0 + u * TRS_WARPS * 32 + tid;
-      if (e < n * n) Ts[e % n][e / n] = v[u];
+    for (int j = 0; j < CPW; j++) {
+      const int r = 32 * q + lane, col = cbase + j;
+      b[q][j] = (r < n && col < m) ? B[(size_t)col * ldb + r] : C{0, 0};
     }
+  // one column of one block per warp and copy, all of them in flight together
+  for (int br = 0; br < nb; br++)
+    for (int bc = UPPER ? br : 0; bc < (UPPER ? nb : br + 1); bc++) {
+      C *dst = Ts + trs_block(br, bc, UPPER);
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const int r = 32 * br + lane, c = 32 * bc + warp + TRS_WARPS * u;
+        const bool ok = r < n && c < n;
+        cp_entry(dst + (warp + TRS_WARPS * u) * 32 + lane, ok ? T + (size_t)c * ldt + r : T, ok);
+      }
+    }
+  cp_commit();
+  if (UPPER && tid < n) {
+    const C u = T[(size_t)tid * ldt + tid];
+    const R d = u.r * u.r + u.i * u.i;
+    dinv[tid] = C{u.r / d, -u.i / d};
   }
+  cp_wait<0>();
   __syncthreads();
-  const int r0 = lane, r1 = lane + 32;
-  const int cbase = blockIdx.x * TRS_COLS + warp * TRS_CPW;
   if (cbase >= m) return;
-  C b0[TRS_CPW], b1[TRS_CPW];
+  if (!UPPER) {
 #pragma unroll
-  for (int j = 0; j < TRS_CPW; j++) {
-    const int col = cbase + j;
-    const C *bc = B + (size_t)col * ldb;
-    b0[j] = (col < m && r0 < n) ? bc[r0] : C{0, 0};
-    b1[j] = (col < m && r1 < n) ? bc[r1] : C{0, 0};
-  }
-  if (!upper) {
-    for (int i = 0; i < n; i++) {
-      const bool u0 = r0 > i && r0 < n, u1 = r1 > i && r1 < n;
-      const C l0 = u0 ? Ts[r0][i] : C{0, 0}, l1 = u1 ? Ts[r1][i] : C{0, 0};
+    for (int q = 0; q < 4; q++) {
+      if (q >= nb) break;
+      const int ni = min(32, n - 32 * q);
+      const C *t0 = Ts + trs_block(q, q, false) + lane;
+#pragma unroll 4
+      for (int i = 0; i < ni; i++) {
+        C x[CPW];
 #pragma unroll
-      for (int j = 0; j < TRS_CPW; j++) {
-        const C x = cshfl(i < 32 ? b0[j] : b1[j], i & 31);
-        if (u0) { b0[j].r -= l0.r * x.r - l0.i * x.i; b0[j].i -= l0.r * x.i + l0.i * x.r; }
-        if (u1) { b1[j].r -= l1.r * x.r - l1.i * x.i; b1[j].i -= l1.r * x.i + l1.i * x.r; }
+        for (int j = 0; j < CPW; j++) x[j] = cshfl(b[q][j], i);
+        const C l0 = lane > i ? lds_c(t0 + i * 32) : C{0, 0};
+#pragma unroll
+        for (int j = 0; j < CPW; j++) b[q][j] = cfms(b[q][j], l0, x[j]);
+#pragma unroll
+        for (int s = q + 1; s < 4; s++)
+          if (s < nb) {
+            const C l = lds_c(Ts + trs_block(s, q, false) + i * 32 + lane);
+#pragma unroll
+            for (int j = 0; j < CPW; j++) b[s][j] = cfms(b[s][j], l, x[j]);
+          }
       }
     }
   } else {
-    for (int i = n - 1; i >= 0; i--) {
-      const C u = Ts[i][i];
-      const R d = u.r * u.r + u.i * u.i;
-      const bool u0 = r0 < i, u1 = r1 < i;
-      const C t0 = u0 ? Ts[r0][i] : C{0, 0}, t1 = u1 ? Ts[r1][i] : C{0, 0};
 #pragma unroll
-      for (int j = 0; j < TRS_CPW; j++) {
-        const C v = cshfl(i < 32 ? b0[j] : b1[j], i & 31);
-        const C x{(v.r * u.r + v.i * u.i) / d, (v.i * u.r - v.r * u.i) / d};
-        if (r0 == i) b0[j] = x;
-        if (r1 == i) b1[j] = x;
-        if (u0) { b0[j].r -= t0.r * x.r - t0.i * x.i; b0[j].i -= t0.r * x.i + t0.i * x.r; }
-        if (u1) { b1[j].r -= t1.r * x.r - t1.i * x.i; b1[j].i -= t1.r * x.i + t1.i * x.r; }
+    for (int q = 3; q >= 0; q--) {
+      if (q >= nb) continue;
+      const int ni = min(32, n - 32 * q);
+      const C *t0 = Ts + trs_block(q, q, true) + lane;
+#pragma unroll 4
+      for (int i = ni - 1; i >= 0; i--) {
+        const C iu = lds_c(dinv + 32 * q + i);
+        C x[CPW];
+#pragma unroll
+        for (int j = 0; j < CPW; j++) {
+          const C v = cshfl(b[q][j], i);
+          x[j] = C{v.r * iu.r - v.i * iu.i, v.r * iu.i + v.i * iu.r};
+          if (lane == i) b[q][j] = x[j];
+        }
+        const C l0 = lane < i ? lds_c(t0 + i * 32) : C{0, 0};
+#pragma unroll
+        for (int j = 0; j < CPW; j++) b[q][j] = cfms(b[q][j], l0, x[j]);
+#pragma unroll
+        for (int s = 0; s < q; s++) {
+          const C l = lds_c(Ts + trs_block(s, q, true) + i * 32 + lane);
+#pragma unroll
+          for (int j = 0; j < CPW; j++) b[s][j] = cfms(b[s][j], l, x[j]);
+        }
       }
     }
   }
 #pragma unroll
-  for (int j = 0; j < TRS_CPW; j++) {
-    const int col = cbase + j;
-    if (col >= m) break;
-    C *bc = B + (size_t)col * ldb;
-    if (r0 < n) bc[r0] = b0[j];
-    if (r1 < n) bc[r1] = b1[j];
+  for (int q = 0; q < 4; q++)
+#pragma unroll
+    for (int j = 0; j < CPW; j++) {
+      const int r = 32 * q + lane, col = cbase + j;
+      if (r < n && col < m) B[(size_t)col * ldb + r] = b[q][j];
+    }
+}
+
+template <class C, int CPW, bool UPPER>
+static int trsm_launch(int n, int m, const C *T, size_t ldt, C *B, size_t ldb) {
+  static bool attr = false;
+  if (!attr) {
+    BG_CUDA_TRY(cudaFuncSetAttribute(k_trsm_leaf<C, CPW, UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     trsm_smem<C>()));
+    attr = true;
   }
+  const int cols = TRS_WARPS * CPW;
+  prof_start(PROF_TRSM);
+  k_trsm_leaf<C, CPW, UPPER><<<(m + cols - 1) / cols, TRS_WARPS * 32, trsm_smem<C>(), stream()>>>(n, m, T, ldt, B, ldb);
+  BG_LAUNCHED();
+  prof_stop(PROF_TRSM, 4.0 * n * (double)n * m);
+  return BG_OK;
 }
 
 // small-N complex64 GEMM (C -= A B, N <= 16): one thread per row, used where
@@ -375,22 +582,17 @@ static int gemm_sub(int M, int N, int K, const cfl *A, size_t lda, const cfl *B,
 template <class C>
 static int trsm(int n, int m, const C *T, size_t ldt, C *B, size_t ldb, int upper) {
   if (n <= 0 || m <= 0) return BG_OK;
-  if (n <= 64) {
-    const int smem = 64 * 65 * (int)sizeof(C);
-    static bool attr = false;
-    if (!attr) {
-      BG_CUDA_TRY(cudaFuncSetAttribute(k_trsm_leaf<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      attr = true;
-    }
-    int blocks = (m + TRS_COLS - 1) / TRS_COLS;
-    prof_start(PROF_TRSM);
-    k_trsm_leaf<C><<<blocks, TRS_WARPS * 32, smem, stream()>>>(n, m, T, ldt, B, ldb, upper);
-    BG_LAUNCHED();
-    prof_stop(PROF_TRSM, 4.0 * n * (double)n * m);
-    return BG_OK;
+  if (n <= TRS_MAX) {
+    const int blocks4 = (m + 4 * TRS_WARPS - 1) / (4 * TRS_WARPS);   // with four columns a warp
+    if (upper)
+      return blocks4 >= 148   ? trsm_launch<C, 4, true>(n, m, T, ldt, B, ldb)
+             : blocks4 >= 74  ? trsm_launch<C, 2, true>(n, m, T, ldt, B, ldb)
+                              : trsm_launch<C, 1, true>(n, m, T, ldt, B, ldb);
+    return blocks4 >= 148   ? trsm_launch<C, 4, false>(n, m, T, ldt, B, ldb)
+           : blocks4 >= 74  ? trsm_launch<C, 2, false>(n, m, T, ldt, B, ldb)
+                            : trsm_launch<C, 1, false>(n, m, T, ldt, B, ldb);
   }
-  int n1 = (n / 2 + 31) / 32 * 32;
-  if (n1 >= n) n1 = n / 2;
+  int n1 = (n / 2 + TRS_MAX - 1) / TRS_MAX * TRS_MAX;   // multiples of the leaf (n > TRS_MAX, so n1 < n)
   int n2 = n - n1;
   int st;
   if (!upper) {
@@ -780,17 +982,6 @@ __device__ __forceinline__ int warp_first_max(unsigned long long &key, bool ok, 
   key = __shfl_sync(0xffffffffu, key, src < 0 ? 0 : src);
   return src;
 }
-// one access per entry of an aligned shared array
-__device__ __forceinline__ cdl lds_c(const cdl *p) {
-  const double2 v = *reinterpret_cast<const double2 *>(p);
-  return cdl{v.x, v.y};
-}
-__device__ __forceinline__ cfl lds_c(const cfl *p) {
-  const float2 v = *reinterpret_cast<const float2 *>(p);
-  return cfl{v.x, v.y};
-}
-__device__ __forceinline__ void sts_c(cdl *p, cdl v) { *reinterpret_cast<double2 *>(p) = make_double2(v.r, v.i); }
-__device__ __forceinline__ void sts_c(cfl *p, cfl v) { *reinterpret_cast<float2 *>(p) = make_float2(v.r, v.i); }
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ unsigned map_cta(unsigned a, int rank) {
   unsigned r;
@@ -811,12 +1002,6 @@ __device__ __forceinline__ void push_c(unsigned dst, cdl v, unsigned bar) {
 }
 __device__ __forceinline__ void push_c(unsigned dst, cfl v, unsigned bar) {
   st_async8(dst, (unsigned long long)__float_as_uint(v.i) << 32 | __float_as_uint(v.r), bar);
-}
-
-// a - l u
-template <class C>
-__device__ __forceinline__ C prf_upd(C a, C l, C u) {
-  return C{fma(-l.r, u.r, fma(l.i, u.i, a.r)), fma(-l.r, u.i, fma(-l.i, u.r, a.i))};
 }
 
 template <class C, int TMAX>
@@ -965,7 +1150,7 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
       PRF_PICK(26) PRF_PICK(27) PRF_PICK(28) PRF_PICK(29) PRF_PICK(30) PRF_PICK(31)
 #undef PRF_PICK
     }
-    if (!zero) cur = prf_upd(cur, l, lds_c(&W.row[j + 1]));
+    if (!zero) cur = cfms(cur, l, lds_c(&W.row[j + 1]));
     key = pivot_key(cur);
     mh = __reduce_max_sync(0xffffffffu, key_hi(key, mine && row > gj));
     if (!zero) {
@@ -973,7 +1158,7 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
       for (int c0 = 0; c0 < 32; c0 += 8)
         if (c0 + 7 > j)
 #pragma unroll
-          for (int c = c0; c < c0 + 8; c++) a[c] = prf_upd(a[c], l, lds_c(&W.row[c]));
+          for (int c = c0; c < c0 + 8; c++) a[c] = cfms(a[c], l, lds_c(&W.row[c]));
     }
   }
   __syncthreads();
@@ -994,10 +1179,14 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
 // interchanges on the data, one thread per column, was a chain of w dependent
 // round trips (27 us for scattered pivots at N = 4,092).
 #define LSW_WARPS 8
+// On the columns [sol0, sol1) the warp also solves with the unit lower
+// triangle of the panel (lane l holds row k0 + l): the rows of U beside the
+// panel inside its block.
 template <class C>
 __global__ void __launch_bounds__(LSW_WARPS * 32) k_laswp(C *A, size_t ld, const int *ipiv, int k0, int w, int ncols,
-                                                           int skip0, int skip1) {
+                                                           int skip0, int skip1, int sol0, int sol1) {
   __shared__ int src[64], slot[32], rowof[64];
+  __shared__ __align__(16) C L[32][32];   // L[c][r]
   const int tid = threadIdx.x, lane = tid & 31;
   if (tid < 32) {
     const int p = lane < w ? ipiv[k0 + lane] - 1 : -1 - lane;
@@ -1016,6 +1205,14 @@ __global__ void __launch_bounds__(LSW_WARPS * 32) k_laswp(C *A, size_t ld, const
         src[q] = x;
       }
   }
+  // the block's columns are blockIdx.x * LSW_WARPS + warp (+ whole grids)
+  bool solves = false;
+  for (int c = blockIdx.x * LSW_WARPS; c < ncols; c += gridDim.x * LSW_WARPS)
+    solves |= c < sol1 && c + LSW_WARPS > sol0;
+  if (solves) {
+    for (int e = tid; e < w * 32; e += LSW_WARPS * 32)
+      L[e >> 5][lane] = lane > (e >> 5) && lane < w ? A[(size_t)(k0 + (e >> 5)) * ld + k0 + lane] : C{0, 0};
+  }
   __syncthreads();
   // place s takes the entry that was at place src[s]
   const int d0 = rowof[lane], d1 = rowof[32 + lane];
@@ -1023,22 +1220,97 @@ __global__ void __launch_bounds__(LSW_WARPS * 32) k_laswp(C *A, size_t ld, const
   const bool m0 = d0 >= 0 && s0 != d0, m1 = d1 >= 0 && s1 != d1;
   for (int c = blockIdx.x * LSW_WARPS + (tid >> 5); c < ncols; c += gridDim.x * LSW_WARPS) {
     if (c >= skip0 && c < skip1) continue;
+    const bool sol = c >= sol0 && c < sol1;
     C *cp = A + (size_t)c * ld;
-    const C v0 = m0 ? cp[s0] : C{0, 0}, v1 = m1 ? cp[s1] : C{0, 0};
+    C v0 = (m0 || (sol && d0 >= 0)) ? cp[s0] : C{0, 0};
+    const C v1 = m1 ? cp[s1] : C{0, 0};
     __syncwarp();   // every load of the column before its stores
-    if (m0) cp[d0] = v0;
+    if (sol) {
+      for (int i = 0; i < w; i++) v0 = cfms(v0, lds_c(&L[i][lane]), cshfl(v0, i));
+      if (d0 >= 0) cp[d0] = v0;
+    } else if (m0) {
+      cp[d0] = v0;
+    }
     if (m1) cp[d1] = v1;
   }
 }
 
 template <class C>
-static int laswp(bg_matrix *m, int k0, int w) {
+static int laswp(bg_matrix *m, int k0, int w, int blk_end) {
   const int blocks = std::min((m->N + LSW_WARPS - 1) / LSW_WARPS, 148 * 8);
   prof_start(PROF_LASWP);
-  k_laswp<C><<<blocks, LSW_WARPS * 32, 0, stream()>>>((C *)m->d, m->ld, m->d_ipiv, k0, w, m->N, k0, k0 + w);
+  k_laswp<C><<<blocks, LSW_WARPS * 32, 0, stream()>>>((C *)m->d, m->ld, m->d_ipiv, k0, w, m->N, k0, k0 + w, k0 + w,
+                                                       blk_end);
   BG_LAUNCHED();
   prof_stop(PROF_LASWP, 0.0);
   return BG_OK;
+}
+
+// -------------------------------------------------------------------------
+// Update inside a block of LU_BLOCK columns after one of its panels:
+// C (M x nc, nc <= LU_BLOCK - 32) -= L (M x K) U (K x nc), K <= 32, on the
+// FP64 (FP32) pipe, whose rate is that of the FP64 tensor path.  A CTA takes
+// 32 rows, a warp 1/4 of the columns (lane = row): L by rows and U by
+// broadcasts from shared memory, accumulators in registers, C read while the
+// operands are staged with cp.async.  Tensor-core tiles of this shape (K = 32,
+// at most 96 columns) were one launch per level of a deeper recursion.
+// -------------------------------------------------------------------------
+#define LU_BLOCK 128
+template <class C, int NC>
+__global__ void __launch_bounds__(128) k_blk_update(int M, int nc, int K, const C *L, const C *U, C *Cm, size_t ld) {
+  __shared__ __align__(16) C Ls[32][32];   // Ls[k][r]
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C *Us = (C *)smem_raw;                   // Us[c * 32 + k]
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const int r = blockIdx.x * 32 + lane, c0 = wid * NC;
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    const int k = wid + 4 * q;
+    const bool ok = r < M && k < K;
+    cp_entry(&Ls[k][lane], ok ? L + (size_t)k * ld + r : L, ok);
+  }
+#pragma unroll
+  for (int q = 0; q < NC; q++) {
+    const int c = wid + 4 * q;
+    const bool ok = lane < K && c < nc;
+    cp_entry(Us + c * 32 + lane, ok ? U + (size_t)c * ld + lane : U, ok);
+  }
+  cp_commit();
+  C acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; c++) acc[c] = (r < M && c0 + c < nc) ? Cm[(size_t)(c0 + c) * ld + r] : C{0, 0};
+  cp_wait<0>();
+  __syncthreads();
+#pragma unroll 2
+  for (int k = 0; k < 32; k++) {
+    const C l = lds_c(&Ls[k][lane]);
+#pragma unroll
+    for (int c = 0; c < NC; c++) acc[c] = cfms(acc[c], l, lds_c(Us + (c0 + c) * 32 + k));
+  }
+#pragma unroll
+  for (int c = 0; c < NC; c++)
+    if (r < M && c0 + c < nc) Cm[(size_t)(c0 + c) * ld + r] = acc[c];
+}
+template <class C, int NC>
+static int blk_update_launch(int M, int nc, int K, const C *L, const C *U, C *Cm, size_t ld) {
+  const int smem = 32 * 4 * NC * (int)sizeof(C);
+  static bool attr = false;
+  if (!attr) {
+    BG_CUDA_TRY(cudaFuncSetAttribute(k_blk_update<C, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    attr = true;
+  }
+  prof_start(PROF_GEMM);
+  k_blk_update<C, NC><<<(M + 31) / 32, 128, smem, stream()>>>(M, nc, K, L, U, Cm, ld);
+  BG_LAUNCHED();
+  prof_stop(PROF_GEMM, 8.0 * M * (double)nc * K);
+  return BG_OK;
+}
+template <class C>
+static int blk_update(int M, int nc, int K, const C *L, const C *U, C *Cm, size_t ld) {
+  if (M <= 0 || nc <= 0) return BG_OK;
+  return nc > 64   ? blk_update_launch<C, 24>(M, nc, K, L, U, Cm, ld)
+         : nc > 32 ? blk_update_launch<C, 16>(M, nc, K, L, U, Cm, ld)
+                   : blk_update_launch<C, 8>(M, nc, K, L, U, Cm, ld);
 }
 
 struct LUWork {
@@ -1129,7 +1401,7 @@ static int panel_rf_cluster() {
 
 // the panel on one cluster with its rows in registers; *done = false: too tall
 template <class C, int TMAX>
-static int panel_rf(bg_matrix *m, const LUWork &W, int k0, int w, bool *done) {
+static int panel_rf(bg_matrix *m, const LUWork &W, int k0, int w, int blk_end, bool *done) {
   const int N = m->N, Mp = N - k0, RS = panel_rf_cluster<C, TMAX>();
   *done = RS && Mp <= RS * TMAX;
   if (!*done) return BG_OK;
@@ -1154,18 +1426,18 @@ static int panel_rf(bg_matrix *m, const LUWork &W, int k0, int w, bool *done) {
   BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_rf<C, TMAX>, P));
   BG_LAUNCHED();
   prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
-  return laswp<C>(m, k0, w);
+  return laswp<C>(m, k0, w, blk_end);
 }
 
 template <class C>
-static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w) {
+static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w, int blk_end) {
   int N = m->N;
   int Mp = N - k0;
   // rows in the registers of one cluster, while they fit (a row per thread:
   // 4,096 rows of complex128, 8,192 of complex64 with 16 CTAs)
   bool done = false;
-  int st = panel_rf<C, PrfCfg<C>::T0>(m, W, k0, w, &done);
-  if (!st && !done) st = panel_rf<C, PrfCfg<C>::T1>(m, W, k0, w, &done);
+  int st = panel_rf<C, PrfCfg<C>::T0>(m, W, k0, w, blk_end, &done);
+  if (!st && !done) st = panel_rf<C, PrfCfg<C>::T1>(m, W, k0, w, blk_end, &done);
   if (st || done) return st;
   // the whole panel in one cluster's shared memory: cluster barriers and
   // distributed shared memory instead of a grid barrier per column
@@ -1194,7 +1466,7 @@ static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w) {
       BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_cl<C>, P));
       BG_LAUNCHED();
       prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
-      return laswp<C>(m, k0, w);
+      return laswp<C>(m, k0, w, blk_end);
     }
   }
   int G = std::min(panel_grid, std::max(1, (Mp + panel_rows_target - 1) / panel_rows_target));
@@ -1216,20 +1488,32 @@ static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w) {
   BG_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_panel<C>, dim3(G), dim3(256), args, smem, stream()));
   BG_LAUNCHED();
   prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
-  return laswp<C>(m, k0, w);
+  return laswp<C>(m, k0, w, blk_end);
 }
 
-// factor columns [k0, k0+n) (rows k0..N-1); interchanges applied to all columns
+// factor columns [k0, k0+n) (rows k0..N-1); interchanges applied to all columns.
+// Blocks of LU_BLOCK columns are factored right-looking in panels of 32 (three
+// launches a panel: panel, interchanges with the panel's triangular solve
+// inside the block, update of the rest of the block); above them the recursion
+// over column halves keeps the Schur complements large.
 template <class C>
 static int getrf_rec(bg_matrix *m, const LUWork &W, int k0, int n) {
-  if (n <= 32) return panel_leaf<C>(m, W, k0, n);
-  int n1 = (n / 2 + 31) / 32 * 32;
-  if (n1 >= n) n1 = 32;
-  int n2 = n - n1;
   int st;
   C *A = (C *)m->d;
   size_t ld = m->ld;
   int N = m->N;
+  if (n <= LU_BLOCK) {
+    for (int p = k0; p < k0 + n; p += 32) {
+      const int w = std::min(32, k0 + n - p), nc = k0 + n - p - w;
+      if ((st = panel_leaf<C>(m, W, p, w, k0 + n))) return st;
+      if ((st = blk_update<C>(N - p - w, nc, w, A + (p + w) + (size_t)p * ld, A + p + (size_t)(p + w) * ld,
+                              A + (p + w) + (size_t)(p + w) * ld, ld)))
+        return st;
+    }
+    return BG_OK;
+  }
+  int n1 = (n / 2 + LU_BLOCK - 1) / LU_BLOCK * LU_BLOCK;   // < n, as n > LU_BLOCK
+  int n2 = n - n1;
   if ((st = getrf_rec<C>(m, W, k0, n1))) return st;
   C *A11 = A + k0 + (size_t)k0 * ld;
   C *A12 = A + k0 + (size_t)(k0 + n1) * ld;
