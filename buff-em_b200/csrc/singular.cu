@@ -25,16 +25,22 @@
 //    two orders agree to flag_tol of their scale (|M0|, |M0| h, |M0| h^2 for
 //    the zeroth, first and second moments of each kernel, h = diameter of A)
 //    the order n + 2 values are final; otherwise the pair is queued.
-//  * k_sing_refine, persistent, one CTA per queued pair at a time: each face
-//    cube is refined level by level.  Every open box is halved along each of
-//    its dimensions in turn (a 6^{6-c}-point rule per half); the split that
-//    changes the box value most is taken; the box closes when that change is
-//    within tol of the scale (its two halves are kept) or stays open as two
-//    boxes for the next level.  At most SG_MAXBOX boxes are open per level
-//    and SG_MAXLEVEL levels are run; a box that cannot be opened for lack of
-//    room, or is still open after the last level, keeps its halves and sets
+//  * refinement (k_sgr_*): each face cube of a queued pair is refined level by
+//    level, all pairs of a batch together.  Every open box is halved along
+//    each of its dimensions in turn (a 6^{6-c}-point rule per half); the split
+//    that changes the box value most is taken; the box closes when that change
+//    is within tol of the scale (its two halves are kept) or stays open as two
+//    boxes for the next level.  At most SG_MAXBOX boxes of a pair are open per
+//    level and SG_MAXLEVEL levels are run; a box that cannot be opened for lack
+//    of room, or is still open after the last level, keeps its halves and sets
 //    bit 0 / bit 1 of the pair's status (never silently: the bits are OR-ed
 //    into the geometry's status word, bg_geometry_singular_stats).
+// Points are not evaluated one by one: along the last dimension of the rule
+// only one of the two points moves, on a straight line, so a thread takes one
+// line of n points, R = Q + u D, and keeps four sums on it (1/R, u/R, R, u R);
+// the eight raw sums per kernel power follow from them once per line.  About
+// 45 instructions a point in place of 350 (barycentrics, table look-ups and 24
+// accumulations per point).  FP64-pipe bound.
 // With the fixed rule only (bg_geometry_set_singular_refine off) the order n
 // values are kept for every pair, as before refinement existed.
 //
@@ -42,6 +48,7 @@
 // boxes closed in level and box order), so results are deterministic.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -53,9 +60,8 @@ namespace bg {
 #define SG_NG 6            // Gauss points per dimension of a refinement box
 #define SG_MAXBOX 2048     // boxes open per level, at most (per pair)
 #define SG_MAXLEVEL 40
-#define SG_TASKS 256       // half-box evaluations per chunk (their sums live in shared memory)
-#define SG_CHUNK_BOXES 64  // boxes per chunk, at most (SG_TASKS / (2 x 2 dimensions))
-#define SG_REC 33          // doubles per box record: lo[4], hi[4], val[24], S
+#define SG_REC 34          // doubles per box record: lo[4], hi[4], val[24], S, pair slot
+#define SG_RES 48          // doubles per evaluated box: the two halves of the split taken
 
 // Gauss-Legendre rules on [0,1]: row n holds the n-point rule (n <= 16)
 __constant__ double c_sgx[17][16], c_sgw[17][16];
@@ -113,13 +119,18 @@ __device__ __forceinline__ double sel4(const double *a, int i) {
   return i == 0 ? a[0] : i == 1 ? a[1] : i == 2 ? a[2] : a[3];
 }
 
-// collapsed map of u[0..k-1] (k <= 3) onto the k+1 barycentrics of Delta_k;
-// returns the Jacobian (1-u0)^{k-1} (1-u1)^{k-2} ...
-__device__ __forceinline__ double sg_collapse(int k, const double *u, double *b) {
-  double rest = 1.0, J = 1.0;
+// Barycentrics of the collapsed map of u[0..k-1] (k <= 3) onto Delta_k with the
+// Jacobian (1-u0)^{k-1} (1-u1)^{k-2} ...  With line set, the last coordinate is
+// left open: the point is b + u (e_{k-1} - e_k) rest, u in [0, 1].
+__device__ __forceinline__ double sg_collapse(int k, const double *u, double *b, bool line, double &rest) {
+  double J = 1.0;
+  rest = 1.0;
+#pragma unroll
+  for (int i = 0; i < 4; i++) b[i] = 0.0;
+  const int kk = line ? k - 1 : k;
 #pragma unroll
   for (int i = 0; i < 3; i++)
-    if (i < k) {
+    if (i < kk) {
       b[i] = rest * u[i];
       rest *= 1.0 - u[i];
       if (i < k - 1) J *= rest;
@@ -130,56 +141,96 @@ __device__ __forceinline__ double sg_collapse(int k, const double *u, double *b)
   return J;
 }
 
-// One angular point of face S with barycentrics al (A side) and be (B side)
-// and weight w.  The 24 moments are linear in eight raw sums per kernel
-// power R^p (p = -1, 0, 1): sum w R^p, sum w R^p A1, sum w R^p B1,
-// sum w R^p A1.B1 (A1, B1: the points of A and B relative to the first
-// common vertex, which is the origin, so VA[0] = 0), so only those are
-// accumulated per point; sg_raw_to_moments applies the Beta factors and the
-// common-simplex moments once per box.
+// One line of the product rule on face S: the coordinates u[0..K-2] fixed
+// (ka of the K collapsed coordinates map onto A's simplex, the others onto
+// B's; A1, B1: the points of A and B relative to the first common vertex,
+// which is the origin, so VA[0] = 0), the last one over the n Gauss points
+// x of [lo, lo + h] with weights wx.  The 24 moments are linear in eight raw
+// sums per kernel power R^p (p = -1, 0, 1): sum w R^p, sum w R^p A1,
+// sum w R^p B1, sum w R^p A1.B1; sg_raw_to_moment applies the Beta factors and
+// the common-simplex moments once per box.  w: weight of the fixed coordinates.
 template <int C>
-__device__ __forceinline__ void sg_point(const SgPair &X_, int S, const double *al, const double *be, double w,
-                                         double raw[24]) {
-  // read the vertices per point (not hoisted into registers for the whole loop)
-  const volatile SgPair &X = X_;
-  double A1[3] = {0, 0, 0}, B1[3] = {0, 0, 0};
+__device__ __forceinline__ void sg_line(const SgPair &X, int S, int ka, const double *u, double w, int n,
+                                        const double *x, const double *wx, double lo, double h, double raw[24]) {
+  constexpr int K = 6 - C;
+  const int kb = K - ka;
+  const bool varB = kb >= 1;
+  double uA[3], uB[3];
+#pragma unroll
+  for (int e = 0; e < 3; e++) {
+    uA[e] = e < K - 1 ? u[e < K - 1 ? e : 0] : 0.0;
+    double v = 0.0;
+#pragma unroll
+    for (int d = 0; d < K - 1; d++)
+      if (d - ka == e) v = u[d];
+    uB[e] = v;
+  }
+  double al[4], be[4], ra, rb;
+  w *= sg_collapse(ka, uA, al, !varB, ra);
+  w *= sg_collapse(kb, uB, be, varB, rb);
+  // vertices in order: common ones by the sign pattern, then the own ones
+  const int kv = varB ? kb : ka;
+  const double rest = varB ? rb : ra;
+  double A1[3] = {0, 0, 0}, B1[3] = {0, 0, 0}, D[3] = {0, 0, 0};
   int ja = 0, jb = 0;
 #pragma unroll
-  for (int k = 0; k < C; k++) {
-    if ((S >> k) & 1) {
-      double z = sel4(al, ja++);
-      if (k > 0) {
+  for (int k = 0; k < 4; k++) {
+    const bool onA = k < C ? (S >> k) & 1 : true, onB = k < C ? !onA : true;
+    if (onA) {
+      const double z = sel4(al, ja), zd = varB ? 0.0 : (ja == kv - 1 ? rest : (ja == kv ? -rest : 0.0));
+      ja++;
+      if (k > 0)
 #pragma unroll
-        for (int x = 0; x < 3; x++) A1[x] += z * X.VA[k][x];
-      }
-    } else {
-      double z = sel4(be, jb++);
-      if (k > 0) {
+        for (int q = 0; q < 3; q++) {
+          const double P = X.VA[k][q];
+          A1[q] = fma(z, P, A1[q]);
+          D[q] = fma(zd, P, D[q]);
+        }
+    }
+    if (onB) {
+      const double z = sel4(be, jb), zd = varB ? (jb == kv - 1 ? rest : (jb == kv ? -rest : 0.0)) : 0.0;
+      jb++;
+      if (k > 0)
 #pragma unroll
-        for (int x = 0; x < 3; x++) B1[x] += z * X.VA[k][x];
-      }
+        for (int q = 0; q < 3; q++) {
+          const double P = k < C ? X.VA[k][q] : X.VB[k][q];
+          B1[q] = fma(z, P, B1[q]);
+          D[q] = fma(zd, P, D[q]);
+        }
     }
   }
+  // F fixed, V + u D moving
+  double Q[3];
 #pragma unroll
-  for (int k = C; k < 4; k++) {
-    double za = sel4(al, ja++), zb = sel4(be, jb++);
-#pragma unroll
-    for (int x = 0; x < 3; x++) { A1[x] += za * X.VA[k][x]; B1[x] += zb * X.VB[k][x]; }
+  for (int q = 0; q < 3; q++) Q[q] = varB ? B1[q] - A1[q] : A1[q] - B1[q];
+  double T0 = 0, U0 = 0, T2 = 0, U2 = 0;
+#pragma unroll 2
+  for (int i = 0; i < n; i++) {
+    const double uu = fma(h, x[i], lo), wi = wx[i];
+    const double R0 = fma(uu, D[0], Q[0]), R1 = fma(uu, D[1], Q[1]), R2 = fma(uu, D[2], Q[2]);
+    const double r2 = fma(R0, R0, fma(R1, R1, R2 * R2)), ir = rsqrt(r2);
+    const double a = wi * ir, b = a * r2;
+    T0 += a;
+    U0 = fma(a, uu, U0);
+    T2 += b;
+    U2 = fma(b, uu, U2);
   }
-  double L0 = A1[0] - B1[0], L1 = A1[1] - B1[1], L2 = A1[2] - B1[2];
-  double R = sqrt(L0 * L0 + L1 * L1 + L2 * L2);
-  double AB = A1[0] * B1[0] + A1[1] * B1[1] + A1[2] * B1[2];
-  double wp[3] = {w / R, w, w * R};
+  w *= h;
+  // R^0: the rule integrates 1 and u exactly
+  const double T[3] = {w * T0, w, w * T2}, U[3] = {w * U0, w * fma(0.5, h, lo), w * U2};
 #pragma unroll
   for (int pk = 0; pk < 3; pk++) {
-    double t = wp[pk];
-    raw[8 * pk] += t;
+    double ab = 0.0;
+    raw[8 * pk] += T[pk];
 #pragma unroll
-    for (int x = 0; x < 3; x++) {
-      raw[8 * pk + 1 + x] += t * A1[x];
-      raw[8 * pk + 4 + x] += t * B1[x];
+    for (int q = 0; q < 3; q++) {
+      const double F = varB ? A1[q] : B1[q], V = varB ? B1[q] : A1[q];
+      const double Y = fma(T[pk], V, U[pk] * D[q]), TF = T[pk] * F;
+      raw[8 * pk + 1 + q] += varB ? TF : Y;
+      raw[8 * pk + 4 + q] += varB ? Y : TF;
+      ab = fma(F, Y, ab);
     }
-    raw[8 * pk + 7] += t * AB;
+    raw[8 * pk + 7] += ab;
   }
 }
 
@@ -215,39 +266,6 @@ __device__ __forceinline__ void sg_moments_from_raw(const SgPair &X, const doubl
 }
 
 
-// point t (digits of base ng, first dimension least significant) of the
-// ng^k product rule (k = 6 - C) on box [lo, hi] of face S; the first ka
-// collapsed coordinates map onto A's simplex, the next kb onto B's
-template <int C>
-__device__ __forceinline__ void sg_box_point(const SgPair &X, int S, int ka, int ng, const double *lo,
-                                             const double *hi, int t, double raw[24]) {
-  constexpr int K = 6 - C;
-  const int kb = K - ka;
-  double u[K], w = 1.0;
-#pragma unroll
-  for (int d = 0; d < K; d++) {
-    int i = t % ng;
-    t /= ng;
-    u[d] = lo[d] + (hi[d] - lo[d]) * c_sgx[ng][i];
-    w *= (hi[d] - lo[d]) * c_sgw[ng][i];
-  }
-  double uA[3], uB[3];
-#pragma unroll
-  for (int e = 0; e < 3; e++) {
-    uA[e] = e < K ? u[e < K ? e : 0] : 0.0;
-    double v = 0.0;
-#pragma unroll
-    for (int d = 0; d < K; d++)
-      if (d - ka == e) v = u[d];
-    uB[e] = v;
-  }
-  double al[4], be[4];
-  double ja = sg_collapse(ka, uA, al);
-  double jb = sg_collapse(kb, uB, be);
-  w *= ja * jb;
-  sg_point<C>(X, S, al, be, w, raw);
-}
-
 __device__ __forceinline__ int sg_face_S(int c, int f) { return c == 4 ? f + 1 : f; }
 __device__ __forceinline__ int sg_nfaces(int c) { return c == 4 ? 14 : (1 << c); }
 
@@ -276,25 +294,29 @@ __device__ void sg_block_sum(double part[24], double (*red)[24], double *out) {
 
 __constant__ double c_sg_gpre[3] = {0.25 / M_PI, 0.25 / M_PI, 0.125 / M_PI};
 
-// whole-face product rule of order n, points strided over the block (raw sums)
+// whole-face product rule of order n (points x, weights wx of [0, 1] in shared
+// memory), lines strided over the block (raw sums)
 template <int C>
-__device__ void sg_fixed_pass(const SgPair &X, int n, double raw[24]) {
+__device__ void sg_fixed_pass(const SgPair &X, int n, const double *x, const double *wx, double raw[24]) {
   constexpr int nown = 4 - C, K = 6 - C, nf = C == 4 ? 14 : (1 << C);
   int per = 1;
 #pragma unroll
-  for (int i = 0; i < K; i++) per *= n;
+  for (int i = 0; i < K - 1; i++) per *= n;
 #pragma unroll
   for (int i = 0; i < 24; i++) raw[i] = 0.0;
-  const double lo[K] = {}, hi[K] = {};
-  double one[K];
-#pragma unroll
-  for (int d = 0; d < K; d++) one[d] = 1.0;
-  (void)hi;
 #pragma unroll 1
   for (int f = threadIdx.x; f < nf * per; f += SG_THREADS) {
     int face = f / per, t = f - face * per;
     int S = sg_face_S(C, face), ns = __popc(S);
-    sg_box_point<C>(X, S, ns + nown - 1, n, lo, one, t, raw);
+    double u[K], w = 1.0;
+#pragma unroll
+    for (int d = 0; d < K - 1; d++) {
+      const int q = t / n, i = t - q * n;
+      t = q;
+      u[d] = x[i];
+      w *= wx[i];
+    }
+    sg_line<C>(X, S, ns + nown - 1, u, w, n, x, wx, 0.0, 1.0, raw);
   }
 }
 
@@ -322,16 +344,15 @@ struct SgLists {
   int *cnt;         // 3 counters
   int start[3];
   unsigned char *flag;   // per singular pair: bit 0 flagged, bits 1-2 refinement status
-  int *work;        // work counter of the refinement kernel
   unsigned int *status;
-  unsigned long long *evals;
 };
 
 template <int C>
 __device__ void sg_fixed_pair(const SgPair &X, int pidx, int first, double *mom, int n, int refine,
-                              double flag_tol, const SgLists &L, double (*red)[24], double *f0, double *f1) {
+                              double flag_tol, const SgLists &L, const double (*tab)[16], double (*red)[24],
+                              double *f0, double *f1) {
   double part[24];
-  sg_fixed_pass<C>(X, n, part);
+  sg_fixed_pass<C>(X, n, tab[0], tab[1], part);
   sg_block_sum(part, red, f1);
   if (threadIdx.x < 24) f0[threadIdx.x] = sg_raw_to_moment(X, f1, threadIdx.x) * c_sg_gpre[threadIdx.x / 8];
   __syncthreads();
@@ -339,7 +360,7 @@ __device__ void sg_fixed_pair(const SgPair &X, int pidx, int first, double *mom,
     if (threadIdx.x < 24) mom[24 * (size_t)pidx + threadIdx.x] = f0[threadIdx.x];
     return;
   }
-  sg_fixed_pass<C>(X, n + 2, part);
+  sg_fixed_pass<C>(X, n + 2, tab[2], tab[3], part);
   sg_block_sum(part, red, f1);
   double m1 = threadIdx.x < 24 ? sg_raw_to_moment(X, f1, threadIdx.x) * c_sg_gpre[threadIdx.x / 8] : 0.0;
   __syncthreads();
@@ -365,243 +386,383 @@ __global__ void __launch_bounds__(SG_THREADS, 2) k_sing_fixed(DevGeom g, const i
                                                               int refine, double flag_tol, SgLists L) {
   __shared__ SgPair X;
   __shared__ double red[SG_THREADS / 32][24];
-  __shared__ double f0[24], f1[24];
+  __shared__ double f0[24], f1[24], tab[4][16];   // points and weights of orders n and n + 2
   const int pidx = first + blockIdx.x;
+  if (threadIdx.x < 64) {
+    const int r = threadIdx.x >> 4, i = threadIdx.x & 15, o = r < 2 ? n : min(n + 2, 16);
+    tab[r][i] = r & 1 ? c_sgw[o][i] : c_sgx[o][i];
+  }
   if (threadIdx.x == 0) sg_setup(g, ordA[pidx], ordB[pidx], tp[pidx].z, X);
   __syncthreads();
   switch (X.c) {
-    case 2: sg_fixed_pair<2>(X, pidx, first, mom, n, refine, flag_tol, L, red, f0, f1); break;
-    case 3: sg_fixed_pair<3>(X, pidx, first, mom, n, refine, flag_tol, L, red, f0, f1); break;
-    default: sg_fixed_pair<4>(X, pidx, first, mom, n, refine, flag_tol, L, red, f0, f1); break;
+    case 2: sg_fixed_pair<2>(X, pidx, first, mom, n, refine, flag_tol, L, tab, red, f0, f1); break;
+    case 3: sg_fixed_pair<3>(X, pidx, first, mom, n, refine, flag_tol, L, tab, red, f0, f1); break;
+    default: sg_fixed_pair<4>(X, pidx, first, mom, n, refine, flag_tol, L, tab, red, f0, f1); break;
   }
 }
 
-// shared state of the refinement kernel
-struct SgShared {
+// ------------------------------------------------------------- refinement
+// A batch of flagged pairs of one class, all levels together: box lists in
+// HBM, the boxes of a pair contiguous and in order.  Per level: k_sgr_eval
+// evaluates the 2K halves of every box and decides, k_sgr_count and
+// k_sgr_scan place every pair's children, k_sgr_next writes them in order and
+// adds the closed boxes to the pair's moments, in level and box order.  One
+// CTA per pair left the pairs with many levels running alone, at 9.6 % FP64-pipe
+// activity.  Jittered sphere, N = 5,760: refinement 201 -> 54 ms, the fixed
+// passes 55 -> 13.7 ms.
+struct SgrPair {
   SgPair X;
   double scale[24], acc[24];
-  double blo[SG_CHUNK_BOXES][4], bhi[SG_CHUNK_BOXES][4];
-  int bS[SG_CHUNK_BOXES], bd[SG_CHUNK_BOXES], bopen[SG_CHUNK_BOXES], bpos[SG_CHUNK_BOXES];
-  double tb[SG_THREADS / 4][8];   // per lane group: the bounds (lo, hi) of its current task
-  int pidx, nn, status;
-  unsigned long long evals;
+  int pidx, status;
+  int beg, n;              // its boxes of this level
+  int nopen, nbeg;         // open ones (children / 2), first child
 };
 
-// Evaluates ntasks boxes of the chunk into sres (24 moments each, unit
-// measure, no kernel prefactor).  split: task t is box t / 2K halved along
-// dimension (t % 2K) / 2, half t % 2; otherwise task t is box t whole.
-// G lanes share a task (a fixed shuffle tree sums their points).
-template <int C>
-__device__ void sg_eval_tasks(SgShared &sh, double *sres, int ntasks, bool split) {
+struct SgrBatch {
+  SgrPair *pair;
+  double *cur, *nxt, *res;       // SG_REC, SG_REC, SG_RES doubles per box
+  int *open;                     // per box: split dimension of an open box, -1 closed; closed ones in cd
+  int *cd;                       // split dimension taken
+  int *total;                    // boxes of the next level
+  int np, cap;
+};
+
+__global__ void k_sgr_setup(DevGeom g, const int4 *tp, const int4 *ordA, const int4 *ordB, const double *mom,
+                            const int *list, SgrBatch B, int nf) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= B.np) return;
+  SgrPair &Q = B.pair[p];
+  const int pidx = list[p];
+  SgPair X;
+  sg_setup(g, ordA[pidx], ordB[pidx], tp[pidx].z, X);
+  Q.X = X;
+  double f1[24], scale[24];
+  for (int i = 0; i < 24; i++) f1[i] = mom[24 * (size_t)pidx + i];
+  sg_scales(X, f1, scale);
+  for (int i = 0; i < 24; i++) { Q.scale[i] = scale[i]; Q.acc[i] = 0.0; }
+  Q.pidx = pidx;
+  Q.status = 0;
+  Q.beg = p * nf;
+  Q.n = nf;
+}
+
+// Moments of one task (a box): its lines over the G lanes of a group, a fixed
+// shuffle tree, the result in every lane of the group
+template <int C, int G>
+__device__ __forceinline__ void sgr_task(const SgPair &X, int S, const double *lo, const double *hi, int gl,
+                                         const double *x, const double *wx, double out[24]) {
   constexpr int K = 6 - C, nown = 4 - C;
-  constexpr int G = C == 2 ? 32 : C == 3 ? 8 : 4;
-  constexpr int P = SG_NG * SG_NG * (K > 2 ? SG_NG : 1) * (K > 3 ? SG_NG : 1);
-  const int gl = threadIdx.x % G, grp = threadIdx.x / G;
-  constexpr int ngrp = SG_THREADS / G;
-  for (int base = 0; base < ntasks; base += ngrp) {
-    int t = base + grp;
-    double part[24];
+  constexpr int LN = SG_NG * (K > 2 ? SG_NG : 1) * (K > 3 ? SG_NG : 1);   // lines: 6^{K-1}
+  const int ka = __popc(S) + nown - 1;
+  double raw[24];
 #pragma unroll
-    for (int i = 0; i < 24; i++) part[i] = 0.0;
-    int j = split ? t / (2 * K) : t;
-    __syncwarp();   // the group's previous task has finished reading its bounds
-    if (t < ntasks && gl == 0) {
-      int sd = split ? (t % (2 * K)) / 2 : -1, h = t & 1;
-#pragma unroll
-      for (int d = 0; d < 4; d++) {
-        double lo = sh.blo[j][d], hi = sh.bhi[j][d];
-        if (d == sd) {
-          double mid = 0.5 * (lo + hi);
-          if (h == 0) hi = mid; else lo = mid;
-        }
-        sh.tb[grp][d] = lo;
-        sh.tb[grp][4 + d] = hi;
-      }
-    }
-    __syncwarp();
-    if (t < ntasks) {
-      int S = sh.bS[j], ns = __popc(S);
-      // bounds read per point from shared memory (keeps registers for the point)
-      const volatile double *tb = sh.tb[grp];
+  for (int i = 0; i < 24; i++) raw[i] = 0.0;
 #pragma unroll 1
-      for (int p = gl; p < P; p += G) {
-        double lo[K], hi[K];
+  for (int t0 = gl; t0 < LN; t0 += G) {
+    int t = t0;
+    double u[K], w = 1.0;
 #pragma unroll
-        for (int d = 0; d < K; d++) { lo[d] = tb[d]; hi[d] = tb[4 + d]; }
-        sg_box_point<C>(sh.X, S, ns + nown - 1, SG_NG, lo, hi, p, part);
+    for (int d = 0; d < K - 1; d++) {
+      const int i = t % SG_NG;
+      t /= SG_NG;
+      const double h = hi[d] - lo[d];
+      u[d] = fma(h, x[i], lo[d]);
+      w *= h * wx[i];
+    }
+    sg_line<C>(X, S, ka, u, w, SG_NG, x, wx, lo[K - 1], hi[K - 1] - lo[K - 1], raw);
+  }
+#pragma unroll
+  for (int i = 0; i < 24; i++)
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) raw[i] += __shfl_xor_sync(0xffffffffu, raw[i], o);
+  sg_moments_from_raw(X, raw, out);
+}
+
+template <int C> struct SgrCfg;
+template <> struct SgrCfg<2> { static constexpr int G = 32, NB = 1; };    // 8 halves a box: 256 lanes
+template <> struct SgrCfg<3> { static constexpr int G = 4, NB = 10; };    // 6 halves: 24 lanes
+template <> struct SgrCfg<4> { static constexpr int G = 2, NB = 32; };    // 4 halves: 8 lanes
+
+// level 0: the whole face cubes of every pair
+template <int C>
+__global__ void __launch_bounds__(SG_THREADS) k_sgr_init(SgrBatch B) {
+  constexpr int K = 6 - C, nf = C == 4 ? 14 : (1 << C), G = SgrCfg<C>::G, NT = SG_THREADS / G;
+  __shared__ double tx[SG_NG], tw[SG_NG];
+  if (threadIdx.x < SG_NG) { tx[threadIdx.x] = c_sgx[SG_NG][threadIdx.x]; tw[threadIdx.x] = c_sgw[SG_NG][threadIdx.x]; }
+  __syncthreads();
+  const int gl = threadIdx.x % G, grp = threadIdx.x / G, total = B.np * nf;
+  for (int base = blockIdx.x * NT; base < total; base += gridDim.x * NT) {
+    const int b = min(base + grp, total - 1);      // idle groups repeat the last box
+    const int p = b / nf, S = sg_face_S(C, b - p * nf);
+    double lo[4] = {0, 0, 0, 0}, hi[4] = {1, 1, 1, 1}, m[24];
+    sgr_task<C, G>(B.pair[p].X, S, lo, hi, gl, tx, tw, m);
+    if (gl == 0 && base + grp < total) {
+      double *r = B.cur + (size_t)b * SG_REC;
+      for (int d = 0; d < 4; d++) { r[d] = 0.0; r[4 + d] = 1.0; }
+#pragma unroll
+      for (int i = 0; i < 24; i++) r[8 + i] = m[i];
+      r[32] = (double)S;
+      r[33] = (double)p;
+    }
+  }
+  (void)K;
+}
+
+// halves of every box, the split that changes it most, open or closed
+template <int C>
+__global__ void __launch_bounds__(SG_THREADS, 2) k_sgr_eval(SgrBatch B, int nbox, double tol) {
+  constexpr int K = 6 - C, G = SgrCfg<C>::G, NB = SgrCfg<C>::NB, LB = 2 * K * G;   // lanes per box
+  extern __shared__ __align__(16) double sm[];
+  double *sres = sm;                             // NB x 2K x 24 moments
+  double *sbox = sres + NB * 2 * K * 24;         // NB x SG_REC
+  double *serr = sbox + NB * SG_REC;             // NB x K
+  SgPair *sX = (SgPair *)(serr + NB * K);        // NB pairs
+  __shared__ double tx[SG_NG], tw[SG_NG];
+  __shared__ int sd[NB];
+  const int tid = threadIdx.x;
+  if (tid < SG_NG) { tx[tid] = c_sgx[SG_NG][tid]; tw[tid] = c_sgw[SG_NG][tid]; }
+  for (int base = blockIdx.x * NB; base < nbox; base += gridDim.x * NB) {
+    const int nb = min(NB, nbox - base);
+    __syncthreads();
+    for (int e = tid; e < nb * SG_REC; e += SG_THREADS) sbox[e] = B.cur[(size_t)base * SG_REC + e];
+    constexpr int XD = sizeof(SgPair) / 8;
+    __syncthreads();
+    for (int e = tid; e < nb * XD; e += SG_THREADS) {
+      const int j = e / XD;
+      ((double *)&sX[j])[e - j * XD] = ((const double *)&B.pair[(int)sbox[j * SG_REC + 33]].X)[e - j * XD];
+    }
+    __syncthreads();
+    {
+      // lanes past the last box repeat it (the shuffles need whole warps)
+      const int jb = tid / LB, j = min(jb, nb - 1), task = (tid % LB) / G, gl = tid % G;
+      const double *r = sbox + j * SG_REC;
+      const int sdim = task >> 1;
+      double lo[K], hi[K];
+#pragma unroll
+      for (int d = 0; d < K; d++) {
+        lo[d] = r[d];
+        hi[d] = r[4 + d];
+        if (d == sdim) {
+          const double mid = 0.5 * (lo[d] + hi[d]);
+          if (task & 1) lo[d] = mid; else hi[d] = mid;
+        }
+      }
+      double m[24];
+      sgr_task<C, G>(sX[j], (int)r[32], lo, hi, gl, tx, tw, m);
+      if (gl == 0 && jb < nb)
+#pragma unroll
+        for (int i = 0; i < 24; i++) sres[(j * 2 * K + task) * 24 + i] = m[i];
+    }
+    __syncthreads();
+    if (tid < nb * K) {
+      const int j = tid / K, d = tid - j * K;
+      const double *v0 = sres + (j * 2 * K + 2 * d) * 24, *v1 = v0 + 24, *val = sbox + j * SG_REC + 8;
+      const double *scale = B.pair[(int)sbox[j * SG_REC + 33]].scale;
+      double e = 0.0;
+      for (int i = 0; i < 24; i++) e = fmax(e, fabs(v0[i] + v1[i] - val[i]) / scale[i]);
+      serr[tid] = e;
+    }
+    __syncthreads();
+    if (tid < nb) {
+      double best = -1.0;
+      int bd = 0;
+      for (int d = 0; d < K; d++)
+        if (serr[tid * K + d] > best) { best = serr[tid * K + d]; bd = d; }
+      sd[tid] = bd;
+      B.cd[base + tid] = bd;
+      B.open[base + tid] = best > tol;
+    }
+    __syncthreads();
+    for (int e = tid; e < nb * SG_RES; e += SG_THREADS) {
+      const int j = e / SG_RES, f = e - j * SG_RES;
+      B.res[(size_t)(base + j) * SG_RES + f] = sres[(j * 2 * K + 2 * sd[j]) * 24 + f];
+    }
+  }
+}
+
+// open boxes of every pair, in order up to the limits
+__global__ void k_sgr_count(SgrBatch B, int last) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= B.np) return;
+  SgrPair &Q = B.pair[p];
+  int n = 0, status = 0;
+  for (int b = Q.beg; b < Q.beg + Q.n; b++)
+    if (B.open[b]) {
+      if (2 * n + 2 > SG_MAXBOX) { status |= 1; B.open[b] = 0; }
+      else if (last) { status |= 2; B.open[b] = 0; }
+      else n++;
+    }
+  Q.nopen = n;
+  Q.status |= status;
+}
+
+__global__ void __launch_bounds__(1024) k_sgr_scan(SgrBatch B) {
+  __shared__ int wsum[32], carry;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid == 0) carry = 0;
+  __syncthreads();
+  for (int base = 0; base < B.np; base += 1024) {
+    const int p = base + tid, v = p < B.np ? 2 * B.pair[p].nopen : 0;
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[wid] = x;
+    __syncthreads();
+    if (wid == 0) {
+      int s = wsum[lane];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, s, o);
+        if (lane >= o) s += y;
+      }
+      wsum[lane] = s;
+    }
+    __syncthreads();
+    if (p < B.np) B.pair[p].nbeg = carry + (wid ? wsum[wid - 1] : 0) + x - v;
+    __syncthreads();
+    if (tid == 0) carry += wsum[31];
+    __syncthreads();
+  }
+  if (tid == 0) *B.total = carry;
+}
+
+// children and closed sums of every pair, one warp per pair, in box order
+__global__ void __launch_bounds__(256) k_sgr_next(SgrBatch B) {
+  const int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (p >= B.np) return;
+  SgrPair &Q = B.pair[p];
+  if (*B.total > B.cap) return;          // the host splits the batch
+  double a = lane < 24 ? Q.acc[lane] : 0.0;
+  int pos = Q.nbeg;
+  const int beg = Q.beg, n = Q.n;
+  // the flags of 32 boxes at a time; the loads of the boxes do not depend on
+  // one another
+  for (int b0 = beg; b0 < beg + n; b0 += 32) {
+    const int nb = min(32, beg + n - b0);
+    const unsigned op = __ballot_sync(0xffffffffu, lane < nb && __ldg(B.open + b0 + lane));
+    const int cd = lane < nb ? __ldg(B.cd + b0 + lane) : 0;
+#pragma unroll 4
+    for (int j = 0; j < nb; j++) {
+      const double *v = B.res + (size_t)(b0 + j) * SG_RES, *r = B.cur + (size_t)(b0 + j) * SG_REC;
+      const int d = __shfl_sync(0xffffffffu, cd, j);
+      if (!(op >> j & 1)) {
+        if (lane < 24) a += __ldg(v + lane) + __ldg(v + 24 + lane);
+        continue;
+      }
+      const int at = pos + 2 * __popc(op & ((1u << j) - 1));
+      const double mid = 0.5 * (__ldg(r + d) + __ldg(r + 4 + d));
+#pragma unroll
+      for (int e0 = 0; e0 < 96; e0 += 32) {
+        const int e = e0 + lane, h = e / SG_REC, f = e - h * SG_REC;
+        if (e >= 2 * SG_REC) break;
+        double x = f < 8 || f >= 32 ? __ldg(r + f) : __ldg(v + 24 * h + f - 8);
+        if (h == 0 && f == 4 + d) x = mid;
+        if (h == 1 && f == d) x = mid;
+        B.nxt[(size_t)(at + h) * SG_REC + f] = x;
       }
     }
-#pragma unroll
-    for (int i = 0; i < 24; i++) {
-      double v = part[i];
-#pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      part[i] = v;
-    }
-    if (t < ntasks && gl == 0) {
-#pragma unroll
-      for (int i = 0; i < 24; i++) sres[24 * t + i] = part[i];
-    }
+    pos += 2 * __popc(op);
   }
-  // raw sums -> moments, one thread per task
-  __syncthreads();
-  for (int t = threadIdx.x; t < ntasks; t += SG_THREADS) {
-    double r[24], m[24];
-#pragma unroll
-    for (int i = 0; i < 24; i++) r[i] = sres[24 * t + i];
-    sg_moments_from_raw(sh.X, r, m);
-#pragma unroll
-    for (int i = 0; i < 24; i++) sres[24 * t + i] = m[i];
-  }
+  if (lane < 24) Q.acc[lane] = a;
+  if (lane == 0) { Q.beg = Q.nbeg; Q.n = 2 * Q.nopen; }
+}
+
+__global__ void k_sgr_store(SgrBatch B, int first, double *mom, SgLists L) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= B.np) return;
+  const SgrPair &Q = B.pair[p];
+  for (int i = 0; i < 24; i++) mom[24 * (size_t)Q.pidx + i] = Q.acc[i] * c_sg_gpre[i / 8];
+  L.flag[Q.pidx - first] |= (unsigned char)(Q.status << 1);
+  if (Q.status) atomicOr(L.status, (unsigned int)Q.status);
 }
 
 template <int C>
-__device__ void sg_refine_pair(SgShared &sh, double *sres, double *cur, double *nxt, double tol) {
-  constexpr int K = 6 - C, nf = C == 4 ? 14 : (1 << C);
-  constexpr int P = SG_NG * SG_NG * (K > 2 ? SG_NG : 1) * (K > 3 ? SG_NG : 1);
-  constexpr int CB = SG_TASKS / (2 * K);
-  // level 0 boxes: the whole face cubes
-  if (threadIdx.x < nf) {
-    sh.bS[threadIdx.x] = sg_face_S(C, threadIdx.x);
-    for (int d = 0; d < 4; d++) { sh.blo[threadIdx.x][d] = 0.0; sh.bhi[threadIdx.x][d] = 1.0; }
-  }
-  __syncthreads();
-  sg_eval_tasks<C>(sh, sres, nf, false);
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < nf * SG_REC; idx += SG_THREADS) {
-    int j = idx / SG_REC, f = idx % SG_REC;
-    double v = f < 4 ? 0.0 : f < 8 ? 1.0 : f < 32 ? sres[24 * j + f - 8] : (double)sh.bS[j];
-    cur[(size_t)j * SG_REC + f] = v;
-  }
-  if (threadIdx.x == 0) sh.evals += (unsigned long long)nf * P;
-  __syncthreads();
-  int ncur = nf;
-  for (int level = 0; level < SG_MAXLEVEL && ncur > 0; level++) {
-    if (threadIdx.x == 0) sh.nn = 0;
-    for (int cb = 0; cb < ncur; cb += CB) {
-      const int nb = min(CB, ncur - cb);
-      for (int idx = threadIdx.x; idx < nb * 9; idx += SG_THREADS) {
-        int j = idx / 9, f = idx % 9;
-        const double *r = cur + (size_t)(cb + j) * SG_REC;
-        if (f < 4) sh.blo[j][f] = r[f];
-        else if (f < 8) sh.bhi[j][f - 4] = r[f];
-        else sh.bS[j] = (int)r[32];
-      }
-      __syncthreads();
-      sg_eval_tasks<C>(sh, sres, nb * 2 * K, true);
-      __syncthreads();
-      // the split that changes each box most, and whether it stays open
-      if (threadIdx.x < nb) {
-        int j = threadIdx.x;
-        const double *val = cur + (size_t)(cb + j) * SG_REC + 8;
-        double best = -1.0;
-        int bestd = 0;
-        for (int d = 0; d < K; d++) {
-          const double *v0 = sres + 24 * (j * 2 * K + 2 * d), *v1 = v0 + 24;
-          double e = 0.0;
-          for (int i = 0; i < 24; i++) e = fmax(e, fabs(v0[i] + v1[i] - val[i]) / sh.scale[i]);
-          if (e > best) { best = e; bestd = d; }
-        }
-        sh.bd[j] = bestd;
-        sh.bopen[j] = best > tol;
-      }
-      __syncthreads();
-      // positions of the opened boxes in the next level, in box order
-      if (threadIdx.x == 0) {
-        int nn = sh.nn;
-        for (int j = 0; j < nb; j++) {
-          if (!sh.bopen[j]) continue;
-          if (nn + 2 > SG_MAXBOX) { sh.bopen[j] = 0; sh.status |= 1; continue; }
-          if (level == SG_MAXLEVEL - 1) { sh.bopen[j] = 0; sh.status |= 2; continue; }
-          sh.bpos[j] = nn;
-          nn += 2;
-        }
-        sh.nn = nn;
-        sh.evals += (unsigned long long)nb * 2 * K * P;
-      }
-      __syncthreads();
-      for (int idx = threadIdx.x; idx < nb * 2 * SG_REC; idx += SG_THREADS) {
-        int j = idx / (2 * SG_REC), r = idx % (2 * SG_REC), h = r / SG_REC, f = r % SG_REC;
-        if (!sh.bopen[j]) continue;
-        int d = sh.bd[j];
-        double v;
-        if (f < 8) {
-          int dd = f & 3;
-          double lo = sh.blo[j][dd], hi = sh.bhi[j][dd];
-          if (dd == d) {
-            double mid = 0.5 * (lo + hi);
-            if (h == 0) hi = mid; else lo = mid;
-          }
-          v = f < 4 ? lo : hi;
-        } else if (f < 32) {
-          v = sres[24 * (j * 2 * K + 2 * d + h) + f - 8];
-        } else {
-          v = (double)sh.bS[j];
-        }
-        nxt[(size_t)(sh.bpos[j] + h) * SG_REC + f] = v;
-      }
-      if (threadIdx.x < 24) {
-        double a = sh.acc[threadIdx.x];
-        for (int j = 0; j < nb; j++) {
-          if (sh.bopen[j]) continue;
-          const double *v0 = sres + 24 * (j * 2 * K + 2 * sh.bd[j]);
-          a += v0[threadIdx.x] + v0[24 + threadIdx.x];
-        }
-        sh.acc[threadIdx.x] = a;
-      }
-      __syncthreads();
-    }
-    double *t = cur;
-    cur = nxt;
-    nxt = t;
-    ncur = sh.nn;
-    __syncthreads();
-  }
+static int sgr_smem() {
+  constexpr int K = 6 - C, NB = SgrCfg<C>::NB;
+  return (int)(sizeof(double) * (NB * 2 * K * 24 + NB * SG_REC + NB * K) + NB * sizeof(SgPair));
 }
 
-// Refinement of the flagged pairs; pool: 2 x SG_MAXBOX box records per CTA.
-__global__ void __launch_bounds__(SG_THREADS, 1) k_sing_refine(DevGeom g, const int4 *tp, const int4 *ordA,
-                                                               const int4 *ordB, int first, double *mom, double tol,
-                                                               double *pool, SgLists L) {
-  extern __shared__ double sres[];   // SG_TASKS x 24 half-box moments
-  __shared__ SgShared sh;
-  double *cur = pool + (size_t)blockIdx.x * 2 * SG_MAXBOX * SG_REC;
-  double *nxt = cur + (size_t)SG_MAXBOX * SG_REC;
-  const int total = L.cnt[0] + L.cnt[1] + L.cnt[2];
-  for (;;) {
-    if (threadIdx.x == 0) {
-      int w = atomicAdd(L.work, 1);
-      int pidx = -1;
-      if (w < L.cnt[0]) pidx = L.list[L.start[0] + w];
-      else if (w < L.cnt[0] + L.cnt[1]) pidx = L.list[L.start[1] + w - L.cnt[0]];
-      else if (w < total) pidx = L.list[L.start[2] + w - L.cnt[0] - L.cnt[1]];
-      sh.pidx = pidx;
-      if (pidx >= 0) {
-        sg_setup(g, ordA[pidx], ordB[pidx], tp[pidx].z, sh.X);
-        double f1[24];
-        for (int i = 0; i < 24; i++) f1[i] = mom[24 * (size_t)pidx + i];
-        sg_scales(sh.X, f1, sh.scale);
-      }
-      sh.status = 0;
-      sh.evals = 0;
-    }
-    if (threadIdx.x < 24) sh.acc[threadIdx.x] = 0.0;
-    __syncthreads();
-    const int pidx = sh.pidx;
-    if (pidx < 0) return;
-    switch (sh.X.c) {
-      case 2: sg_refine_pair<2>(sh, sres, cur, nxt, tol); break;
-      case 3: sg_refine_pair<3>(sh, sres, cur, nxt, tol); break;
-      default: sg_refine_pair<4>(sh, sres, cur, nxt, tol); break;
-    }
-    if (threadIdx.x < 24) mom[24 * (size_t)pidx + threadIdx.x] = sh.acc[threadIdx.x] * c_sg_gpre[threadIdx.x / 8];
-    if (threadIdx.x == 0) {
-      L.flag[pidx - first] |= (unsigned char)(sh.status << 1);
-      if (sh.status) atomicOr(L.status, (unsigned int)sh.status);
-      atomicAdd(L.evals, sh.evals);
-    }
-    __syncthreads();
+// refines list[0 .. np); halves the batch while its boxes outgrow the lists
+template <int C>
+static int sgr_run(bg_geometry *g, const int *list, int np, SgrBatch B, const SgLists &L, long long *evals) {
+  NearData &nd = g->near;
+  constexpr int K = 6 - C, nf = C == 4 ? 14 : (1 << C), NB = SgrCfg<C>::NB;
+  constexpr long long P = (long long)SG_NG * SG_NG * (K > 2 ? SG_NG : 1) * (K > 3 ? SG_NG : 1);
+  static bool attr = false;
+  if (!attr) {
+    BG_CUDA_TRY(cudaFuncSetAttribute(k_sgr_eval<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, sgr_smem<C>()));
+    attr = true;
   }
+  B.np = np;
+  const int pb = (np + 127) / 128;
+  k_sgr_setup<<<pb, 128, 0, stream()>>>(g->dev, nd.tp, nd.tpOrdA, nd.tpOrdB, nd.tpMom, list, B, nf);
+  BG_LAUNCHED();
+  const int grid = 148 * 4;
+  constexpr int NT = SG_THREADS / SgrCfg<C>::G;
+  k_sgr_init<C><<<std::min(grid, (np * nf + NT - 1) / NT), SG_THREADS, 0, stream()>>>(B);
+  BG_LAUNCHED();
+  long long ev = (long long)np * nf * P;
+  int nbox = np * nf;
+  for (int level = 0; level < SG_MAXLEVEL && nbox > 0; level++) {
+    k_sgr_eval<C><<<std::min(grid, (nbox + NB - 1) / NB), SG_THREADS, sgr_smem<C>(), stream()>>>(B, nbox, g->sing_tol);
+    BG_LAUNCHED();
+    ev += (long long)nbox * 2 * K * P;
+    k_sgr_count<<<pb, 128, 0, stream()>>>(B, level == SG_MAXLEVEL - 1);
+    BG_LAUNCHED();
+    k_sgr_scan<<<1, 1024, 0, stream()>>>(B);
+    BG_LAUNCHED();
+    k_sgr_next<<<(np + 7) / 8, 256, 0, stream()>>>(B);
+    BG_LAUNCHED();
+    BG_CUDA_TRY(cudaMemcpyAsync(&nbox, B.total, sizeof(int), cudaMemcpyDeviceToHost, stream()));
+    BG_CUDA_TRY(cudaStreamSynchronize(stream()));
+    if (nbox > B.cap) {
+      const int h = np / 2;              // one pair holds at most SG_MAXBOX <= cap boxes
+      int st = sgr_run<C>(g, list, h, B, L, evals);
+      return st ? st : sgr_run<C>(g, list + h, np - h, B, L, evals);
+    }
+    std::swap(B.cur, B.nxt);
+  }
+  k_sgr_store<<<pb, 128, 0, stream()>>>(B, nd.ntp_reg, nd.tpMom, L);
+  BG_LAUNCHED();
+  *evals += ev;
+  return BG_OK;
+}
+
+// all flagged pairs of the three classes, in batches
+static int sgr_refine(bg_geometry *g, const SgLists &L, const int cnt[3], long long *evals) {
+  const int most = std::max(cnt[0], std::max(cnt[1], cnt[2]));
+  if (most <= 0) return BG_OK;
+  // 32 boxes a pair on average (8-14 start, about 30 at the widest level)
+  const int batch = std::min(most, 8192);
+  SgrBatch B{};
+  B.cap = std::max(2 * SG_MAXBOX, 32 * batch);
+  const size_t nb = (size_t)B.cap;
+  const size_t bytes = sizeof(double) * nb * (2 * SG_REC + SG_RES) + sizeof(SgrPair) * (size_t)batch + 2 * sizeof(int) * nb + 64;
+  char *blk = nullptr;
+  if (cudaMallocAsync((void **)&blk, bytes, stream()) != cudaSuccess) {
+    cudaGetLastError();
+    set_error("singular near-field precompute: cannot allocate the refinement box lists");
+    return BG_ERR_NOMEM;
+  }
+  char *q = blk;
+  B.cur = (double *)q; q += sizeof(double) * nb * SG_REC;
+  B.nxt = (double *)q; q += sizeof(double) * nb * SG_REC;
+  B.res = (double *)q; q += sizeof(double) * nb * SG_RES;
+  B.pair = (SgrPair *)q; q += sizeof(SgrPair) * (size_t)batch;
+  B.open = (int *)q; q += sizeof(int) * nb;
+  B.cd = (int *)q; q += sizeof(int) * nb;
+  B.total = (int *)q;
+  int st = BG_OK;
+  for (int cls = 0; cls < 3 && !st; cls++)
+    for (int b = 0; b < cnt[cls] && !st; b += batch) {
+      const int n = std::min(batch, cnt[cls] - b);
+      const int *list = L.list + L.start[cls] + b;
+      st = cls == 0 ? sgr_run<2>(g, list, n, B, L, evals)
+         : cls == 1 ? sgr_run<3>(g, list, n, B, L, evals) : sgr_run<4>(g, list, n, B, L, evals);
+    }
+  cudaFreeAsync(blk, stream());
+  return st;
 }
 
 // Singular pairs of the near table: [ntp_reg, ntp), sorted by class (2, 3, 4
@@ -625,53 +786,38 @@ int singular_precompute(bg_geometry *g) {
   }
   g->sing_stats[0] = nsing;
   g->sing_stats[2] = fixed_pts;
-  // small device block: counters (3), work counter, status, evals, then the
-  // list and the per-pair flags
+  // small device block: counters (3), status, then the list and the per-pair
+  // flags
   size_t hdr = 64, bytes = hdr + sizeof(int) * (size_t)nsing + (size_t)nsing;
   char *blk = nullptr;
   BG_CUDA_TRY(cudaMallocAsync((void **)&blk, bytes, stream()));
   SgLists L;
   L.cnt = (int *)blk;
-  L.work = (int *)(blk + 16);
-  L.status = (unsigned int *)(blk + 20);
-  L.evals = (unsigned long long *)(blk + 24);
+  L.status = (unsigned int *)(blk + 16);
   L.list = (int *)(blk + hdr);
   L.flag = (unsigned char *)(blk + hdr + sizeof(int) * (size_t)nsing);
   L.start[0] = 0;
   L.start[1] = nd.nsing_c[0];
   L.start[2] = nd.nsing_c[0] + nd.nsing_c[1];
   int rc = BG_OK;
-  double *pool = nullptr;
+  long long evals = 0;
   do {
     if (cudaMemsetAsync(blk, 0, bytes, stream()) != cudaSuccess) { rc = BG_ERR_CUDA; break; }
     k_sing_fixed<<<nsing, SG_THREADS, 0, stream()>>>(g->dev, nd.tp, nd.tpOrdA, nd.tpOrdB, nd.ntp_reg, nd.tpMom, n,
                                                      refine ? 1 : 0, g->sing_flag_tol, L);
     if (cudaGetLastError() != cudaSuccess) { rc = BG_ERR_CUDA; break; }
     g_launches.fetch_add(1, std::memory_order_relaxed);
+    struct { int cnt[4]; unsigned int status; } h;
+    if (cudaMemcpyAsync(&h, blk, sizeof h, cudaMemcpyDeviceToHost, stream()) != cudaSuccess ||
+        cudaStreamSynchronize(stream()) != cudaSuccess) { rc = BG_ERR_CUDA; break; }
     if (refine) {
-      const size_t smem = sizeof(double) * SG_TASKS * 24;
-      static bool attr = false;
-      if (!attr) {
-        if (cudaFuncSetAttribute(k_sing_refine, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-            cudaSuccess) { rc = BG_ERR_CUDA; break; }
-        attr = true;
-      }
-      int dev = 0, nsm = 0, per = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_sing_refine, SG_THREADS, smem);
-      int grid = std::max(1, nsm * std::max(1, per));
-      grid = std::min(grid, nsing);
-      size_t pbytes = sizeof(double) * (size_t)grid * 2 * SG_MAXBOX * SG_REC;
-      if (cudaMallocAsync((void **)&pool, pbytes, stream()) != cudaSuccess) { rc = BG_ERR_NOMEM; break; }
-      k_sing_refine<<<grid, SG_THREADS, smem, stream()>>>(g->dev, nd.tp, nd.tpOrdA, nd.tpOrdB, nd.ntp_reg, nd.tpMom,
-                                                          g->sing_tol, pool, L);
-      if (cudaGetLastError() != cudaSuccess) { rc = BG_ERR_CUDA; break; }
-      g_launches.fetch_add(1, std::memory_order_relaxed);
+      // the order of a list comes from an atomic counter and its pairs are
+      // independent of one another: no result depends on it
+      if ((rc = sgr_refine(g, L, h.cnt, &evals))) break;
+      if (cudaMemcpyAsync(&h, blk, sizeof h, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) { rc = BG_ERR_CUDA; break; }
     }
-    struct { int cnt[4]; int work; unsigned int status; unsigned long long evals; } h;
-    if (cudaMemcpyAsync(&h, blk, sizeof h, cudaMemcpyDeviceToHost, stream()) != cudaSuccess) { rc = BG_ERR_CUDA; break; }
     if (!nd.tpFlag && cudaMallocAsync((void **)&nd.tpFlag, (size_t)nsing, stream()) != cudaSuccess) {
+      set_error("singular near-field precompute: cannot allocate the pair flags");
       rc = BG_ERR_NOMEM;
       break;
     }
@@ -681,13 +827,11 @@ int singular_precompute(bg_geometry *g) {
     }
     if (cudaStreamSynchronize(stream()) != cudaSuccess) { rc = BG_ERR_CUDA; break; }
     g->sing_stats[1] = (long long)h.cnt[0] + h.cnt[1] + h.cnt[2];
-    g->sing_stats[3] = (long long)h.evals;
+    g->sing_stats[3] = evals;
     g->sing_stats[4] = h.status;
     g->sing_stats[5] = refine ? 1 : 0;
   } while (0);
   if (rc == BG_ERR_CUDA) set_error("singular near-field precompute: %s", cudaGetErrorString(cudaGetLastError()));
-  else if (rc == BG_ERR_NOMEM) set_error("singular near-field precompute: cannot allocate the refinement box pool");
-  if (pool) cudaFreeAsync(pool, stream());
   cudaFreeAsync(blk, stream());
   if (rc == BG_OK) BG_CUDA_TRY(cudaStreamSynchronize(stream()));
   return rc;
