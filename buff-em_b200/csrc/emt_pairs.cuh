@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(EMT_JT, 4) k_emt_far(DevGeom g, EmtKernel K, E
           const double x = s[0], y = s[1], z = s[2];
           const double R0 = x - P[0], R1 = y - P[1], R2 = z - P[2];
           const double r2 = fma(R0, R0, fma(R1, R1, R2 * R2));
-          const double ir = rsqrt(r2), kr = K.k * (r2 * ir);
+          const double ir = rsqrt_fast(r2), kr = K.k * (r2 * ir);
           double sn, cs;
           sincos(kr, &sn, &cs);
           const double ir2 = ir * ir, fr = cs * ir, fi = sn * ir;
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(EMT_DJ) k_emt_far_dr(PftArgs P, EmtKernel K, E
                 H[c] = fma(t, y[q][c], H[c]);
               }
             } else {
-              const double ir = rsqrt(r2), kr = K.k * (r2 * ir);
+              const double ir = rsqrt_fast(r2), kr = K.k * (r2 * ir);
               double sn, cs;
               sincos(kr, &sn, &cs);
               const cd phi = cmk(cs * ir, sn * ir), psi = cscale(cmul(phi, cmk(-1.0, kr)), ir * ir);

@@ -16,6 +16,7 @@
 #include <cstdio>
 #include <vector>
 
+#include "devmath.cuh"
 #include "internal.h"
 
 namespace bg {
@@ -106,8 +107,8 @@ __device__ __forceinline__ cd expikr(cd k, double r) {
 // form (one fused multiply-add per term), then cos x = c^2 - s^2,
 // sin x = 2 c s.  Terms to y^14 / y^15: the first omitted terms, y^16/16!
 // and y^17/17!, are below 1e-18 for |y| <= 1/2.  expi_small_short serves
-// |x| <= 1/4 (|y| <= 1/8) with terms to y^10 / y^11 (first omitted terms
-// below 2e-20).
+// |x| <= 1/4 with the series of x itself, terms to x^12 / x^11 (first omitted
+// terms x^14/14! and x^13/13!, below 5e-20 and 3e-18).
 #define EXPI_C(n, f) (((n) & 1 ? -1.0 : 1.0) / (f))
 __device__ __forceinline__ cd expi_halfangle(double c, double sn) { return cd{c * c - sn * sn, 2.0 * c * sn}; }
 __device__ __forceinline__ cd expi_small(double x) {
@@ -131,20 +132,21 @@ __device__ __forceinline__ cd expi_small(double x) {
   return expi_halfangle(c, sn);
 }
 __device__ __forceinline__ cd expi_small_short(double x) {
-  double y = 0.5 * x, y2 = y * y;
-  double c = EXPI_C(5, 3628800.0);               // 1/10!
-  c = fma(c, y2, EXPI_C(4, 40320.0));
-  c = fma(c, y2, EXPI_C(3, 720.0));
-  c = fma(c, y2, EXPI_C(2, 24.0));
-  c = fma(c, y2, EXPI_C(1, 2.0));
-  c = fma(c, y2, 1.0);
+  const double x2 = x * x;
+  double c = EXPI_C(6, 479001600.0);             // 1/12!
+  c = fma(c, x2, EXPI_C(5, 3628800.0));
+  c = fma(c, x2, EXPI_C(4, 40320.0));
+  c = fma(c, x2, EXPI_C(3, 720.0));
+  c = fma(c, x2, EXPI_C(2, 24.0));
+  c = fma(c, x2, EXPI_C(1, 2.0));
+  c = fma(c, x2, 1.0);
   double sn = EXPI_C(5, 39916800.0);             // 1/11!
-  sn = fma(sn, y2, EXPI_C(4, 362880.0));
-  sn = fma(sn, y2, EXPI_C(3, 5040.0));
-  sn = fma(sn, y2, EXPI_C(2, 120.0));
-  sn = fma(sn, y2, EXPI_C(1, 6.0));
-  sn = fma(sn, y2, 1.0) * y;
-  return expi_halfangle(c, sn);
+  sn = fma(sn, x2, EXPI_C(4, 362880.0));
+  sn = fma(sn, x2, EXPI_C(3, 5040.0));
+  sn = fma(sn, x2, EXPI_C(2, 120.0));
+  sn = fma(sn, x2, EXPI_C(1, 6.0));
+  sn = fma(sn, x2, 1.0) * x;
+  return cd{c, sn};
 }
 
 // e^x - 1 - x - x^2/2: GetExpRelTable(x,3,3), GMatrixElements.cc:59-93 -- the
@@ -397,10 +399,14 @@ __device__ __forceinline__ double warp_sum(double v) {
 #define FTF BG_FAR_TILE
 #define FTT BG_FAR_TILE_TETS
 #define FTHR 256     // threads of the far kernel
+#define FPS 13       // doubles per staged tetrahedron (odd: conflict-free 8-byte reads)
 
 struct FarSmem {
-  cd slot[FTF][FTF][4];         // term (sa, sb) of the basis-function pair (row ra, column rb) of the tile
-  double pA[FTT][4][3], pB[FTT][4][3];
+  // term (sa, sb) of the basis-function pair (row ra, column rb) of the tile:
+  // a plane per (sa, sb), rows padded, so that the lanes of a warp (columns
+  // rb running) store to different banks
+  double2 slot[4][FTF][FTF + 1];
+  double pA[FTT][FPS], pB[FTT][FPS];   // 4 points x 3, padded: lanes read different tetrahedra
   double oA[FTT][3], oB[FTT][3];
   double rA[FTT], rB[FTT];      // largest distance of a rule point from its centroid
   double uA[FTF][2][4], uB[FTF][2][4];   // s A (1, Q - o) per side
@@ -418,16 +424,16 @@ __device__ __forceinline__ cd dev_invk2(double wr, double wi) {
   return cd{(wr * wr - wi * wi) / d, -2 * wr * wi / d};
 }
 
-__device__ void far_stage_tets(const DevGeom &g, int tile, double (*P)[4][3], int tid) {
+__device__ void far_stage_tets(const DevGeom &g, int tile, double (*P)[FPS], int tid) {
   int nt = g.tileNT[tile];
   for (int e = tid; e < nt * 12; e += FTHR) {
     int t = e / 12, r = e % 12;
     int tet = g.tileTet[(size_t)tile * FTT + t];
-    P[t][r / 3][r % 3] = g.tetP4[16 * (size_t)tet + 4 * (r / 3) + (r % 3)];
+    P[t][r] = g.tetP4[16 * (size_t)tet + 4 * (r / 3) + (r % 3)];
   }
 }
 
-__device__ void far_stage_bfs(const DevGeom &g, int tile, double (*P)[4][3], double (*u)[2][4], int (*l)[2],
+__device__ void far_stage_bfs(const DevGeom &g, int tile, double (*P)[FPS], double (*u)[2][4], int (*l)[2],
                               int (*v)[5], int tid) {
   if (tid < 2 * FTF) {
     int r = tid >> 1, s = tid & 1;
@@ -442,7 +448,7 @@ __device__ void far_stage_bfs(const DevGeom &g, int tile, double (*P)[4][3], dou
       double coef = (s == 0 ? 1.0 : -1.0) * g.bfArea[bf];
       u[r][s][0] = coef;
       for (int c = 0; c < 3; c++) {
-        double o = 0.25 * (P[lt][0][c] + P[lt][1][c] + P[lt][2][c] + P[lt][3][c]);
+        double o = 0.25 * (P[lt][c] + P[lt][3 + c] + P[lt][6 + c] + P[lt][9 + c]);
         u[r][s][1 + c] = coef * (Q[c] - o);
       }
       l[r][s] = lt;
@@ -455,14 +461,14 @@ __device__ void far_stage_bfs(const DevGeom &g, int tile, double (*P)[4][3], dou
 }
 
 // centroid, point radius and the sides resting on tetrahedron t of a tile
-__device__ void far_stage_tet_info(int t, const double (*P)[4][3], double (*o)[3], double *rad, const int (*l)[2],
+__device__ void far_stage_tet_info(int t, const double (*P)[FPS], double (*o)[3], double *rad, const int (*l)[2],
                                    unsigned char (*sides)[4], int *ns) {
-  for (int c = 0; c < 3; c++) o[t][c] = 0.25 * (P[t][0][c] + P[t][1][c] + P[t][2][c] + P[t][3][c]);
+  for (int c = 0; c < 3; c++) o[t][c] = 0.25 * (P[t][c] + P[t][3 + c] + P[t][6 + c] + P[t][9 + c]);
   double r2 = 0.0;
   for (int i = 0; i < 4; i++) {
     double a2 = 0.0;
     for (int c = 0; c < 3; c++) {
-      double d = P[t][i][c] - o[t][c];
+      double d = P[t][3 * i + c] - o[t][c];
       a2 += d * d;
     }
     r2 = fmax(r2, a2);
@@ -473,6 +479,62 @@ __device__ void far_stage_tet_info(int t, const double (*P)[4][3], double (*o)[3
     for (int s = 0; s < 2; s++)
       if (l[r][s] == t && n < 4) sides[t][n++] = (unsigned char)(r << 1 | s);
   ns[t] = n;
+}
+
+// The 8 moments of one tetrahedron pair (1/(4 pi) included): row points pA
+// about oA, column points pB about oB.  MODE as in k_far, without 3.  No
+// branch per point (coincident points, r < 1e-12, get factor 0), so the four
+// columns of a row are in flight together.  FP64-pipe bound (54 % active, the
+// rest barriers of the tile's four rounds and shared-memory latency): 24.6 ->
+// 17.7 ms at N = 19,872, 100 -> 73 ms at N = 39,150 (with the term
+// factorisation and the padded shared layouts of k_far).
+template <int MODE>
+__device__ __forceinline__ void far_moments(cd k, const double *pA, const double *oA, const double *pB,
+                                            const double *oB, cd m[8]) {
+  const double inv4pi = 0.25 / M_PI;
+#pragma unroll
+  for (int q = 0; q < 8; q++) m[q] = cmk(0, 0);
+  const double e0 = oA[0] - oB[0], e1 = oA[1] - oB[1], e2 = oA[2] - oB[2];
+  const double rc = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
+  // exp(ikr) = exp(ik rc) e: the first factor is common to all points and
+  // multiplies the moments at the end
+  const cd ec = MODE ? cscale(expikr(k, rc), inv4pi) : cmk(inv4pi, 0.0);
+  const double krc = k.r * rc;
+  double yt[4][3];
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) yt[j][c] = pB[3 * j + c] - oB[c];
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const double x0 = pA[3 * i] - oA[0], x1 = pA[3 * i + 1] - oA[1], x2 = pA[3 * i + 2] - oA[2];
+    // x - y from the points themselves: differences of the centroid-relative
+    // coordinates would add two roundings to every distance
+    const double z0 = pA[3 * i], z1 = pA[3 * i + 1], z2 = pA[3 * i + 2];
+    cd ph = cmk(0, 0), W[3] = {cmk(0, 0), cmk(0, 0), cmk(0, 0)};   // sums over the columns: phi, phi y~
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const double R0 = z0 - pB[3 * j], R1 = z1 - pB[3 * j + 1], R2 = z2 - pB[3 * j + 2];
+      const double r2 = fma(R0, R0, fma(R1, R1, R2 * R2));
+      const double ir = r2 < 1.0e-24 ? 0.0 : rsqrt_fast(r2), r = r2 * ir;
+      const cd e = MODE == 2 ? expi_small_short(fma(k.r, r, -krc))
+                             : (MODE == 1 ? expi_small(fma(k.r, r, -krc)) : expikr(k, r));
+      const cd phi = cscale(e, ir);
+      ph = cadd(ph, phi);
+#pragma unroll
+      for (int c = 0; c < 3; c++) W[c] = cmk(fma(phi.r, yt[j][c], W[c].r), fma(phi.i, yt[j][c], W[c].i));
+    }
+    m[0] = cadd(m[0], ph);
+    m[1] = cadd(m[1], cscale(ph, x0));
+    m[2] = cadd(m[2], cscale(ph, x1));
+    m[3] = cadd(m[3], cscale(ph, x2));
+#pragma unroll
+    for (int c = 0; c < 3; c++) m[4 + c] = cadd(m[4 + c], W[c]);
+    m[7] = cmk(fma(W[0].r, x0, fma(W[1].r, x1, fma(W[2].r, x2, m[7].r))),
+               fma(W[0].i, x0, fma(W[1].i, x1, fma(W[2].i, x2, m[7].i))));
+  }
+#pragma unroll
+  for (int q = 0; q < 8; q++) m[q] = MODE ? cmul(ec, m[q]) : cscale(m[q], inv4pi);
 }
 
 // one CTA per 32 x 32 tile of basis-function pairs (upper triangle of tiles).
@@ -507,66 +569,47 @@ __global__ void __launch_bounds__(FTHR, 2) k_far(DevGeom g, cd k, cd invk2, cd *
     if (tid - FTT < nB) far_stage_tet_info(tid - FTT, S.pB, S.oB, S.rB, S.lB, S.sB, S.nsB);
   }
   __syncthreads();
-  const double inv4pi = 0.25 / M_PI;
   for (int p = tid; p < nA * nB; p += FTHR) {
     const int iA = p / nB, tB = p - iA * nB;
     cd m[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) m[q] = cmk(0, 0);
-    // phase about the centroid distance rc (see above); mode 2: |k|(rA+rB)
-    // <= 1/4 (every pair of a fine mesh at moderate frequency), mode 1:
-    // <= 1, mode 0: a sincos per point pair.  1/(4 pi) rides on ec.
-    const double e0 = S.oA[iA][0] - S.oB[tB][0], e1 = S.oA[iA][1] - S.oB[tB][1], e2 = S.oA[iA][2] - S.oB[tB][2];
-    const double rc = sqrt(e0 * e0 + e1 * e1 + e2 * e2);
-    const double span = fabs(k.r) * (S.rA[iA] + S.rB[tB]);
-    const int mode = MODE != 3 ? MODE : (k.i != 0.0 ? 0 : (span <= 0.25 ? 2 : (span <= 1.0 ? 1 : 0)));
-    const cd ec = mode ? cscale(expikr(k, rc), inv4pi) : cmk(inv4pi, 0.0);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const double xt0 = S.pA[iA][i][0] - S.oA[iA][0], xt1 = S.pA[iA][i][1] - S.oA[iA][1],
-                   xt2 = S.pA[iA][i][2] - S.oA[iA][2];
-      cd phiI = cmk(0, 0);
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const double y0 = S.pB[tB][j][0], y1 = S.pB[tB][j][1], y2 = S.pB[tB][j][2];
-        double R0 = S.pA[iA][i][0] - y0, R1 = S.pA[iA][i][1] - y1, R2 = S.pA[iA][i][2] - y2;
-        double r2 = R0 * R0 + R1 * R1 + R2 * R2;
-        if (r2 < 1.0e-24) continue;           // r < 1e-12
-        double ir = rsqrt(r2), r = r2 * ir;   // one reciprocal square root instead of sqrt and a division
-        cd ph = mode == 2 ? cmul(ec, expi_small_short(k.r * (r - rc)))
-                          : (mode == 1 ? cmul(ec, expi_small(k.r * (r - rc))) : cscale(expikr(k, r), inv4pi));
-        cd phi = cscale(ph, ir);
-        const double yt0 = y0 - S.oB[tB][0], yt1 = y1 - S.oB[tB][1], yt2 = y2 - S.oB[tB][2];
-        phiI = cadd(phiI, phi);
-        m[4] = cadd(m[4], cscale(phi, yt0));
-        m[5] = cadd(m[5], cscale(phi, yt1));
-        m[6] = cadd(m[6], cscale(phi, yt2));
-        m[7] = cadd(m[7], cscale(phi, xt0 * yt0 + xt1 * yt1 + xt2 * yt2));
-      }
-      m[0] = cadd(m[0], phiI);
-      m[1] = cadd(m[1], cscale(phiI, xt0));
-      m[2] = cadd(m[2], cscale(phiI, xt1));
-      m[3] = cadd(m[3], cscale(phiI, xt2));
+    if (MODE != 3) {
+      far_moments<MODE == 3 ? 0 : MODE>(k, S.pA[iA], S.oA[iA], S.pB[tB], S.oB[tB], m);
+    } else {
+      // phase about the centroid distance (see above): short series, series or
+      // sincos per point pair, by the span of this pair
+      const double span = fabs(k.r) * (S.rA[iA] + S.rB[tB]);
+      if (k.i != 0.0 || span > 1.0) far_moments<0>(k, S.pA[iA], S.oA[iA], S.pB[tB], S.oB[tB], m);
+      else if (span > 0.25) far_moments<1>(k, S.pA[iA], S.oA[iA], S.pB[tB], S.oB[tB], m);
+      else far_moments<2>(k, S.pA[iA], S.oA[iA], S.pB[tB], S.oB[tB], m);
     }
     // terms of the basis-function pairs on (iA, tB):
     //   s s' A A' [M2/144 - M0/(16 k^2) - q'.M1/144 - q.M1'/144 + q.q' M0/144]
-    const cd kM0 = cmul(invk2, m[0]);
+    // = u0 c + u.g - u0 v0 M0/(16 k^2) with, per column side,
+    // c = (v0 M2 - v.M1)/144 and g = (v M0 - v0 M1')/144.  The last term is
+    // the largest and cancels between the four tetrahedron pairs of a
+    // basis-function pair, so it is added once, at the end.
+    const cd kM0 = cscale(cmul(invk2, m[0]), 1.0 / 16.0);
+#pragma unroll
+    for (int q = 0; q < 8; q++) m[q] = cscale(m[q], 1.0 / 144.0);
     const int na = S.nsA[iA], nb = S.nsB[tB];
-    for (int ia = 0; ia < na; ia++) {
-      const int ca = S.sA[iA][ia], ra = ca >> 1, sa = ca & 1;
-      const double *u = S.uA[ra][sa];
-      const double u0 = u[0], u1 = u[1], u2 = u[2], u3 = u[3];
-      // the row side's part: u0 M2 - u0 (.M1 with v) ... arranged per column below
-      for (int ib = 0; ib < nb; ib++) {
-        const int cb = S.sB[tB][ib], rb = cb >> 1, sb = cb & 1;
-        const double *v = S.uB[rb][sb];
-        double uv = u1 * v[1] + u2 * v[2] + u3 * v[3];
-        cd t = cscale(m[7], u0 * v[0]);
-        t = csub(t, cscale(cadd(cadd(cscale(m[1], v[1]), cscale(m[2], v[2])), cscale(m[3], v[3])), u0));
-        t = csub(t, cscale(cadd(cadd(cscale(m[4], u1), cscale(m[5], u2)), cscale(m[6], u3)), v[0]));
-        t = cadd(t, cscale(m[0], uv));
-        t = csub(cscale(t, 1.0 / 144.0), cscale(kM0, u0 * v[0] / 16.0));
-        S.slot[ra][rb][2 * sa + sb] = t;
+    for (int ib = 0; ib < nb; ib++) {
+      const int cb = S.sB[tB][ib], rb = cb >> 1, sb = cb & 1;
+      const double *v = S.uB[rb][sb];
+      const double v0 = v[0], v1 = v[1], v2 = v[2], v3 = v[3];
+      cd c = cscale(m[7], v0), gv[3];
+      c = cmk(fma(-v1, m[1].r, fma(-v2, m[2].r, fma(-v3, m[3].r, c.r))),
+              fma(-v1, m[1].i, fma(-v2, m[2].i, fma(-v3, m[3].i, c.i))));
+      gv[0] = cmk(fma(v1, m[0].r, -v0 * m[4].r), fma(v1, m[0].i, -v0 * m[4].i));
+      gv[1] = cmk(fma(v2, m[0].r, -v0 * m[5].r), fma(v2, m[0].i, -v0 * m[5].i));
+      gv[2] = cmk(fma(v3, m[0].r, -v0 * m[6].r), fma(v3, m[0].i, -v0 * m[6].i));
+      for (int ia = 0; ia < na; ia++) {
+        const int ca = S.sA[iA][ia], ra = ca >> 1, sa = ca & 1;
+        const double *u = S.uA[ra][sa];
+        const double u0 = u[0], u1 = u[1], u2 = u[2], u3 = u[3];
+        const double uv = u0 * v0;
+        const double tr = fma(u0, c.r, fma(u1, gv[0].r, fma(u2, gv[1].r, u3 * gv[2].r)));
+        const double ti = fma(u0, c.i, fma(u1, gv[0].i, fma(u2, gv[1].i, u3 * gv[2].i)));
+        S.slot[2 * sa + sb][ra][rb] = make_double2(fma(-uv, kM0.r, tr), fma(-uv, kM0.i, ti));
       }
     }
   }
@@ -585,8 +628,8 @@ __global__ void __launch_bounds__(FTHR, 2) k_far(DevGeom g, cd k, cd invk2, cd *
       for (int p = 0; p < 5; p++)
         for (int q = 0; q < 5; q++) ncv += (S.vA[ra][p] == S.vB[rb][q]);
       if (ncv) continue;
-      const cd *sl = S.slot[ra][rb];
-      cd v = cadd(cadd(cadd(sl[0], sl[1]), sl[2]), sl[3]);
+      const double2 s0 = S.slot[0][ra][rb], s1 = S.slot[1][ra][rb], s2 = S.slot[2][ra][rb], s3 = S.slot[3][ra][rb];
+      const cd v = cmk(s0.x + s1.x + s2.x + s3.x, s0.y + s1.y + s2.y + s3.y);
       M[(size_t)a + (size_t)b * ld] = v;
       if (a != b) M[(size_t)b + (size_t)a * ld] = v;
       if (F) {   // the complex64 copy, as k_c128_to_c64 would convert it

@@ -52,6 +52,7 @@
 #include <cmath>
 #include <vector>
 
+#include "devmath.cuh"
 #include "internal.h"
 
 namespace bg {
@@ -208,7 +209,7 @@ __device__ __forceinline__ void sg_line(const SgPair &X, int S, int ka, const do
   for (int i = 0; i < n; i++) {
     const double uu = fma(h, x[i], lo), wi = wx[i];
     const double R0 = fma(uu, D[0], Q[0]), R1 = fma(uu, D[1], Q[1]), R2 = fma(uu, D[2], Q[2]);
-    const double r2 = fma(R0, R0, fma(R1, R1, R2 * R2)), ir = rsqrt(r2);
+    const double r2 = fma(R0, R0, fma(R1, R1, R2 * R2)), ir = rsqrt_fast(r2);
     const double a = wi * ir, b = a * r2;
     T0 += a;
     U0 = fma(a, uu, U0);
