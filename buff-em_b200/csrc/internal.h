@@ -227,6 +227,7 @@ struct bg_geometry {
   double obj_diam = 0.0;        // bound on the distance of two points of one object
   bg::NearGraph graph;
   double *d_scratch = nullptr;  // general scratch (PFT partial sums etc.)
+  double field_rmax = 0.0;      // largest distance of a vertex from its tetrahedron's centroid (with the tables)
   double *d_fieldTet = nullptr, *d_fieldFace = nullptr;  // GetFields tables, 16 doubles per tet each
   void *gnn_cache = nullptr;    // graph-network inference buffers, reused across learned preconditioners
   size_t scratch_bytes = 0;
