@@ -377,10 +377,16 @@ static int zgemm_sub(int M, int N, int K, const cdl *A, size_t lda, const cdl *B
   return st;
 }
 
-// a - l u
+// a - l u with one rounding of the size of a per part (two fused operations
+// on a would round twice; over a factorisation that is 1.5 times the error)
 template <class C>
 __device__ __forceinline__ C cfms(C a, C l, C u) {
-  return C{fma(-l.r, u.r, fma(l.i, u.i, a.r)), fma(-l.r, u.i, fma(-l.i, u.r, a.i))};
+  return C{a.r - fma(l.r, u.r, -(l.i * u.i)), a.i - fma(l.r, u.i, l.i * u.r)};
+}
+// s + a b
+template <class C>
+__device__ __forceinline__ C cmac(C s, C a, C b) {
+  return C{fma(a.r, b.r, fma(-a.i, b.i, s.r)), fma(a.r, b.i, fma(a.i, b.r, s.i))};
 }
 template <class C>
 __device__ __forceinline__ C cshfl(C v, int src) {
@@ -451,6 +457,11 @@ __global__ void __launch_bounds__(TRS_WARPS * 32) k_trsm_leaf(int n, int m, cons
       if (q >= nb) break;
       const int ni = min(32, n - 32 * q);
       const C *t0 = Ts + trs_block(q, q, false) + lane;
+      C sum[4][CPW];       // products for the following blocks, subtracted once
+#pragma unroll
+      for (int s = 0; s < 4; s++)
+#pragma unroll
+        for (int j = 0; j < CPW; j++) sum[s][j] = C{0, 0};
 #pragma unroll 4
       for (int i = 0; i < ni; i++) {
         C x[CPW];
@@ -464,9 +475,13 @@ __global__ void __launch_bounds__(TRS_WARPS * 32) k_trsm_leaf(int n, int m, cons
           if (s < nb) {
             const C l = lds_c(Ts + trs_block(s, q, false) + i * 32 + lane);
 #pragma unroll
-            for (int j = 0; j < CPW; j++) b[s][j] = cfms(b[s][j], l, x[j]);
+            for (int j = 0; j < CPW; j++) sum[s][j] = cmac(sum[s][j], l, x[j]);
           }
       }
+#pragma unroll
+      for (int s = q + 1; s < 4; s++)
+#pragma unroll
+        for (int j = 0; j < CPW; j++) b[s][j] = C{b[s][j].r - sum[s][j].r, b[s][j].i - sum[s][j].i};
     }
   } else {
 #pragma unroll
@@ -474,6 +489,11 @@ __global__ void __launch_bounds__(TRS_WARPS * 32) k_trsm_leaf(int n, int m, cons
       if (q >= nb) continue;
       const int ni = min(32, n - 32 * q);
       const C *t0 = Ts + trs_block(q, q, true) + lane;
+      C sum[4][CPW];
+#pragma unroll
+      for (int s = 0; s < 4; s++)
+#pragma unroll
+        for (int j = 0; j < CPW; j++) sum[s][j] = C{0, 0};
 #pragma unroll 4
       for (int i = ni - 1; i >= 0; i--) {
         const C iu = lds_c(dinv + 32 * q + i);
@@ -491,9 +511,13 @@ __global__ void __launch_bounds__(TRS_WARPS * 32) k_trsm_leaf(int n, int m, cons
         for (int s = 0; s < q; s++) {
           const C l = lds_c(Ts + trs_block(s, q, true) + i * 32 + lane);
 #pragma unroll
-          for (int j = 0; j < CPW; j++) b[s][j] = cfms(b[s][j], l, x[j]);
+          for (int j = 0; j < CPW; j++) sum[s][j] = cmac(sum[s][j], l, x[j]);
         }
       }
+#pragma unroll
+      for (int s = 0; s < q; s++)
+#pragma unroll
+        for (int j = 0; j < CPW; j++) b[s][j] = C{b[s][j].r - sum[s][j].r, b[s][j].i - sum[s][j].i};
     }
   }
 #pragma unroll
@@ -1276,20 +1300,24 @@ __global__ void __launch_bounds__(128) k_blk_update(int M, int nc, int K, const 
     cp_entry(Us + c * 32 + lane, ok ? U + (size_t)c * ld + lane : U, ok);
   }
   cp_commit();
-  C acc[NC];
+  // the products are summed first and subtracted from C once
+  C acc[NC], old[NC];
 #pragma unroll
-  for (int c = 0; c < NC; c++) acc[c] = (r < M && c0 + c < nc) ? Cm[(size_t)(c0 + c) * ld + r] : C{0, 0};
+  for (int c = 0; c < NC; c++) {
+    acc[c] = C{0, 0};
+    old[c] = (r < M && c0 + c < nc) ? Cm[(size_t)(c0 + c) * ld + r] : C{0, 0};
+  }
   cp_wait<0>();
   __syncthreads();
 #pragma unroll 2
   for (int k = 0; k < 32; k++) {
     const C l = lds_c(&Ls[k][lane]);
 #pragma unroll
-    for (int c = 0; c < NC; c++) acc[c] = cfms(acc[c], l, lds_c(Us + (c0 + c) * 32 + k));
+    for (int c = 0; c < NC; c++) acc[c] = cmac(acc[c], l, lds_c(Us + (c0 + c) * 32 + k));
   }
 #pragma unroll
   for (int c = 0; c < NC; c++)
-    if (r < M && c0 + c < nc) Cm[(size_t)(c0 + c) * ld + r] = acc[c];
+    if (r < M && c0 + c < nc) Cm[(size_t)(c0 + c) * ld + r] = C{old[c].r - acc[c].r, old[c].i - acc[c].i};
 }
 template <class C, int NC>
 static int blk_update_launch(int M, int nc, int K, const C *L, const C *U, C *Cm, size_t ld) {
@@ -1631,11 +1659,6 @@ constexpr int trsv_smem() {
   return TV_B * (TV_B + 1) * (int)sizeof(C) + 3 * TV_B * TV_MAXRHS * (int)sizeof(C);
 }
 
-// products and sums on plain complex values
-template <class C>
-__device__ __forceinline__ C cmac(C s, C a, C b) {
-  return C{fma(a.r, b.r, fma(-a.i, b.i, s.r)), fma(a.r, b.i, fma(a.i, b.r, s.i))};
-}
 __device__ __forceinline__ int ld_acquire(const int *p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
