@@ -636,6 +636,7 @@ static int trsm(int n, int m, const C *T, size_t ldt, C *B, size_t ldb, int uppe
 // consecutive threads on consecutive rows, free of bank conflicts.  One grid
 // barrier per column exchanges the CTAs' pivot candidates.
 // =========================================================================
+static constexpr int panel_max_grid = 148;   // CTAs of a grid-wide panel at most
 template <class C>
 struct PanelArgs {
   C *A;
@@ -649,6 +650,7 @@ struct PanelArgs {
   int *cidx;       // [2][grid] candidate row
   C *crow;         // [2][grid][32] candidate row values
   C *jrow;         // [2][32] values of row k0+j before the swap
+  unsigned long long *slots;   // k_panel_rf over the grid: tagged candidate messages
 };
 
 __device__ __forceinline__ bool better(double v, int i, double bv, int bi) {
@@ -784,141 +786,6 @@ __device__ __forceinline__ cfl ldcg_c<cfl>(const cfl *p) {
   return cfl{v.x, v.y};
 }
 
-// The same panel on one thread-block cluster (up to 16 CTAs, the slices in
-// their shared memory): when the panel fits, the per-column grid barrier
-// becomes a cluster barrier and the candidate exchange reads the other CTAs'
-// shared memory directly (distributed shared memory) instead of global
-// memory.  Pivot choice, interchanges and arithmetic are those of k_panel.
-// Candidate slots are double-buffered by column parity: a CTA writing the
-// slots of column j + 2 has passed the barrier of column j + 1, which every
-// CTA reaches only after reading column j's slots.  The last barrier keeps
-// every CTA's shared memory alive until all remote reads are done.
-#define PCL_THREADS 512     // threads per CTA of the cluster panel (about one row each)
-template <class C>
-__global__ void __launch_bounds__(PCL_THREADS) k_panel_cl(PanelArgs<C> P) {
-  typedef typename CxT<C>::R R;
-  cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C *S = (C *)smem_raw;                     // [w][rows_per]: column c at S + c * rows_per
-  __shared__ double rv[PCL_THREADS / 32];
-  __shared__ int ri[PCL_THREADS / 32];
-  __shared__ double cval[2];                // this CTA's candidate, per column parity
-  __shared__ int cidx[2];
-  __shared__ C crow[2][32];                 // its candidate row
-  __shared__ C jrow[2][32];                 // row k0 + j before the swap (CTA holding it)
-  __shared__ int s_piv;
-  __shared__ C prow[32], jr[32];
-  const int w = P.w, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int rank = (int)cl.block_rank(), G = (int)cl.num_blocks();
-  const int r0 = P.k0 + rank * P.rows_per;
-  const int r1 = min(P.Nr, r0 + P.rows_per);
-  const int nr = max(0, r1 - r0), lds = P.rows_per;
-  for (int e0 = 0; e0 < nr * w; e0 += 8 * PCL_THREADS) {
-    C v[8];
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int e = e0 + u * PCL_THREADS + tid;
-      v[u] = e < nr * w ? P.A[(size_t)(P.k0 + e / nr) * P.ld + r0 + e % nr] : C{0, 0};
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-      const int e = e0 + u * PCL_THREADS + tid;
-      if (e < nr * w) S[(e / nr) * lds + e % nr] = v[u];
-    }
-  }
-  __syncthreads();
-  for (int j = 0; j < w; j++) {
-    const int gj = P.k0 + j, buf = j & 1;
-    // 1. local pivot candidate (i[cz]amax: max |re|+|im|, first index on ties)
-    double bv = -1.0;
-    int bi = 0x7fffffff;
-    for (int r = tid; r < nr; r += PCL_THREADS) {
-      int gr = r0 + r;
-      if (gr < gj) continue;
-      C v = S[j * lds + r];
-      double a = (double)(fabs(v.r) + fabs(v.i));
-      if (better(a, gr, bv, bi)) { bv = a; bi = gr; }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      double ov = __shfl_xor_sync(0xffffffffu, bv, o);
-      int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-      if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-    }
-    if (lane == 0) { rv[wid] = bv; ri[wid] = bi; }
-    __syncthreads();
-    if (tid == 0) {
-      for (int k = 1; k < PCL_THREADS / 32; k++)
-        if (better(rv[k], ri[k], rv[0], ri[0])) { rv[0] = rv[k]; ri[0] = ri[k]; }
-      cval[buf] = rv[0];
-      cidx[buf] = ri[0];
-    }
-    __syncthreads();
-    const int myc = ri[0];
-    if (rv[0] >= 0.0 && tid < w) crow[buf][tid] = S[tid * lds + myc - r0];
-    if (gj >= r0 && gj < r1 && tid < w) jrow[buf][tid] = S[tid * lds + gj - r0];
-    cl.sync();   // every CTA's candidate is visible in the cluster
-    // 2. global pivot: lane k reads CTA k's candidate
-    if (tid < 32) {
-      double v = -1.0;
-      int i = 0x7fffffff, b = 0;
-      if (lane < G) {
-        v = *cl.map_shared_rank(&cval[buf], lane);
-        i = *cl.map_shared_rank(&cidx[buf], lane);
-        b = lane;
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        double ov = __shfl_xor_sync(0xffffffffu, v, o);
-        int oi = __shfl_xor_sync(0xffffffffu, i, o);
-        int ob = __shfl_xor_sync(0xffffffffu, b, o);
-        if (better(ov, oi, v, i)) { v = ov; i = oi; b = ob; }
-      }
-      const int owner = (gj - P.k0) / P.rows_per;   // CTA holding row gj
-      if (lane < w) {
-        prow[lane] = *cl.map_shared_rank(&crow[buf][lane], b);
-        jr[lane] = *cl.map_shared_rank(&jrow[buf][lane], owner);
-      }
-      if (lane == 0) s_piv = i;
-    }
-    __syncthreads();
-    const int piv = s_piv;
-    if (rank == 0 && tid == 0) P.ipiv[gj] = piv + 1;
-    // 3. swap rows gj and piv inside the panel
-    if (piv != gj) {
-      if (piv >= r0 && piv < r1 && tid < w) S[tid * lds + piv - r0] = jr[tid];
-      if (gj >= r0 && gj < r1 && tid < w) S[tid * lds + gj - r0] = prow[tid];
-    }
-    __syncthreads();
-    // 4. scale the column below the pivot and update the rest of the panel
-    C p = prow[j];
-    R d = p.r * p.r + p.i * p.i;
-    if (d == (R)0) {
-      if (rank == 0 && tid == 0) atomicCAS(P.info, 0, gj + 1);
-    } else {
-      C inv{p.r / d, -p.i / d};
-      int ncol = w - j - 1;
-      for (int r = tid; r < nr; r += PCL_THREADS) {
-        int gr = r0 + r;
-        if (gr <= gj) continue;
-        C v = S[j * lds + r];
-        C l{v.r * inv.r - v.i * inv.i, v.r * inv.i + v.i * inv.r};
-        S[j * lds + r] = l;
-        for (int c = 1; c <= ncol; c++) {
-          C u = prow[j + c];
-          C &t = S[(j + c) * lds + r];
-          t.r -= l.r * u.r - l.i * u.i;
-          t.i -= l.r * u.i + l.i * u.r;
-        }
-      }
-    }
-    __syncthreads();
-  }
-  for (int e = tid; e < nr * w; e += PCL_THREADS) {
-    const int r = e % nr, c = e / nr;
-    P.A[(size_t)(P.k0 + c) * P.ld + r0 + r] = S[c * lds + r];
-  }
-  cl.sync();   // no CTA leaves while another may still read its shared memory
-}
-
 // -------------------------------------------------------------------------
 // The panel with its rows in registers, on one cluster.  A thread owns one row
 // of the panel in registers, so the rank-1 update reads and writes registers
@@ -950,6 +817,16 @@ __global__ void __launch_bounds__(PCL_THREADS) k_panel_cl(PanelArgs<C> P) {
 // every candidate of column j + 1, which each CTA sends only after all its
 // warps have finished with column j.  Waits are bounded; one that runs out is
 // reported through info, and the CTA goes on so that the cluster ends.
+//
+// GRID: panels taller than one cluster.  The same CTAs over the whole grid (a
+// cooperative launch), one row a thread, and the exchange through L2: a CTA
+// stores its candidate as 64-bit words that carry a 32-bit tag (launch count
+// and column) beside 32 bits of data, so no fence and no flag orders them; one
+// warp per CTA polls all keys, finds the winner and fetches its row and
+// reciprocal, which arrive by the same tags.  Two block barriers a column
+// instead of a grid barrier; three trips through L2 (keys out, keys in, row in)
+// set the time: panels of one factorisation at N = 19,872 77 -> 71 ms, complex64
+// 64 -> 53 ms.
 //
 // Pivot choice (first index on ties), interchanges and arithmetic are those of
 // k_panel.  A NaN never wins; a column of NaNs takes its own row.
@@ -1028,7 +905,56 @@ __device__ __forceinline__ void push_c(unsigned dst, cfl v, unsigned bar) {
   st_async8(dst, (unsigned long long)__float_as_uint(v.i) << 32 | __float_as_uint(v.r), bar);
 }
 
-template <class C, int TMAX>
+// tagged words: 32 bits of data each.  A complex entry takes 4 (complex128) or
+// 2 (complex64) of them.
+#define PRG_STRIDE 136            // words per CTA and buffer: key (3, pad to 4), inv (4), row (32 x 4)
+template <class C> struct PrgWords { static constexpr int N = sizeof(C) / 4; };
+__device__ __forceinline__ void prg_split(cdl v, unsigned (&x)[4]) {
+  x[0] = (unsigned)__double2loint(v.r); x[1] = (unsigned)__double2hiint(v.r);
+  x[2] = (unsigned)__double2loint(v.i); x[3] = (unsigned)__double2hiint(v.i);
+}
+__device__ __forceinline__ void prg_split(cfl v, unsigned (&x)[2]) { x[0] = __float_as_uint(v.r); x[1] = __float_as_uint(v.i); }
+__device__ __forceinline__ void prg_join(const unsigned (&x)[4], cdl &v) {
+  v = cdl{__hiloint2double((int)x[1], (int)x[0]), __hiloint2double((int)x[3], (int)x[2])};
+}
+__device__ __forceinline__ void prg_join(const unsigned (&x)[2], cfl &v) { v = cfl{__uint_as_float(x[0]), __uint_as_float(x[1])}; }
+__device__ __forceinline__ void st_word(unsigned long long *p, unsigned tag, unsigned v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"((unsigned long long)tag << 32 | v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+template <class C>
+__device__ __forceinline__ void prg_put(unsigned long long *p, unsigned tag, C v) {
+  unsigned x[PrgWords<C>::N];
+  prg_split(v, x);
+#pragma unroll
+  for (int k = 0; k < PrgWords<C>::N; k++) st_word(p + k, tag, x[k]);
+}
+// one entry once its tags have arrived; false when the wait runs out
+template <class C>
+__device__ __forceinline__ bool prg_get(const unsigned long long *p, unsigned tag, int limit, C &v) {
+  unsigned x[PrgWords<C>::N];
+  for (int it = 0; it < limit; it++) {
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < PrgWords<C>::N; k++) {
+      const unsigned long long q = ld_word(p + k);
+      ok = ok && (unsigned)(q >> 32) == tag;
+      x[k] = (unsigned)q;
+    }
+    if (ok) {
+      prg_join(x, v);
+      return true;
+    }
+  }
+  v = C{0, 0};
+  return false;
+}
+
+template <class C, int TMAX, bool GRID>
 __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
   typedef typename CxT<C>::R R;
   constexpr int T = TMAX + 1;      // column stride of Ls: a row's columns fall into different banks
@@ -1037,7 +963,7 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
   C *Ls = reinterpret_cast<C *>(smem_raw + sizeof(PrfSmem<C>));   // [32][T]
   cg::cluster_group cl = cg::this_cluster();
   const int w = P.w, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = (int)(blockDim.x >> 5) - 1;
-  const int rank = (int)cl.block_rank(), G = (int)cl.num_blocks();
+  const int rank = GRID ? (int)blockIdx.x : (int)cl.block_rank(), G = GRID ? (int)gridDim.x : (int)cl.num_blocks();
   const int r0 = P.k0 + rank * P.rows_per, nr = max(0, min(P.rows_per, P.Nr - r0));
   const bool top = wid == nw;                      // the copy of the top rows
   const int row = top ? P.k0 + lane : r0 + tid;
@@ -1050,12 +976,19 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
   for (int c = 0; c < 32; c++) a[c] = (held && c < w) ? P.A[(size_t)(P.k0 + c) * P.ld + row] : C{0, 0};
   const unsigned base = smem_addr(&S);
   const unsigned bar0 = smem_addr(&S.bar[0]);
-  if (tid == 0) {
+  // GRID: launch count at ctr[0] (the last CTA of a launch raises it), tickets
+  // of finished CTAs at ctr[1]
+  unsigned long long *ctr = P.slots + 2 * (size_t)panel_max_grid * PRG_STRIDE;
+  unsigned tag0 = 0;
+  __shared__ int s_piv;
+  if (GRID) {
+    tag0 = (unsigned)ld_word(ctr) * 64u + 1u;
+  } else if (tid == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  cl.sync();   // barriers of every CTA are ready
+  if (!GRID) cl.sync();   // barriers of every CTA are ready
   const unsigned bytes = (unsigned)(G * (33 * sizeof(C) + 16));
   int limit = PRF_SPIN;
   // search state of the coming column: this row's entry, its key, the warp's maximum
@@ -1065,7 +998,7 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
   for (int j = 0; j < w; j++) {
     const int gj = P.k0 + j, buf = j & 1;
     const unsigned bar = bar0 + 8 * buf;
-    if (tid == 0)
+    if (!GRID && tid == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
     // 1. candidate of every warp; its row, and row gj from the top copy
     int src = j;
@@ -1085,60 +1018,146 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
 #pragma unroll
           for (int c = c0; c < c0 + 8; c++) sts_c(keep + c, a[c]);
     __syncthreads();
-    // 2. the CTA's candidate, pushed to every CTA: its row by warp q to CTAs
-    // q, q + nw, ..., key and reciprocal by the extra warp, lane q to CTA q
-    {
-      unsigned long long k2 = lane < nw ? S.wkey[buf][lane] : 0ull;
-      const int idx = lane < nw ? S.widx[buf][lane] : 0x7fffffff;
-      const bool ok = idx != 0x7fffffff;
-      const int bw = warp_first_max<C>(k2, ok, __reduce_max_sync(0xffffffffu, key_hi(k2, ok)));
-      const unsigned msg = smem_addr(&S.msg[buf][rank]) - base;
-      if (top) {
+    int b = 0, piv = gj;
+    if (GRID) {
+      // 2. the CTA's candidate: key and row by the first warp, the reciprocal
+      // of its pivot by the extra warp
+      const unsigned tag = tag0 + j;
+      unsigned long long *slot = P.slots + ((size_t)buf * panel_max_grid + rank) * PRG_STRIDE;
+      if (wid == 0 || top) {
+        unsigned long long k2 = lane < nw ? S.wkey[buf][lane] : 0ull;
+        const int idx = lane < nw ? S.widx[buf][lane] : 0x7fffffff;
+        const bool ok = idx != 0x7fffffff;
+        const int bw = warp_first_max<C>(k2, ok, __reduce_max_sync(0xffffffffu, key_hi(k2, ok)));
         const int bi = __shfl_sync(0xffffffffu, idx, bw < 0 ? 0 : bw);
-        if (lane < G) {
-          const unsigned rbase = map_cta(base, lane), rb = rbase + (bar - base);
-          st_async16(rbase + msg + 32 * (unsigned)sizeof(C), k2, (unsigned long long)(bw < 0 ? -1ll : (long long)bi), rb);
+        if (top) {
           C iv = C{0, 0};
           if (bw >= 0) {
             const C p = lds_c(&S.wrow[buf][bw][j]);
             const R d = p.r * p.r + p.i * p.i;
             iv = C{p.r / d, -p.i / d};
           }
-          push_c(rbase + msg + 32 * (unsigned)sizeof(C) + 16, iv, rb);
-        }
-      } else {
-        const int bi = __shfl_sync(0xffffffffu, idx, bw < 0 ? 0 : bw);
-        C v = C{0, 0};
-        if (bw >= 0 && lane < w) v = lds_c(lane < j ? &Ls[lane * T + (bi - r0)] : &S.wrow[buf][bw][lane]);
-        const unsigned dst = msg + lane * (unsigned)sizeof(C);
-        for (int q = wid; q < G; q += nw) {
-          const unsigned rbase = map_cta(base, q);
-          push_c(rbase + dst, v, rbase + (bar - base));
+          if (lane == 0) prg_put(slot + 4, tag, iv);
+        } else {
+          if (lane < 3) st_word(slot + lane, tag, lane == 0 ? (unsigned)(k2 >> 32) : lane == 1 ? (unsigned)k2 : (unsigned)(bw < 0 ? 0x7fffffff : bi));
+          C v = C{0, 0};
+          if (bw >= 0 && lane < w) v = lds_c(lane < j ? &Ls[lane * T + (bi - r0)] : &S.wrow[buf][bw][lane]);
+          prg_put(slot + 8 + lane * PrgWords<C>::N, tag, v);
         }
       }
+      // 3. the first warp polls every key, then fetches the winner's row
+      if (wid == 0) {
+        unsigned long long bk = 0;
+        int bidx = 0x7fffffff;
+        // the lane's up to five CTAs together where the registers allow it
+        // (complex64: 67 -> 64 us a panel; complex128 keeps 128 registers of rows
+        // and spills: 71 -> 92 ms of panels at N = 19,872)
+        constexpr int NQ = sizeof(C) == 8 ? (panel_max_grid + 31) / 32 : 1;
+        bool fine = true;
+        for (int q0 = lane; q0 < G; q0 += 32 * NQ) {
+          unsigned long long x[NQ][3];
+          bool in = false;
+          for (int it = 0; it < limit && !in; it++) {
+            in = true;
+#pragma unroll
+            for (int u = 0; u < NQ; u++) {
+              const int q = q0 + 32 * u;
+              const unsigned long long *ps = P.slots + ((size_t)buf * panel_max_grid + (q < G ? q : q0)) * PRG_STRIDE;
+              x[u][0] = ld_word(ps);
+              x[u][1] = ld_word(ps + 1);
+              x[u][2] = ld_word(ps + 2);
+            }
+#pragma unroll
+            for (int u = 0; u < NQ; u++)
+              in = in && (unsigned)(x[u][0] >> 32) == tag && (unsigned)(x[u][1] >> 32) == tag && (unsigned)(x[u][2] >> 32) == tag;
+          }
+          fine = fine && in;
+#pragma unroll
+          for (int u = 0; u < NQ; u++) {
+            const unsigned long long k = x[u][0] << 32 | (unsigned)x[u][1];
+            const int id = (int)(unsigned)x[u][2];
+            // the lane's CTAs come in row order: the first of equal keys stays
+            if (in && q0 + 32 * u < G && id != 0x7fffffff && (bidx == 0x7fffffff || k > bk)) { bk = k; bidx = id; }
+          }
+        }
+        const bool has = bidx != 0x7fffffff;
+        const unsigned mh2 = __reduce_max_sync(0xffffffffu, has ? (unsigned)(bk >> 32) : 0u);
+        bool c = has && (unsigned)(bk >> 32) == mh2;
+        const unsigned ml2 = __reduce_max_sync(0xffffffffu, c ? (unsigned)bk : 0u);
+        c = c && (unsigned)bk == ml2;
+        piv = (int)__reduce_min_sync(0xffffffffu, c ? (unsigned)bidx : 0x7fffffffu);
+        if (piv < gj || piv >= P.Nr) piv = gj;
+        const int wq = min((piv - P.k0) / P.rows_per, G - 1);
+        const unsigned long long *ps = P.slots + ((size_t)buf * panel_max_grid + wq) * PRG_STRIDE;
+        C v, iv = C{0, 0};
+        fine = prg_get(ps + 8 + lane * PrgWords<C>::N, tag, limit, v) && fine;
+        if (lane == 0) fine = prg_get(ps + 4, tag, limit, iv) && fine;
+        sts_c(&S.msg[buf][0].row[lane], v);
+        if (lane == 0) {
+          sts_c(&S.msg[buf][0].inv, iv);
+          s_piv = piv;
+        }
+        if (!fine) { limit = 1; atomicExch(P.info, 0x7fffffff); atomicExch(P.info + 1, 300); }
+      }
+      __syncthreads();
+      piv = s_piv;
+    } else {
+      // 2. the CTA's candidate, pushed to every CTA: its row by warp q to CTAs
+      // q, q + nw, ..., key and reciprocal by the extra warp, lane q to CTA q
+      {
+        unsigned long long k2 = lane < nw ? S.wkey[buf][lane] : 0ull;
+        const int idx = lane < nw ? S.widx[buf][lane] : 0x7fffffff;
+        const bool ok = idx != 0x7fffffff;
+        const int bw = warp_first_max<C>(k2, ok, __reduce_max_sync(0xffffffffu, key_hi(k2, ok)));
+        const unsigned msg = smem_addr(&S.msg[buf][rank]) - base;
+        if (top) {
+          const int bi = __shfl_sync(0xffffffffu, idx, bw < 0 ? 0 : bw);
+          if (lane < G) {
+            const unsigned rbase = map_cta(base, lane), rb = rbase + (bar - base);
+            st_async16(rbase + msg + 32 * (unsigned)sizeof(C), k2, (unsigned long long)(bw < 0 ? -1ll : (long long)bi), rb);
+            C iv = C{0, 0};
+            if (bw >= 0) {
+              const C p = lds_c(&S.wrow[buf][bw][j]);
+              const R d = p.r * p.r + p.i * p.i;
+              iv = C{p.r / d, -p.i / d};
+            }
+            push_c(rbase + msg + 32 * (unsigned)sizeof(C) + 16, iv, rb);
+          }
+        } else {
+          const int bi = __shfl_sync(0xffffffffu, idx, bw < 0 ? 0 : bw);
+          C v = C{0, 0};
+          if (bw >= 0 && lane < w) v = lds_c(lane < j ? &Ls[lane * T + (bi - r0)] : &S.wrow[buf][bw][lane]);
+          const unsigned dst = msg + lane * (unsigned)sizeof(C);
+          for (int q = wid; q < G; q += nw) {
+            const unsigned rbase = map_cta(base, q);
+            push_c(rbase + dst, v, rbase + (bar - base));
+          }
+        }
+      }
+      // 3. everyone's candidates
+      {
+        unsigned done = 0;
+        for (int it = 0; it < limit && !done; it++)
+          asm volatile(
+              "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+              " selp.u32 %0, 1, 0, p;\n}\n"
+              : "=r"(done)
+              : "r"(bar), "r"((unsigned)((j >> 1) & 1))
+              : "memory");
+        if (!done) { limit = 1; atomicExch(P.info, 0x7fffffff); atomicExch(P.info + 1, 300); }
+      }
+      const int ql = lane < G ? lane : 0;
+      unsigned long long k3 = S.msg[buf][ql].key;
+      const int idx = (int)S.msg[buf][ql].idx;
+      const bool ok = lane < G && idx >= 0;
+      b = warp_first_max<C>(k3, ok, __reduce_max_sync(0xffffffffu, key_hi(k3, ok)));
+      if (b < 0) b = 0;
+      piv = __shfl_sync(0xffffffffu, idx, b);
+      if (piv < gj || piv >= P.Nr) piv = gj;   // no candidate, or a wait ran out
     }
-    // 3. everyone's candidates
-    {
-      unsigned done = 0;
-      for (int it = 0; it < limit && !done; it++)
-        asm volatile(
-            "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-            " selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(bar), "r"((unsigned)((j >> 1) & 1))
-            : "memory");
-      if (!done) { limit = 1; atomicExch(P.info, 0x7fffffff); atomicExch(P.info + 1, 300); }
-    }
-    const int ql = lane < G ? lane : 0;
-    unsigned long long k3 = S.msg[buf][ql].key;
-    const int idx = (int)S.msg[buf][ql].idx;
-    const bool ok = lane < G && idx >= 0;
-    int b = warp_first_max<C>(k3, ok, __reduce_max_sync(0xffffffffu, key_hi(k3, ok)));
-    if (b < 0) b = 0;
-    const int piv = __shfl_sync(0xffffffffu, idx, b);
     const PrfMsg<C> &W = S.msg[buf][b];
     const C p = lds_c(&W.row[j]), pinv = lds_c(&W.inv);
-    __syncthreads();   // every warp has read the rows it pushes (Ls changes below)
+    if (!GRID) __syncthreads();   // every warp has read the rows it pushes (Ls changes below)
     // 4. interchange: row gj is final and goes to Ls (a warp of rank 0); the
     // pivot's place takes over the old row gj
     if (rank == 0) {
@@ -1190,7 +1209,15 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
   // to Ls by step 4; the others hold their L
   if (mine)
     for (int c = 0; c < w; c++) P.A[(size_t)(P.k0 + c) * P.ld + row] = lds_c(&Ls[c * T + tid]);
-  cl.sync();   // no CTA leaves while messages for it may be in flight
+  if (GRID) {
+    // every CTA has read the launch count before any CTA can finish
+    if (tid == 0 && atomicAdd(ctr + 1, 1ull) == (unsigned long long)(G - 1)) {
+      ctr[1] = 0;
+      ctr[0] = ctr[0] + 1;
+    }
+  } else {
+    cl.sync();   // no CTA leaves while messages for it may be in flight
+  }
 }
 
 // Row interchanges ipiv[k0..k0+w) on the columns [0, ncols) outside
@@ -1346,52 +1373,10 @@ struct LUWork {
   int *cidx;
   void *crow, *jrow;
   int *info;
+  unsigned long long *slots;
 };
 
 static int panel_grid = 0, panel_smem_max = 0, panel_rows_target = 32;
-
-// cluster size of k_panel_cl<C> on this device (0: no cluster path), found
-// once: the largest of 16 and 8 that the occupancy query allows with a full
-// slice of shared memory per CTA
-static int panel_cl_smem_max = 0;
-template <class C>
-static int panel_cluster_size() {
-  static int cs = -1;
-  if (cs >= 0) return cs;
-  cs = 0;
-  int dev = 0, smemopt = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&smemopt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
-    return cs;
-  panel_cl_smem_max = smemopt - 6 * 1024;   // room for the kernel's static shared memory
-  if (cudaFuncSetAttribute(k_panel_cl<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_cl_smem_max) != cudaSuccess ||
-      cudaFuncSetAttribute(k_panel_cl<C>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-    cudaGetLastError();
-    return cs;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(16);
-  cfg.blockDim = dim3(PCL_THREADS);
-  cfg.dynamicSmemBytes = panel_cl_smem_max;
-  int best = 0;
-  if (cudaOccupancyMaxPotentialClusterSize(&best, (void *)k_panel_cl<C>, &cfg) != cudaSuccess) best = 0;
-  int want = best >= 16 ? 16 : (best >= 8 ? 8 : 0);
-  if (want) {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = want;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(want);
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, (void *)k_panel_cl<C>, &cfg) != cudaSuccess || nclusters < 1) want = 0;
-  }
-  cudaGetLastError();
-  cs = want;
-  return cs;
-}
 
 template <class C, int TMAX>
 constexpr int panel_rf_smem() { return (int)sizeof(PrfSmem<C>) + 32 * (TMAX + 1) * (int)sizeof(C); }
@@ -1403,8 +1388,8 @@ static int panel_rf_cluster() {
   if (cs >= 0) return cs;
   cs = 0;
   const int smem = panel_rf_smem<C, TMAX>();
-  if (cudaFuncSetAttribute(k_panel_rf<C, TMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-      cudaFuncSetAttribute(k_panel_rf<C, TMAX>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+  if (cudaFuncSetAttribute(k_panel_rf<C, TMAX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_panel_rf<C, TMAX, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
     cudaGetLastError();
     return cs;
   }
@@ -1421,7 +1406,7 @@ static int panel_rf_cluster() {
     cfg.attrs = at;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, (void *)k_panel_rf<C, TMAX>, &cfg) == cudaSuccess && n >= 1) cs = want;
+    if (cudaOccupancyMaxActiveClusters(&n, (void *)k_panel_rf<C, TMAX, false>, &cfg) == cudaSuccess && n >= 1) cs = want;
   }
   cudaGetLastError();
   return cs;
@@ -1437,7 +1422,7 @@ static int panel_rf(bg_matrix *m, const LUWork &W, int k0, int w, int blk_end, b
   // (rank 0 owns the w rows of the diagonal block)
   const int G = std::min(RS, std::max(1, (Mp + 127) / 128));
   const int rows = (Mp + G - 1) / G, threads = (rows + 31) / 32 * 32 + 32;
-  PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow};
+  PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow, W.slots};
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(G);
   cfg.blockDim = dim3(threads);
@@ -1451,7 +1436,34 @@ static int panel_rf(bg_matrix *m, const LUWork &W, int k0, int w, int blk_end, b
   cfg.attrs = at;
   cfg.numAttrs = 1;
   prof_start(PROF_PANEL);
-  BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_rf<C, TMAX>, P));
+  BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_rf<C, TMAX, false>, P));
+  BG_LAUNCHED();
+  prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
+  return laswp<C>(m, k0, w, blk_end);
+}
+
+// the same panel over the grid, through L2
+#define PRG_T 256
+#define PRG_ROWS 192     // rows per CTA until the grid is full
+template <class C>
+static int panel_rg(bg_matrix *m, const LUWork &W, int k0, int w, int blk_end, bool *done) {
+  const int N = m->N, Mp = N - k0;
+  const int maxg = std::min(panel_max_grid, panel_grid);
+  *done = Mp <= maxg * PRG_T;
+  if (!*done) return BG_OK;
+  static bool attr = false;
+  if (!attr) {
+    BG_CUDA_TRY(cudaFuncSetAttribute(k_panel_rf<C, PRG_T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     panel_rf_smem<C, PRG_T>()));
+    attr = true;
+  }
+  const int G = std::min(maxg, (Mp + PRG_ROWS - 1) / PRG_ROWS);
+  const int rows = (Mp + G - 1) / G, threads = (rows + 31) / 32 * 32 + 32;
+  PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow, W.slots};
+  void *args[] = {&P};
+  prof_start(PROF_PANEL);
+  BG_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_panel_rf<C, PRG_T, true>, dim3(G), dim3(threads), args,
+                                          (size_t)panel_rf_smem<C, PRG_T>(), stream()));
   BG_LAUNCHED();
   prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
   return laswp<C>(m, k0, w, blk_end);
@@ -1466,37 +1478,9 @@ static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w, int blk_end)
   bool done = false;
   int st = panel_rf<C, PrfCfg<C>::T0>(m, W, k0, w, blk_end, &done);
   if (!st && !done) st = panel_rf<C, PrfCfg<C>::T1>(m, W, k0, w, blk_end, &done);
+  if (!st && !done) st = panel_rg<C>(m, W, k0, w, blk_end, &done);
   if (st || done) return st;
-  // the whole panel in one cluster's shared memory: cluster barriers and
-  // distributed shared memory instead of a grid barrier per column
-  const int CS = panel_cluster_size<C>();
-  if (CS) {
-    const int G = std::min(CS, std::max(1, (Mp + panel_rows_target - 1) / panel_rows_target));
-    const int rows = (Mp + G - 1) / G;
-    const size_t smem = (size_t)rows * w * sizeof(C);
-    // past ~512 rows per CTA the row updates of 16 CTAs cost more than the
-    // grid barrier they save (148 CTAs share them in the grid form)
-    if (rows <= 512 && smem <= (size_t)panel_cl_smem_max) {
-      PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow};
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(G);
-      cfg.blockDim = dim3(PCL_THREADS);
-      cfg.dynamicSmemBytes = smem;
-      cfg.stream = stream();
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = G;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      prof_start(PROF_PANEL);
-      BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_cl<C>, P));
-      BG_LAUNCHED();
-      prof_stop(PROF_PANEL, 8.0 * Mp * (double)w * w / 2);
-      return laswp<C>(m, k0, w, blk_end);
-    }
-  }
+  // still taller (more than 37,888 rows): slices in shared memory
   int G = std::min(panel_grid, std::max(1, (Mp + panel_rows_target - 1) / panel_rows_target));
   while (G < panel_grid && (size_t)((Mp + G - 1) / G) * w * sizeof(C) > (size_t)panel_smem_max) G++;
   int rows = (Mp + G - 1) / G;
@@ -1510,7 +1494,7 @@ static int panel_leaf(bg_matrix *m, const LUWork &W, int k0, int w, int blk_end)
     BG_CUDA_TRY(cudaFuncSetAttribute(k_panel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem_max));
     attr = true;
   }
-  PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow};
+  PanelArgs<C> P{(C *)m->d, m->ld, N, k0, w, rows, m->d_ipiv, W.info, W.cval, W.cidx, (C *)W.crow, (C *)W.jrow, W.slots};
   void *args[] = {&P};
   prof_start(PROF_PANEL);
   BG_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_panel<C>, dim3(G), dim3(256), args, smem, stream()));
@@ -1566,6 +1550,24 @@ static int panel_init() {
   return BG_OK;
 }
 
+#define PRG_BYTES (sizeof(unsigned long long) * (2 * (size_t)panel_max_grid * PRG_STRIDE + 2))   // slots, launch count, tickets
+static size_t lu_work_bytes(bg_matrix *m) {
+  const size_t csz = m->precision == BG_C128 ? sizeof(cdl) : sizeof(cfl);
+  return PRG_BYTES + csz * 2 * panel_grid * 32 + csz * 64 + sizeof(double) * 2 * panel_grid +
+         sizeof(int) * 2 * panel_grid + 256;
+}
+static int lu_work_alloc(bg_matrix *m, size_t need) {
+  if (m->work_bytes >= need) return BG_OK;
+  if (m->d_work) cudaFree(m->d_work);
+  m->d_work = nullptr;
+  m->work_bytes = 0;
+  BG_CUDA_TRY(cudaMalloc(&m->d_work, need));
+  m->work_bytes = need;
+  // tags, launch count and tickets of the grid-wide panel start at zero
+  BG_CUDA_TRY(cudaMemsetAsync(m->d_work, 0, PRG_BYTES, stream()));
+  return BG_OK;
+}
+
 int lu_factor(bg_matrix *m) {
   int st = ensure_device();
   if (!st) st = panel_init();
@@ -1576,17 +1578,11 @@ int lu_factor(bg_matrix *m) {
   // flag, and (complex64) the expanded-A scratch of the tensor-core GEMM
   size_t at_floats = 0;
   if (m->precision == BG_C64) at_floats = (size_t)2 * TC_MCHUNK * (((size_t)2 * N + 31) / 32 * 32);
-  size_t need = csz * 2 * panel_grid * 32 + csz * 64 + sizeof(double) * 2 * panel_grid + sizeof(int) * 2 * panel_grid +
-                256 + sizeof(float) * at_floats;
-  if (m->work_bytes < need) {
-    if (m->d_work) cudaFree(m->d_work);
-    m->d_work = nullptr;
-    m->work_bytes = 0;
-    BG_CUDA_TRY(cudaMalloc(&m->d_work, need));
-    m->work_bytes = need;
-  }
+  size_t need = lu_work_bytes(m) + sizeof(float) * at_floats;
+  if ((st = lu_work_alloc(m, need))) return st;
   char *w = (char *)m->d_work;
   LUWork W;
+  W.slots = (unsigned long long *)w; w += PRG_BYTES;
   W.crow = (void *)w; w += csz * 2 * panel_grid * 32;
   W.jrow = (void *)w; w += csz * 64;
   W.cval = (double *)w; w += sizeof(double) * 2 * panel_grid;
@@ -2073,25 +2069,13 @@ __global__ void k_build_perm(int N, const int *ipiv, int *perm, int use_smem) {
     for (int i = threadIdx.x; i < N; i += blockDim.x) perm[i] = p[i];
 }
 
-static size_t lu_work_bytes(bg_matrix *m) {
-  const size_t csz = m->precision == BG_C128 ? sizeof(cdl) : sizeof(cfl);
-  return csz * 2 * panel_grid * 32 + csz * 64 + sizeof(double) * 2 * panel_grid + sizeof(int) * 2 * panel_grid + 256;
-}
-
 // allocates everything the captured factor/solve touch (complex128 only)
 int lu_capture_prepare(bg_matrix *m) {
   int st = ensure_device();
   if (!st) st = panel_init();
   if (st) return st;
   if (m->precision != BG_C128) { set_error("batched sweeps factor complex128 matrices"); return BG_ERR_ARG; }
-  size_t need = lu_work_bytes(m);
-  if (m->work_bytes < need) {
-    if (m->d_work) cudaFree(m->d_work);
-    m->d_work = nullptr;
-    m->work_bytes = 0;
-    BG_CUDA_TRY(cudaMalloc(&m->d_work, need));
-    m->work_bytes = need;
-  }
+  if ((st = lu_work_alloc(m, lu_work_bytes(m)))) return st;
   int N = m->N;
   if (!m->d_perm) BG_CUDA_TRY(cudaMalloc(&m->d_perm, sizeof(int) * (N + 2 * ((N + TV_B - 1) / TV_B) + 8)));
   BG_CUDA_TRY(cudaMemsetAsync(m->d_perm + N, 0, sizeof(int) * (2 * ((N + TV_B - 1) / TV_B) + 8), stream()));
@@ -2111,6 +2095,7 @@ int lu_factor_enqueue(bg_matrix *m) {
   int N = m->N;
   char *w = (char *)m->d_work;
   LUWork W;
+  W.slots = (unsigned long long *)w; w += PRG_BYTES;
   W.crow = (void *)w; w += sizeof(cdl) * 2 * panel_grid * 32;
   W.jrow = (void *)w; w += sizeof(cdl) * 64;
   W.cval = (double *)w; w += sizeof(double) * 2 * panel_grid;
@@ -2129,7 +2114,7 @@ int lu_factor_enqueue(bg_matrix *m) {
 // device address of the factorisation status of the last captured factor
 // (LAPACK info; 0 = ok) and of the triangular sweeps' sticky error word
 int *lu_capture_info_ptr(bg_matrix *m) {
-  char *w = (char *)m->d_work + sizeof(cdl) * 2 * panel_grid * 32 + sizeof(cdl) * 64 +
+  char *w = (char *)m->d_work + PRG_BYTES + sizeof(cdl) * 2 * panel_grid * 32 + sizeof(cdl) * 64 +
             sizeof(double) * 2 * panel_grid + sizeof(int) * 2 * panel_grid;
   return (int *)w;
 }
