@@ -41,8 +41,8 @@ namespace bg {
 
 __global__ void k_batch_status(const int *info, const int *solve_err, int *acc) {
   if (threadIdx.x == 0) {
-    if (*info) atomicMax(acc, *info);
-    if (*solve_err) atomicMax(acc + 1, 1);
+    if (info[0]) atomicMax(acc, info[0]);
+    if (info[1] || *solve_err) atomicMax(acc + 1, 1);   // a wait of the factorisation or the sweeps ran out
   }
 }
 

@@ -34,6 +34,7 @@
 #include <cstdio>
 
 #include "internal.h"
+#include "tcgen05.cuh"
 
 namespace bg {
 
@@ -43,7 +44,6 @@ namespace bg {
 #define TC_GROUP 16          // row blocks per raster group
 #define TC_THREADS 192       // producer warp, MMA warp, 4 epilogue warps
 #define TC_A_BYTES (TC_BM * TC_BK * 4)
-#define TC_SPIN_LIMIT (1u << 26)
 
 template <int BN>
 struct TcCfg {
@@ -60,46 +60,6 @@ struct TcArgs {
   int *err;              // device error flag
   int ntm, ntn;          // row and column blocks
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes));
-}
-// bounded wait on phase parity; returns false on timeout
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < TC_SPIN_LIMIT; it++) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(addr), "r"(parity));
-    if (done) return true;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// K-major, 128-byte swizzle shared-memory matrix descriptor (sm_100 UMMA):
-// start>>4 in [0,14), LBO (unused for swizzled K-major) = 1 in [16,30),
-// SBO = 1024 B (one 8-row swizzle atom) >> 4 in [32,46), version 1 in [46,48),
-// layout SWIZZLE_128B = 2 in [61,64).
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
 
 // instruction descriptor, kind::tf32: D f32 (bits 4-5 = 1), A/B tf32 (2 at
 // bits 7-9 and 10-12), both K-major, N>>3 at 17-22, M>>4 at 24-28
@@ -299,22 +259,6 @@ __global__ void __launch_bounds__(256) k_expand_a(int M, int K, const float2 *A,
 }
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*PFN_encodeTiled)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                    const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static PFN_encodeTiled get_encode() {
-  static PFN_encodeTiled fn = nullptr;
-  if (!fn) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = (PFN_encodeTiled)p;
-  }
-  return fn;
-}
-
 // 2D fp32 tensor map over a row-major (rows x cols) array with leading
 // dimension ld floats; box = 32 floats (128 B, swizzled) x box_rows (<= 256)
 static int make_map(CUtensorMap *map, const float *base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_rows) {

@@ -18,6 +18,7 @@
 #include <mutex>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <vector>
@@ -35,6 +36,9 @@ template <> struct CxT<cdl> { typedef double R; };
 template <> struct CxT<cfl> { typedef float R; };
 
 // tensor-core complex-FP32 GEMM (gemm_tc.cu)
+size_t zgemm_i8_bytes(int M, int N, int K);
+int zgemm_i8(int M, int N, int K, const void *A, size_t lda, const void *B, size_t ldb, void *C, size_t ldc, void *work,
+             size_t bytes, int *err);
 int cgemm_sub_tf32(int M, int N, int K, const void *A, size_t lda, const void *B, size_t ldb, void *C, size_t ldc,
                    float *At, int *err);
 
@@ -364,9 +368,35 @@ static int zgemm_launch(int M, int N, int K, const cdl *A, size_t lda, const cdl
   return BG_OK;
 }
 
+// scratch of the INT8 path, set around the calls that may take it
+struct I8Scratch {
+  void *p;
+  size_t bytes;
+  int *err;
+};
+static thread_local I8Scratch *t_i8 = nullptr;
+// Which products go there, from measured times in us: 128 x 32 tiles in waves of
+// 148 at 0.078 us per column of K and 1.5 us of epilogue, 25 us of launches,
+// splitting at 64 bytes per element of A and B and 3 TB/s; the FP64 tiles at 28
+// TFLOP/s.  Measured INT8 / FP64: 2048 x 1024 x 128 90 / 90 us, 4096 x 4096 x
+// 128 370 / 640, 1024^3 196 / 304, 9936 x 9936 x 1024 13.2 / 24.9 ms; 3968 x 128
+// x 128 50 / 27.
+static bool i8_takes(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return false;
+  const double tiles = std::ceil((double)M / 128) * std::ceil((double)N / 32);
+  const double split = 25.0 + ((double)M + N) * K * (64 / 3e6);
+  const double i8 = std::ceil(tiles / 148) * (0.078 * K + 1.5) + split, fp64 = 8.0 * M * (double)N * K / 28e6;
+  return i8 < 0.95 * fp64;
+}
+
 static int zgemm_sub(int M, int N, int K, const cdl *A, size_t lda, const cdl *B, size_t ldb, cdl *C, size_t ldc) {
   if (M <= 0 || N <= 0 || K <= 0) return BG_OK;
   prof_start(PROF_GEMM);
+  if (t_i8 && i8_takes(M, N, K) && zgemm_i8_bytes(M, N, K) <= t_i8->bytes) {
+    int st = zgemm_i8(M, N, K, A, lda, B, ldb, C, ldc, t_i8->p, t_i8->bytes, t_i8->err);
+    prof_stop(PROF_GEMM, 8.0 * M * (double)N * K);
+    return st;
+  }
   // few 64 x 64 tiles leave SMs without work (both sides measured, see k_zgemm_small)
   const long tiles = (long)((M + 63) / 64) * ((N + 63) / 64);
   int st = tiles <= ZG_SMALL ? zgemm_small(M, N, K, A, lda, B, ldb, C, ldc)
@@ -1568,6 +1598,12 @@ static int lu_work_alloc(bg_matrix *m, size_t need) {
   return BG_OK;
 }
 
+// scratch of the INT8 products of a factorisation (0: every product is too small for them)
+static size_t i8_factor_bytes(int N) {
+  const int h = N / 2 + LU_BLOCK;
+  return i8_takes(N, h, h) ? zgemm_i8_bytes(N, h, h) : 0;
+}
+
 int lu_factor(bg_matrix *m) {
   int st = ensure_device();
   if (!st) st = panel_init();
@@ -1592,7 +1628,16 @@ int lu_factor(bg_matrix *m) {
   w += 256;
   BG_CUDA_TRY(cudaMemsetAsync(W.info, 0, 2 * sizeof(int), stream()));
   if (m->precision == BG_C128) {
-    if ((st = getrf_rec<cdl>(m, W, 0, N))) return st;
+    I8Scratch sc{nullptr, i8_factor_bytes(N), W.info + 1};
+    if (sc.bytes && cudaMallocAsync(&sc.p, sc.bytes, stream()) != cudaSuccess) {
+      cudaGetLastError();      // no room: the FP64 tiles need no scratch
+      sc.p = nullptr;
+    }
+    t_i8 = sc.p ? &sc : nullptr;
+    st = getrf_rec<cdl>(m, W, 0, N);
+    t_i8 = nullptr;
+    if (sc.p) cudaFreeAsync(sc.p, stream());
+    if (st) return st;
   } else {
     TcScratch sc;
     sc.At = (float *)w;
@@ -1617,7 +1662,27 @@ int lu_factor(bg_matrix *m) {
 int zgemm_sub_device(int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C, int ldc) {
   int st = ensure_device();
   if (st) return st;
-  return zgemm_sub(M, N, K, (const cdl *)A, (size_t)lda, (const cdl *)B, (size_t)ldb, (cdl *)C, (size_t)ldc);
+  I8Scratch sc{nullptr, 0, nullptr};
+  if (M > 0 && N > 0 && K > 0 && i8_takes(M, N, K)) {
+    sc.bytes = zgemm_i8_bytes(M, N, K);
+    if (cudaMallocAsync(&sc.p, sc.bytes + 256, stream()) != cudaSuccess) {
+      cudaGetLastError();      // no scratch: the FP64 tiles need none
+      sc.p = nullptr;
+    }
+  }
+  if (!sc.p) return zgemm_sub(M, N, K, (const cdl *)A, (size_t)lda, (const cdl *)B, (size_t)ldb, (cdl *)C, (size_t)ldc);
+  sc.err = (int *)((char *)sc.p + sc.bytes);
+  cudaError_t e = cudaMemsetAsync(sc.err, 0, sizeof(int), stream());
+  t_i8 = &sc;
+  st = zgemm_sub(M, N, K, (const cdl *)A, (size_t)lda, (const cdl *)B, (size_t)ldb, (cdl *)C, (size_t)ldc);
+  t_i8 = nullptr;
+  int h = 0;
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, sc.err, sizeof(int), cudaMemcpyDeviceToHost, stream());
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream());
+  cudaFreeAsync(sc.p, stream());
+  if (!st && e != cudaSuccess) { set_error("zgemm: %s", cudaGetErrorString(e)); st = BG_ERR_CUDA; }
+  if (!st && h) { set_error("zgemm: a tensor-core wait timed out (code %d)", h); st = BG_ERR_CUDA; }
+  return st;
 }
 
 // =========================================================================
@@ -1911,17 +1976,38 @@ int lu_solve_many(bg_matrix *m, void *dB, size_t ldb, int nrhs) {
   int w = std::min(chunk, nrhs);
   if (w <= 0) return BG_OK;
   BG_CUDA_TRY(cudaMallocAsync((void **)&T, sizeof(cdl) * (size_t)N * w, stream()));
-  int st = BG_OK;
+  // scratch of the INT8 products, where some are large enough for them
+  const int h = N / 2 + TRS_MAX;
+  I8Scratch sc{nullptr, i8_takes(h, w, h) ? zgemm_i8_bytes(h, w, h) : 0, nullptr};
+  if (sc.bytes && cudaMallocAsync(&sc.p, sc.bytes + 256, stream()) != cudaSuccess) {
+    cudaGetLastError();
+    sc.p = nullptr;
+  }
+  int st = BG_OK, tcerr = 0;
+  if (sc.p) {
+    sc.err = (int *)((char *)sc.p + sc.bytes);
+    if (cudaMemsetAsync(sc.err, 0, sizeof(int), stream()) != cudaSuccess) { cudaGetLastError(); st = BG_ERR_CUDA; }
+    t_i8 = &sc;
+  }
   for (int r0 = 0; r0 < nrhs && !st; r0 += chunk) {
     int nr = std::min(chunk, nrhs - r0);
     cdl *Bp = B + (size_t)r0 * ldb;
     k_gather_rows<cdl><<<dim3((N + 255) / 256, nr), 256, 0, stream()>>>(N, nr, m->d_perm, Bp, ldb, T, N);
-    BG_LAUNCHED();
+    if (cudaGetLastError() != cudaSuccess) { set_error("lu_solve_many: launch failed"); st = BG_ERR_CUDA; break; }
+    g_launches++;
     if ((st = trsm<cdl>(N, nr, A, m->ld, T, N, 0))) break;
     if ((st = trsm<cdl>(N, nr, A, m->ld, T, N, 1))) break;
     cudaError_t e = cudaMemcpy2DAsync(Bp, sizeof(cdl) * ldb, T, sizeof(cdl) * N, sizeof(cdl) * N, nr,
                                       cudaMemcpyDeviceToDevice, stream());
     if (e != cudaSuccess) { set_error("lu_solve_many: %s", cudaGetErrorString(e)); st = BG_ERR_CUDA; }
+  }
+  t_i8 = nullptr;
+  if (sc.p) {
+    cudaError_t e = cudaMemcpyAsync(&tcerr, sc.err, sizeof(int), cudaMemcpyDeviceToHost, stream());
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream());
+    cudaFreeAsync(sc.p, stream());
+    if (!st && e != cudaSuccess) { set_error("lu_solve_many: %s", cudaGetErrorString(e)); st = BG_ERR_CUDA; }
+    if (!st && tcerr) { set_error("lu_solve_many: a tensor-core wait timed out (code %d)", tcerr); st = BG_ERR_CUDA; }
   }
   cudaFreeAsync(T, stream());
   return st;
@@ -2075,8 +2161,11 @@ int lu_capture_prepare(bg_matrix *m) {
   if (!st) st = panel_init();
   if (st) return st;
   if (m->precision != BG_C128) { set_error("batched sweeps factor complex128 matrices"); return BG_ERR_ARG; }
-  if ((st = lu_work_alloc(m, lu_work_bytes(m)))) return st;
   int N = m->N;
+  if (lu_work_alloc(m, lu_work_bytes(m) + i8_factor_bytes(N)) != BG_OK) {
+    cudaGetLastError();        // no room for the INT8 products' scratch: without
+    if ((st = lu_work_alloc(m, lu_work_bytes(m)))) return st;
+  }
   if (!m->d_perm) BG_CUDA_TRY(cudaMalloc(&m->d_perm, sizeof(int) * (N + 2 * ((N + TV_B - 1) / TV_B) + 8)));
   BG_CUDA_TRY(cudaMemsetAsync(m->d_perm + N, 0, sizeof(int) * (2 * ((N + TV_B - 1) / TV_B) + 8), stream()));
   BG_CUDA_TRY(cudaStreamSynchronize(stream()));
@@ -2101,8 +2190,12 @@ int lu_factor_enqueue(bg_matrix *m) {
   W.cval = (double *)w; w += sizeof(double) * 2 * panel_grid;
   W.cidx = (int *)w; w += sizeof(int) * 2 * panel_grid;
   W.info = (int *)w;
+  w += 256;
   BG_CUDA_TRY(cudaMemsetAsync(W.info, 0, 2 * sizeof(int), stream()));
+  I8Scratch sc{w, i8_factor_bytes(N), W.info + 1};
+  if (sc.bytes && m->work_bytes >= lu_work_bytes(m) + sc.bytes) t_i8 = &sc;
   int st = getrf_rec<cdl>(m, W, 0, N);
+  t_i8 = nullptr;
   if (st) return st;
   int use_smem = (size_t)8 * N <= 200 * 1024;
   k_build_perm<<<1, 1024, use_smem ? 8 * (size_t)N : 0, stream()>>>(N, m->d_ipiv, m->d_perm, use_smem);
