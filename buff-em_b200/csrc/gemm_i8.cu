@@ -21,17 +21,21 @@
 // the two parts of column n.
 //
 // Kernel: persistent, tiles of 128 rows x 64 real columns, eight accumulators =
-// all 512 TMEM columns; two stages of 64 bytes of K of all 16 slices (96 KB
-// each); warp 0 loads (two TMA boxes a stage), warp 1 issues the 72 MMAs of a
-// stage, warps 2-9 hold their part of C in registers since before the
+// all 512 TMEM columns; four stages of 32 bytes of K of all 16 slices (48 KB
+// each, two contiguous copies); warp 0 loads, warp 1 issues the 36 MMAs of a
+// stage, warps 2-17 hold their part of C in registers since before the
 // accumulators are ready and combine.  Every wait is bounded; on a timeout the
 // error word is set, copies in flight are waited for and TMEM is freed.
 //
-// What bounds it: shared-memory reads, 6 KB of operands per 128 x 64 x 32 MMA
-// (48 cycles at 128 bytes, 32 of arithmetic) beside the loads.  9936 x 9936 x
-// 1024: FP64 tiles 24.9 ms (32.5 TFLOP/s) -> 13.3 ms (61); factorisation of N =
-// 19,872: products 660 -> 378 ms.  Error of 256 x 256 x 512 products against
-// 80-bit sums: rms 1.7e-16 of the largest entry with FP64 tiles, 2.2e-17 here.
+// What bounds it: shared memory, 6 KB of operands read per 128 x 64 x 32 MMA and
+// 48 KB written per 36 of them, 57 cycles an MMA at 128 bytes where the
+// arithmetic takes 32 (a 64-column MMA alone runs at 3.04 of 4.56 POP/s), and
+// the combination, which no second set of accumulators can hide (about 4 us a
+// tile).  A CTA pair (256 rows, half of B in each) was slower: 14.9 ms where
+// this takes 12.9.  9936 x 9936 x 1024: FP64 tiles 24.9 ms (32.5 TFLOP/s) -> 12.9
+// ms (62.6); 4096 x 4096 x 128: 0.64 -> 0.37 ms.  Factorisation of N = 19,872:
+// products 660 -> 367 ms.  Error of 256 x 256 x 512 products against 80-bit
+// sums: rms 1.7e-16 of the largest entry with FP64 tiles, 2.2e-17 here.
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -49,17 +53,18 @@ struct z2i { double r, i; };
 #define I8_S 8                    // digits per number
 #define I8_BM 128                 // rows of a tile
 #define I8_BN 64                  // real columns of a tile (32 complex)
-#define I8_BK 64                  // bytes of K per stage (one 64-byte swizzle row)
-#define I8_STAGES 2
+#define I8_BK 32                  // bytes of K per stage: one MMA deep, one 32-byte swizzle row
+#define I8_STAGES 4
 #define I8_GROUP 16               // row blocks per raster group
-#define I8_THREADS 320
+#define I8_THREADS 576
 #define I8_A_BYTES (I8_S * I8_BM * I8_BK)
 #define I8_B_BYTES (I8_S * I8_BN * I8_BK)
 #define I8_STAGE (I8_A_BYTES + I8_B_BYTES)
 #define I8_SMEM (I8_STAGES * I8_STAGE + 1024 + 256)
 
 struct I8Args {
-  int M, N, K2;                   // rows, complex columns, real reduction length
+  int M, N, nk;                   // rows, complex columns, K blocks
+  const int8_t *A, *B;            // digit blocks
   z2i *C;
   size_t ldc;
   const double *sa, *sb;          // scale of each row of A and column of B
@@ -82,7 +87,7 @@ __device__ __forceinline__ double pair_to_double(int a, int b) {
 }
 
 __global__ void __launch_bounds__(I8_THREADS, 1)
-    k_zgemm_i8(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, I8Args P) {
+    k_zgemm_i8(const I8Args P) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *ring = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t *full = (uint64_t *)(ring + I8_STAGES * I8_STAGE);
@@ -93,13 +98,13 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
   __shared__ int s_issued, s_consumed;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nk = (P.K2 + I8_BK - 1) / I8_BK;
+  const int nk = P.nk;
   const int ntiles = P.ntm * P.ntn;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < I8_STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(acc_full, 1);
-    mbar_init(acc_empty, 8);
+    mbar_init(acc_empty, 16);
     mbar_init(mma_done, 1);
     s_fail = 0;
     s_issued = 0;
@@ -127,8 +132,8 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
           if (kc >= I8_STAGES && !mbar_wait(&empty[s], ((kc / I8_STAGES) - 1) & 1)) { s_fail = 1; break; }
           unsigned char *sa = ring + s * I8_STAGE;
           mbar_expect_tx(&full[s], I8_STAGE);
-          tma_load_3d(sa, &mapA, kb * I8_BK, tm * I8_BM, 0, &full[s]);
-          tma_load_3d(sa + I8_A_BYTES, &mapB, kb * I8_BK, tn * I8_BN, 0, &full[s]);
+          bulk_load(sa, P.A + ((size_t)tm * nk + kb) * I8_A_BYTES, I8_A_BYTES, &full[s]);
+          bulk_load(sa + I8_A_BYTES, P.B + ((size_t)tn * nk + kb) * I8_B_BYTES, I8_B_BYTES, &full[s]);
           s_issued = kc + 1;
         }
       }
@@ -148,22 +153,19 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
           if (!mbar_wait(&full[s], (kc / I8_STAGES) & 1)) { s_fail = 2; break; }
           asm volatile("tcgen05.fence::after_thread_sync;");
           const uint32_t sa = smem_u32(ring + s * I8_STAGE), sb = sa + I8_A_BYTES;
-          const uint64_t da0 = sw64_desc(sa), db0 = sw64_desc(sb);
+          const uint64_t da0 = sw32_desc(sa), db0 = sw32_desc(sb);
 #pragma unroll
-          for (int k = 0; k < I8_BK / 32; k++) {
+          for (int a = 0; a < I8_S; a++) {
 #pragma unroll
-            for (int a = 0; a < I8_S; a++) {
-#pragma unroll
-              for (int b = 0; b < I8_S - a; b++) {
-                const uint64_t da = da0 + ((a * I8_BM * I8_BK + k * 32) >> 4);
-                const uint64_t db = db0 + ((b * I8_BN * I8_BK + k * 32) >> 4);
-                const uint32_t acc = (kb > 0 || k > 0 || a > 0) ? 1u : 0u;   // group a + b is first met at a = 0
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-                    ::"r"(tmem + (uint32_t)((a + b) * I8_BN)), "l"(da), "l"(db), "r"(idesc), "r"(acc));
-              }
+            for (int b = 0; b < I8_S - a; b++) {
+              const uint64_t da = da0 + ((a * I8_BM * I8_BK) >> 4);
+              const uint64_t db = db0 + ((b * I8_BN * I8_BK) >> 4);
+              const uint32_t acc = (kb > 0 || a > 0) ? 1u : 0u;   // group a + b is first met at a = 0
+              asm volatile(
+                  "{\n\t.reg .pred p;\n\t"
+                  "setp.ne.b32 p, %4, 0;\n\t"
+                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+                  ::"r"(tmem + (uint32_t)((a + b) * I8_BN)), "l"(da), "l"(db), "r"(idesc), "r"(acc));
             }
           }
           mma_commit(&empty[s]);
@@ -177,25 +179,25 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
       if (!mbar_wait(mma_done, 0) && !s_fail) s_fail = 5;
     }
   } else {
-    // warps 2 .. 9: TMEM lanes 32 (warp % 4) .. + 31, 16 complex columns each
+    // warps 2 .. 17: TMEM lanes 32 (warp % 4) .. + 31, 8 complex columns each
     const int q = warp & 3, h = (warp - 2) >> 2;
     int i = 0;
     for (int t = blockIdx.x; t < ntiles && !s_fail; t += gridDim.x, i++) {
       int tm, tn;
       i8_tile(P, t, tm, tn);
-      const int row = tm * I8_BM + q * 32 + lane, col0 = tn * (I8_BN / 2) + 16 * h;
+      const int row = tm * I8_BM + q * 32 + lane, col0 = tn * (I8_BN / 2) + 8 * h;
       z2i *pc = P.C + (size_t)col0 * P.ldc + row;
-      z2i cv[16];
+      z2i cv[8];
       const double sa = row < P.M ? P.sa[row] : 0.0;
 #pragma unroll
-      for (int j = 0; j < 16; j++)
+      for (int j = 0; j < 8; j++)
         cv[j] = row < P.M && col0 + j < P.N ? pc[(size_t)j * P.ldc] : z2i{0.0, 0.0};
       if (!mbar_wait(acc_full, i & 1)) { s_fail = 3; break; }
       asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-      for (int c = 0; c < 16; c += 2) {      // two complex = four real columns at a time
+      for (int c = 0; c < 8; c += 2) {      // two complex = four real columns at a time
         uint32_t r[8][4];
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(32 * h + 2 * c);
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(16 * h + 2 * c);
 #pragma unroll
         for (int g = 0; g < I8_S; g++)
           asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
@@ -289,16 +291,24 @@ __global__ void __launch_bounds__(128) k_i8_rowmax(int M, int K, const z2i *A, s
   atomicMax(mx + m, x);
 }
 
-// slices of A: S[s][m][2k, 2k + 1] = digit s of (re, im); a thread takes one
-// row and 16 columns, 32 bytes a slice
+// Digit blocks: 32 bytes of K (16 columns, re and im interleaved) of 128 rows of
+// A or 64 rows of B, [digit][row][32 bytes], one contiguous piece per block in the
+// order the stages read them, the two 16-byte halves of a row exchanged where
+// bit 2 of the row is set (the tensor core's 32-byte swizzle).  Loads are then
+// whole lines; as planes of rows, a stage read half a line per row.
+__device__ __forceinline__ size_t digit_row(int row, int kb, int nk, int rows) {
+  return ((size_t)(row / rows) * nk + kb) * (I8_S * rows * I8_BK) + (row % rows) * I8_BK;
+}
+
+// a thread takes one row and 16 columns
 __global__ void __launch_bounds__(128) k_i8_slice_a(int M, int K, const z2i *A, size_t lda,
-                                                    const unsigned long long *mx, int8_t *S, size_t pitch,
-                                                    size_t plane, double *sa) {
+                                                    const unsigned long long *mx, int8_t *S, int nk, double *sa) {
   const int m = blockIdx.x * 128 + threadIdx.x, k0 = blockIdx.y * 16;
   if (m >= M) return;
   const unsigned long long top = mx[m];
   const DigitScale sc = split_scale(top);
   if (blockIdx.y == 0) sa[m] = digit_scale(top);
+  int8_t *p = S + digit_row(m, blockIdx.y, nk, I8_BM);
 #pragma unroll
   for (int h = 0; h < 2; h++) {
     uint32_t w[4][8];
@@ -314,16 +324,16 @@ __global__ void __launch_bounds__(128) k_i8_slice_a(int M, int K, const z2i *A, 
                                        digits(to_int(a[2 * i + 1].r, sc)), digits(to_int(a[2 * i + 1].i, sc))};
       transpose8(d, w[i]);
     }
-    int8_t *p = S + (size_t)m * pitch + 2 * k0 + 16 * h;
+    const int o = 16 * (h ^ ((m >> 2) & 1));
 #pragma unroll
-    for (int s = 0; s < I8_S; s++) *(uint4 *)(p + s * plane) = make_uint4(w[0][s], w[1][s], w[2][s], w[3][s]);
+    for (int s = 0; s < I8_S; s++)
+      *(uint4 *)(p + s * (I8_BM * I8_BK) + o) = make_uint4(w[0][s], w[1][s], w[2][s], w[3][s]);
   }
 }
 
 // slices of B, K <= I8_KC: a block takes a column; rows 2n: (br, -bi), 2n + 1: (bi, br)
 #define I8_KC 1024
-__global__ void __launch_bounds__(128) k_i8_slice_b(int K, const z2i *B, size_t ldb, int8_t *S, size_t pitch,
-                                                    size_t plane, double *sb) {
+__global__ void __launch_bounds__(128) k_i8_slice_b(int K, const z2i *B, size_t ldb, int8_t *S, int nk, double *sb) {
   const int n = blockIdx.x, t = threadIdx.x;
   const z2i *b = B + (size_t)n * ldb;
   z2i v[4][2];
@@ -346,7 +356,7 @@ __global__ void __launch_bounds__(128) k_i8_slice_b(int K, const z2i *B, size_t 
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int k = 2 * t + 256 * i;
-    if ((size_t)2 * k >= pitch) continue;
+    if (k / 16 >= nk) continue;
     long long r[2], m[2];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -358,41 +368,30 @@ __global__ void __launch_bounds__(128) k_i8_slice_b(int K, const z2i *B, size_t 
     const unsigned long long d1[4] = {digits(m[0]), digits(r[0]), digits(m[1]), digits(r[1])};
     transpose8(d0, w0);
     transpose8(d1, w1);
-    int8_t *p = S + (size_t)(2 * n) * pitch + 2 * k;
+    int8_t *p = S + digit_row(2 * n, k / 16, nk, I8_BN);
+    const int o = 2 * (k % 16) ^ (((2 * n) >> 2) & 1) * 16;      // rows 2n and 2n + 1: the same half
 #pragma unroll
     for (int s = 0; s < I8_S; s++) {
-      *(uint32_t *)(p + s * plane) = w0[s];
-      *(uint32_t *)(p + s * plane + pitch) = w1[s];
+      *(uint32_t *)(p + s * (I8_BN * I8_BK) + o) = w0[s];
+      *(uint32_t *)(p + s * (I8_BN * I8_BK) + I8_BK + o) = w1[s];
     }
   }
 }
 
 // ------------------------------------------------------------------ host side
-// planes of digits (cols bytes a row, padded to pitch), box = 64 bytes x box_rows x all planes
-static int make_i8_map(CUtensorMap *map, const int8_t *base, uint64_t cols, uint64_t rows, uint64_t pitch,
-                       uint64_t plane, uint32_t box_rows) {
-  PFN_encodeTiled enc = get_encode();
-  if (!enc) { set_error("cuTensorMapEncodeTiled unavailable"); return BG_ERR_CUDA; }
-  cuuint64_t dims[3] = {cols, rows, I8_S};
-  cuuint64_t strides[2] = {pitch, plane};
-  cuuint32_t box[3] = {I8_BK, box_rows, I8_S};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, (void *)base, dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled failed (%d)", (int)r); return BG_ERR_CUDA; }
-  return BG_OK;
-}
-
 #define I8_MC 8192                // rows of A and complex columns of B sliced at a time at most
 #define I8_NC 4096
 
 static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// digits of r rows (in whole blocks) and k columns
+static size_t digit_bytes(int r, int rows, int k) {
+  return up256((size_t)((r + rows - 1) / rows) * ((k + 15) / 16) * (I8_S * rows * I8_BK));
+}
 // scratch for products of at most M x N x K
 size_t zgemm_i8_bytes(int M, int N, int K) {
-  const size_t mc = std::min(M, I8_MC), nc = std::min(N, I8_NC), pitch = ((size_t)2 * std::min(K, I8_KC) + 31) / 32 * 32;
-  return up256(I8_S * mc * pitch) + up256(I8_S * 2 * nc * pitch) + up256(8 * mc) * 2 + up256(8 * nc);
+  const int mc = std::min(M, I8_MC), nc = std::min(N, I8_NC), kc = std::min(K, I8_KC);
+  return digit_bytes(mc, I8_BM, kc) + digit_bytes(2 * nc, I8_BN, kc) + up256(8 * mc) * 2 + up256(8 * nc);
 }
 
 // C -= A B with the scratch `work` of `bytes`; err: device int, nonzero after a failed wait
@@ -408,39 +407,30 @@ int zgemm_i8(int M, int N, int K, const void *Av, size_t lda, const void *Bv, si
   if (zgemm_i8_bytes(M, N, K) > bytes) { set_error("zgemm: scratch too small"); return BG_ERR_STATE; }
   const z2i *A = (const z2i *)Av, *B = (const z2i *)Bv;
   z2i *C = (z2i *)Cv;
-  const size_t mc = std::min(M, I8_MC), nc = std::min(N, I8_NC), pitch0 = ((size_t)2 * std::min(K, I8_KC) + 31) / 32 * 32;
+  const int mc = std::min(M, I8_MC), nc = std::min(N, I8_NC), kc = std::min(K, I8_KC);
   char *w = (char *)work;
-  int8_t *Sa = (int8_t *)w; w += up256(I8_S * mc * pitch0);
-  int8_t *Sb = (int8_t *)w; w += up256(I8_S * 2 * nc * pitch0);
+  int8_t *Sa = (int8_t *)w; w += digit_bytes(mc, I8_BM, kc);
+  int8_t *Sb = (int8_t *)w; w += digit_bytes(2 * nc, I8_BN, kc);
   unsigned long long *mx = (unsigned long long *)w; w += up256(8 * mc);
   double *sa = (double *)w; w += up256(8 * mc);
   double *sb = (double *)w;
-  int st;
-  for (int k0 = 0; k0 < K; k0 += I8_KC) {
-    const int kk = std::min(I8_KC, K - k0);
-    const size_t pitch = ((size_t)2 * kk + 31) / 32 * 32;
-    for (int n0 = 0; n0 < N; n0 += (int)nc) {
-      const int nn = std::min((int)nc, N - n0);
-      const size_t planeB = pitch * 2 * nn;
-      k_i8_slice_b<<<nn, 128, 0, stream()>>>(kk, B + k0 + (size_t)n0 * ldb, ldb, Sb, pitch, planeB, sb);
+  for (int k0 = 0; k0 < K; k0 += kc) {
+    const int kk = std::min(kc, K - k0), nk = (kk + 15) / 16;
+    for (int n0 = 0; n0 < N; n0 += nc) {
+      const int nn = std::min(nc, N - n0);
+      k_i8_slice_b<<<nn, 128, 0, stream()>>>(kk, B + k0 + (size_t)n0 * ldb, ldb, Sb, nk, sb);
       BG_LAUNCHED();
-      CUtensorMap mB;
-      if ((st = make_i8_map(&mB, Sb, 2 * kk, 2 * (uint64_t)nn, pitch, planeB, I8_BN))) return st;
-      for (int m0 = 0; m0 < M; m0 += (int)mc) {
-        const int mm = std::min((int)mc, M - m0);
+      for (int m0 = 0; m0 < M; m0 += mc) {
+        const int mm = std::min(mc, M - m0);
         const z2i *Am = A + m0 + (size_t)k0 * lda;
-        const size_t planeA = pitch * mm;
         BG_CUDA_TRY(cudaMemsetAsync(mx, 0, 8 * (size_t)mm, stream()));
         k_i8_rowmax<<<dim3((mm + 127) / 128, (kk + 31) / 32), 128, 0, stream()>>>(mm, kk, Am, lda, mx);
         BG_LAUNCHED();
-        k_i8_slice_a<<<dim3((mm + 127) / 128, (kk + 15) / 16), 128, 0, stream()>>>(mm, kk, Am, lda, mx, Sa, pitch,
-                                                                                  planeA, sa);
+        k_i8_slice_a<<<dim3((mm + 127) / 128, nk), 128, 0, stream()>>>(mm, kk, Am, lda, mx, Sa, nk, sa);
         BG_LAUNCHED();
-        CUtensorMap mA;
-        if ((st = make_i8_map(&mA, Sa, 2 * kk, mm, pitch, planeA, I8_BM))) return st;
-        I8Args P{mm, nn, 2 * kk, C + m0 + (size_t)n0 * ldc, ldc, sa, sb, err, (mm + I8_BM - 1) / I8_BM,
-                 (2 * nn + I8_BN - 1) / I8_BN};
-        k_zgemm_i8<<<std::min(P.ntm * P.ntn, sms), I8_THREADS, I8_SMEM, stream()>>>(mA, mB, P);
+        I8Args P{mm, nn, nk, Sa, Sb, C + m0 + (size_t)n0 * ldc, ldc, sa, sb, err,
+                 (mm + I8_BM - 1) / I8_BM, (2 * nn + I8_BN - 1) / I8_BN};
+        k_zgemm_i8<<<std::min(P.ntm * P.ntn, sms), I8_THREADS, I8_SMEM, stream()>>>(P);
         BG_LAUNCHED();
       }
     }

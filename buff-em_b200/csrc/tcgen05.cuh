@@ -6,7 +6,7 @@
 
 namespace bg {
 
-#define TC_SPIN_LIMIT (1u << 26)
+#define TC_WAIT_CYCLES (1ll << 32)   // two seconds and more: no wait of a sound run comes near it
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -22,7 +22,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
 // bounded wait on phase parity; returns false on timeout
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
   uint32_t addr = smem_u32(bar);
-  for (uint32_t it = 0; it < TC_SPIN_LIMIT; it++) {
+  const long long t0 = clock64();
+  do {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -31,7 +32,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity) {
         : "=r"(done)
         : "r"(addr), "r"(parity));
     if (done) return true;
-  }
+  } while (clock64() - t0 < TC_WAIT_CYCLES);
   return false;
 }
 
@@ -41,11 +42,12 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
       ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
       : "memory");
 }
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(smem_u32(dst)), "l"((uint64_t)map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
+// contiguous bytes (a multiple of 16, both ends 16-byte aligned)
+__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   smem_u32(dst)),
+               "l"((uint64_t)__cvta_generic_to_global(src)), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 // arrive on bar when every MMA issued so far by this thread has finished
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
@@ -54,15 +56,15 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 
 // K-major shared-memory matrix descriptors (sm_100 UMMA): start>>4 in [0,14),
 // LBO (unused for swizzled K-major) = 1 in [16,30), SBO = one 8-row swizzle
-// atom (1024 or 512 bytes) >> 4 in [32,46), version 1 in [46,48), layout in
-// [61,64): SWIZZLE_128B = 2, SWIZZLE_64B = 4.
+// atom (1024 or 256 bytes) >> 4 in [32,46), version 1 in [46,48), layout in
+// [61,64): SWIZZLE_128B = 2, SWIZZLE_32B = 6.
 __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
   return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-__device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) |
-         ((uint64_t)1 << 46) | ((uint64_t)4 << 61);
+__device__ __forceinline__ uint64_t sw32_desc(uint32_t saddr) {
+  return (uint64_t)((saddr >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(256 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)6 << 61);
 }
 
 // ------------------------------------------------------------------ host side
