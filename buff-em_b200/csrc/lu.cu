@@ -31,6 +31,34 @@ namespace bg {
 
 struct cdl { double r, i; };
 struct cfl { float r, i; };
+// The kernels of the factorisation's chain follow one another within a few
+// microseconds of work: each is launched while its predecessor still runs
+// (programmatic dependent launch) and starts with pdl_enter, which lets its own
+// successor launch and then waits until the predecessor has finished and its
+// writes are visible.  Factor and solve 18.6 -> 17.9 ms at N = 4,092, small body
+// of N = 1,350 4.87 -> 4.79 ms.  Only where one factorisation has the device to
+// itself (t_pdl): CTAs that wait take room from the other streams of a batched
+// sweep (217 -> 246 ms).
+static thread_local bool t_pdl = false;
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <class... P, class... A>
+static cudaError_t pdl_launch(void (*kern)(P...), dim3 grid, int threads, size_t smem, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream();
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = t_pdl;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
+
 template <class C> struct CxT;
 template <> struct CxT<cdl> { typedef double R; };
 template <> struct CxT<cfl> { typedef float R; };
@@ -104,6 +132,7 @@ template <int BM, int BN, int BK, int STAGES>
 __global__ void __launch_bounds__(GemmCfg<BM, BN, BK, STAGES>::THREADS)
     k_zgemm_sub(int M, int N, int K, const cdl *__restrict__ A, size_t lda, const cdl *__restrict__ B, size_t ldb,
                 cdl *C, size_t ldc) {
+  pdl_enter();
   using Cfg = GemmCfg<BM, BN, BK, STAGES>;
   constexpr int T = Cfg::THREADS, AP = Cfg::AP, BP = Cfg::BP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -240,6 +269,7 @@ __device__ __forceinline__ void dmma8(double (&d)[4], const double (&a)[4], cons
 __global__ void __launch_bounds__(128) k_zgemm_small(int M, int N, int K, const cdl *__restrict__ A, size_t lda,
                                                       const cdl *__restrict__ B, size_t ldb, cdl *C, size_t ldc) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_enter();
   cdl *sm = (cdl *)smem_raw;
   const int m0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
   const int tid = threadIdx.x, lane = tid & 31, wk = tid >> 5, t0 = lane & 3, t1 = lane >> 2;
@@ -340,7 +370,7 @@ static int zgemm_small(int M, int N, int K, const cdl *A, size_t lda, const cdl 
     BG_CUDA_TRY(cudaFuncSetAttribute(k_zgemm_small, cudaFuncAttributeMaxDynamicSharedMemorySize, ZS_SMEM));
     attr = true;
   }
-  k_zgemm_small<<<dim3((M + 31) / 32, (N + 31) / 32), 128, ZS_SMEM, stream()>>>(M, N, K, A, lda, B, ldb, C, ldc);
+  BG_CUDA_TRY(pdl_launch(k_zgemm_small, dim3((M + 31) / 32, (N + 31) / 32), 128, ZS_SMEM, M, N, K, A, lda, B, ldb, C, ldc));
   BG_LAUNCHED();
   return BG_OK;
 }
@@ -363,7 +393,7 @@ static int zgemm_launch(int M, int N, int K, const cdl *A, size_t lda, const cdl
   }
   dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN);
   if (grid.y > 65535) { set_error("zgemm: N too large"); return BG_ERR_ARG; }
-  kern<<<grid, Cfg::THREADS, Cfg::SMEM, stream()>>>(M, N, K, A, lda, B, ldb, C, ldc);
+  BG_CUDA_TRY(pdl_launch(kern, grid, Cfg::THREADS, Cfg::SMEM, M, N, K, A, lda, B, ldb, C, ldc));
   BG_LAUNCHED();
   return BG_OK;
 }
@@ -446,6 +476,7 @@ __device__ __forceinline__ int trs_block(int br, int bc, bool upper) {
 }
 template <class C, int CPW, bool UPPER>
 __global__ void __launch_bounds__(TRS_WARPS * 32) k_trsm_leaf(int n, int m, const C *T, size_t ldt, C *B, size_t ldb) {
+  pdl_enter();
   typedef typename CxT<C>::R R;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *Ts = (C *)smem_raw;
@@ -569,7 +600,8 @@ static int trsm_launch(int n, int m, const C *T, size_t ldt, C *B, size_t ldb) {
   }
   const int cols = TRS_WARPS * CPW;
   prof_start(PROF_TRSM);
-  k_trsm_leaf<C, CPW, UPPER><<<(m + cols - 1) / cols, TRS_WARPS * 32, trsm_smem<C>(), stream()>>>(n, m, T, ldt, B, ldb);
+  BG_CUDA_TRY(pdl_launch(k_trsm_leaf<C, CPW, UPPER>, dim3((m + cols - 1) / cols), TRS_WARPS * 32, trsm_smem<C>(), n, m, T,
+                         ldt, B, ldb));
   BG_LAUNCHED();
   prof_stop(PROF_TRSM, 4.0 * n * (double)n * m);
   return BG_OK;
@@ -1001,6 +1033,7 @@ __global__ void __launch_bounds__(TMAX + 32) k_panel_rf(PanelArgs<C> P) {
   // finished columns of this thread's row: column c at Lrow[c * Lstep]
   C *Lrow = top ? &S.Lt[0][lane] : Ls + tid;
   const int Lstep = top ? 32 : T;
+  pdl_enter();
   C a[32];
 #pragma unroll
   for (int c = 0; c < 32; c++) a[c] = (held && c < w) ? P.A[(size_t)(P.k0 + c) * P.ld + row] : C{0, 0};
@@ -1268,6 +1301,7 @@ __global__ void __launch_bounds__(LSW_WARPS * 32) k_laswp(C *A, size_t ld, const
                                                            int skip0, int skip1, int sol0, int sol1) {
   __shared__ int src[64], slot[32], rowof[64];
   __shared__ __align__(16) C L[32][32];   // L[c][r]
+  pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31;
   if (tid < 32) {
     const int p = lane < w ? ipiv[k0 + lane] - 1 : -1 - lane;
@@ -1320,8 +1354,8 @@ template <class C>
 static int laswp(bg_matrix *m, int k0, int w, int blk_end) {
   const int blocks = std::min((m->N + LSW_WARPS - 1) / LSW_WARPS, 148 * 8);
   prof_start(PROF_LASWP);
-  k_laswp<C><<<blocks, LSW_WARPS * 32, 0, stream()>>>((C *)m->d, m->ld, m->d_ipiv, k0, w, m->N, k0, k0 + w, k0 + w,
-                                                       blk_end);
+  BG_CUDA_TRY(pdl_launch(k_laswp<C>, dim3(blocks), LSW_WARPS * 32, 0, (C *)m->d, m->ld, m->d_ipiv, k0, w, m->N, k0,
+                         k0 + w, k0 + w, blk_end));
   BG_LAUNCHED();
   prof_stop(PROF_LASWP, 0.0);
   return BG_OK;
@@ -1342,6 +1376,7 @@ __global__ void __launch_bounds__(128) k_blk_update(int M, int nc, int K, const 
   __shared__ __align__(16) C Ls[32][32];   // Ls[k][r]
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C *Us = (C *)smem_raw;                   // Us[c * 32 + k]
+  pdl_enter();
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int r = blockIdx.x * 32 + lane, c0 = wid * NC;
 #pragma unroll
@@ -1385,7 +1420,7 @@ static int blk_update_launch(int M, int nc, int K, const C *L, const C *U, C *Cm
     attr = true;
   }
   prof_start(PROF_GEMM);
-  k_blk_update<C, NC><<<(M + 31) / 32, 128, smem, stream()>>>(M, nc, K, L, U, Cm, ld);
+  BG_CUDA_TRY(pdl_launch(k_blk_update<C, NC>, dim3((M + 31) / 32), 128, smem, M, nc, K, L, U, Cm, ld));
   BG_LAUNCHED();
   prof_stop(PROF_GEMM, 8.0 * M * (double)nc * K);
   return BG_OK;
@@ -1458,13 +1493,15 @@ static int panel_rf(bg_matrix *m, const LUWork &W, int k0, int w, int blk_end, b
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = panel_rf_smem<C, TMAX>();
   cfg.stream = stream();
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = G;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = t_pdl;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   prof_start(PROF_PANEL);
   BG_CUDA_TRY(cudaLaunchKernelEx(&cfg, k_panel_rf<C, TMAX, false>, P));
   BG_LAUNCHED();
@@ -1627,6 +1664,7 @@ int lu_factor(bg_matrix *m) {
   int *tcerr = W.info + 1;
   w += 256;
   BG_CUDA_TRY(cudaMemsetAsync(W.info, 0, 2 * sizeof(int), stream()));
+  t_pdl = true;
   if (m->precision == BG_C128) {
     I8Scratch sc{nullptr, i8_factor_bytes(N), W.info + 1};
     if (sc.bytes && cudaMallocAsync(&sc.p, sc.bytes, stream()) != cudaSuccess) {
@@ -1636,6 +1674,7 @@ int lu_factor(bg_matrix *m) {
     t_i8 = sc.p ? &sc : nullptr;
     st = getrf_rec<cdl>(m, W, 0, N);
     t_i8 = nullptr;
+    t_pdl = false;
     if (sc.p) cudaFreeAsync(sc.p, stream());
     if (st) return st;
   } else {
@@ -1646,6 +1685,7 @@ int lu_factor(bg_matrix *m) {
     t_tc = &sc;
     st = getrf_rec<cfl>(m, W, 0, N);
     t_tc = nullptr;
+    t_pdl = false;
     if (st) return st;
   }
   int info[2] = {0, 0};
@@ -1989,6 +2029,7 @@ int lu_solve_many(bg_matrix *m, void *dB, size_t ldb, int nrhs) {
     if (cudaMemsetAsync(sc.err, 0, sizeof(int), stream()) != cudaSuccess) { cudaGetLastError(); st = BG_ERR_CUDA; }
     t_i8 = &sc;
   }
+  t_pdl = true;
   for (int r0 = 0; r0 < nrhs && !st; r0 += chunk) {
     int nr = std::min(chunk, nrhs - r0);
     cdl *Bp = B + (size_t)r0 * ldb;
@@ -2001,6 +2042,7 @@ int lu_solve_many(bg_matrix *m, void *dB, size_t ldb, int nrhs) {
                                       cudaMemcpyDeviceToDevice, stream());
     if (e != cudaSuccess) { set_error("lu_solve_many: %s", cudaGetErrorString(e)); st = BG_ERR_CUDA; }
   }
+  t_pdl = false;
   t_i8 = nullptr;
   if (sc.p) {
     cudaError_t e = cudaMemcpyAsync(&tcerr, sc.err, sizeof(int), cudaMemcpyDeviceToHost, stream());
