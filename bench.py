@@ -176,7 +176,7 @@ def zgemm_peak_tflops():
 
 
 def gemm_kernel_bench(n, reps=5):
-    """Library complex GEMM (C -= A B, DMMA f64) on one n^3 problem, CUDA events
+    """Library complex GEMM (C -= A B, INT8 digit products) on one n^3 problem, CUDA events
     on the library stream, best of reps; cuBLAS ZGEMM on the same shape beside it."""
     import torch
     import buffem
@@ -200,7 +200,7 @@ def gemm_kernel_bench(n, reps=5):
     # check one column against torch (column-major: C = -(B^T A^T)^T ... use transposes)
     ref = -(B.T @ A.T).T if False else None
     cub = zgemm_peak_tflops()
-    return {"kernel": "k_zgemm_sub", "shape": [n, n, n], "tflops": ours, "ms": best * 1e3,
+    return {"kernel": "k_zgemm_i8 (+ splits)", "shape": [n, n, n], "tflops": ours, "ms": best * 1e3,
             "cublas_zgemm_tflops": cub, "frac_of_cublas": ours / cub}
 
 

@@ -2,16 +2,14 @@
 // sm_100a: replaces HMatrix::LUFactorize / LUSolve (LAPACK zgetrf / zgetrs,
 // call sites buff-scatter.cc:285,314).
 //
-// Factorisation: recursive right-looking LU over column halves.  Leaves of
-// width <= 32 are factored by one cooperative kernel (all CTAs own a slice of
-// the panel rows in shared memory; one grid barrier per column: pivot
-// candidates of every CTA -> global winner -> swap, scale, rank-1 update).
-// Row interchanges are then applied to every other column (LAPACK ipiv
-// semantics: ipiv[i] is the 1-based row swapped with row i, applied in
-// order).  Off-diagonal blocks use a unit-lower TRSM (leaf kernel + GEMM
-// recursion) and the Schur complements use a complex GEMM on the FP64 tensor
-// cores (mma.sync m8n8k4 f64; tcgen05 has no f64 kind), 4M complex product,
-// three-stage cp.async pipeline.
+// Factorisation: recursive right-looking LU over column halves down to blocks of
+// 128 columns, which are factored in panels of 32 with the panel's rows in
+// registers (one cluster, or the whole grid for tall panels).  Row interchanges
+// are applied to every other column (LAPACK ipiv semantics: ipiv[i] is the
+// 1-based row swapped with row i, applied in order).  Off-diagonal blocks use a
+// unit-lower TRSM (128-row leaf + GEMM recursion).  The Schur complements go to
+// the INT8 tensor cores (gemm_i8.cu) where they are large enough, else to the
+// FP64 tensor path (mma.sync f64), 4M complex product, cp.async pipelines.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -692,7 +690,8 @@ static int trsm(int n, int m, const C *T, size_t ldt, C *B, size_t ldb, int uppe
 }
 
 // =========================================================================
-// cooperative panel factorisation of A[k0:Nr, k0:k0+w] (w <= 32).  Each CTA
+// cooperative panel factorisation of A[k0:Nr, k0:k0+w] (w <= 32) for panels too
+// tall for the register form below (more than 37,888 rows).  Each CTA
 // holds a slice of rows_per rows in shared memory, column-major (column c at
 // S + c * rows_per): the pivot scan and the rank-1 update walk a column with
 // consecutive threads on consecutive rows, free of bank conflicts.  One grid
