@@ -26,6 +26,7 @@
 // The incident plane wave adds E0 e^{ik nhat.X} and nhat x E / Z0.
 //
 // HBM layout (per tetrahedron, built once per geometry):
+//   (all in the order of field_tables, which follows the doubles of fieldTet)
 //   fieldTet  16 doubles: V0..V3 (12), centroid (3), R_all (1), where
 //             |X - centroid| > R_all implies every face of T is far from X
 //   fieldFace 16 doubles: per local face k, (centroid, radius), radius 0 if the
@@ -39,6 +40,7 @@
 // finishing kernel (deterministic).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -187,9 +189,10 @@ __device__ __forceinline__ void rule16(const FieldK &K, const FieldPhase &F, con
 }
 
 // g_k per tetrahedron from the basis-function coefficients
-__global__ void k_fields_coef(DevGeom g, const z *J, z *coef) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= g.NT) return;
+__global__ void k_fields_coef(DevGeom g, const int *order, const z *J, z *coef) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= g.NT) return;
+  const int t = order[i];
   int4 fi = g.tetFI[t];
   int f[4] = {fi.x, fi.y, fi.z, fi.w};
 #pragma unroll
@@ -201,7 +204,7 @@ __global__ void k_fields_coef(DevGeom g, const z *J, z *coef) {
       z Ja = J[a];
       v = z{s * Ja.r, s * Ja.i};
     }
-    coef[4 * t + k] = v;
+    coef[4 * (size_t)i + k] = v;
   }
 }
 
@@ -276,19 +279,34 @@ __device__ __forceinline__ void tet_point(const FieldK &K, const double *x, cons
   if (any16) rule16<MODE>(K, F, x, T.V, a16, b16, acc);
 }
 
-// warp sum of the 12 accumulators of point p into the warp's shared slot
+// warp sum of the 12 accumulators of point p into the warp's shared slot: the
+// lanes' tree of pairs l, l ^ 16, l ^ 8, ... with each exchange halving the
+// values a lane still carries (12, 6, 3, 2, 1: 26 shuffles in place of 120,
+// beside about 300 other instructions of a far point: 11.3 -> 10.9 ms for 4,225
+// points of a plane, N = 57,222)
 __device__ __forceinline__ void warp_flush(double *acc, double (*slot)[12], int p, int lane) {
+  double v[6], u[4], w[2];
 #pragma unroll
-  for (int q = 0; q < 12; q++) {
-    double v = acc[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    acc[q] = v;
+  for (int q = 0; q < 6; q++) {
+    const bool up = lane & 16;
+    v[q] = (up ? acc[q + 6] : acc[q]) + __shfl_xor_sync(0xffffffffu, up ? acc[q] : acc[q + 6], 16);
   }
-  if (lane == 0) {
 #pragma unroll
-    for (int q = 0; q < 12; q++) slot[p][q] = acc[q];
+  for (int q = 0; q < 3; q++) {
+    const bool up = lane & 8;
+    u[q] = (up ? v[q + 3] : v[q]) + __shfl_xor_sync(0xffffffffu, up ? v[q] : v[q + 3], 8);
   }
+  u[3] = 0.0;
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const bool up = lane & 4;
+    w[q] = (up ? u[q + 2] : u[q]) + __shfl_xor_sync(0xffffffffu, up ? u[q] : u[q + 2], 4);
+  }
+  const bool up = lane & 2;
+  double r = (up ? w[1] : w[0]) + __shfl_xor_sync(0xffffffffu, up ? w[0] : w[1], 2);
+  r += __shfl_xor_sync(0xffffffffu, r, 1);
+  const int k = (lane >> 1) & 3;
+  if (!(lane & 1) && k < 3) slot[p][6 * (lane >> 4) + 3 * ((lane >> 3) & 1) + k] = r;
 }
 
 template <int MODE, bool ONE>
@@ -382,40 +400,78 @@ __global__ void k_fields_finish(const double *__restrict__ part, int nblk, int P
 static int field_tables(bg_geometry *g) {
   if (g->d_fieldTet && g->d_fieldFace) return BG_OK;
   double rmax = 0.0;      // largest distance of a vertex from its tetrahedron's centroid
-  std::vector<double> T, F;
-  T.reserve(16 * (size_t)g->NT);
-  F.reserve(16 * (size_t)g->NT);
-  for (const Object &o : g->objs) {
-    for (int t = 0; t < o.nt; t++) {
-      double ctr[3] = {0, 0, 0};
-      for (int k = 0; k < 4; k++)
-        for (int c = 0; c < 3; c++) {
-          double v = o.V[3 * o.VI[4 * t + k] + c];
-          T.push_back(v);
-          ctr[c] += 0.25 * v;
-        }
-      double Rall = 0.0;
-      for (int k = 0; k < 4; k++) {
-        const double *v = &T[T.size() - 12 + 3 * k];
-        rmax = std::fmax(rmax, std::sqrt((v[0] - ctr[0]) * (v[0] - ctr[0]) + (v[1] - ctr[1]) * (v[1] - ctr[1]) +
-                                         (v[2] - ctr[2]) * (v[2] - ctr[2])));
-      }
-      for (int k = 0; k < 4; k++) {
-        int f = o.FI[4 * t + k];
-        if (f >= 0 && f < o.nif) {
-          const Face &Fc = o.F[f];
-          double d = std::sqrt((Fc.cen[0] - ctr[0]) * (Fc.cen[0] - ctr[0]) + (Fc.cen[1] - ctr[1]) * (Fc.cen[1] - ctr[1]) +
-                               (Fc.cen[2] - ctr[2]) * (Fc.cen[2] - ctr[2]));
-          Rall = std::fmax(Rall, 10.0 * Fc.radius + d);
-          F.insert(F.end(), {Fc.cen[0], Fc.cen[1], Fc.cen[2], Fc.radius});
-        } else {
-          F.insert(F.end(), {0.0, 0.0, 0.0, 0.0});
-        }
-      }
-      // margin so that rounding never calls a face far that the per-face test would not
-      Rall = Rall * (1.0 + 1e-12) + 1e-300;
-      T.insert(T.end(), {ctr[0], ctr[1], ctr[2], Rall});
+  // Order of the tetrahedra: by place (bits of the centroid's grid coordinates
+  // interleaved), so that the 32 of a warp are neighbours in space and take the
+  // same rule for most points.  In mesh order (rows of cells) 24.6 of 32 lanes
+  // were active on average, now 26.4: 10.9 -> 9.8 ms for 4,225 points of a plane,
+  // N = 57,222.
+  double lo[3] = {HUGE_VAL, HUGE_VAL, HUGE_VAL}, hi[3] = {-HUGE_VAL, -HUGE_VAL, -HUGE_VAL};
+  for (const Object &o : g->objs)
+    for (size_t i = 0; i < o.V.size(); i++) {
+      lo[i % 3] = std::fmin(lo[i % 3], o.V[i]);
+      hi[i % 3] = std::fmax(hi[i % 3], o.V[i]);
     }
+  const double ext = std::fmax(std::fmax(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
+  const double cells = ext > 0 ? 1023.0 / ext : 0.0;
+  auto spread = [](uint64_t x) {      // 10 bits to every third place
+    x = (x | x << 16) & 0x030000ff;
+    x = (x | x << 8) & 0x0300f00f;
+    x = (x | x << 4) & 0x030c30c3;
+    return (x | x << 2) & 0x09249249;
+  };
+  std::vector<uint64_t> order;
+  order.reserve(g->NT);
+  std::vector<std::pair<const Object *, int>> where;
+  where.reserve(g->NT);
+  for (const Object &o : g->objs)
+    for (int t = 0; t < o.nt; t++) {
+      uint64_t key = 0;
+      for (int c = 0; c < 3; c++) {
+        double v = 0;
+        for (int k = 0; k < 4; k++) v += 0.25 * o.V[3 * o.VI[4 * t + k] + c];
+        key |= spread((uint64_t)std::fmin(1023.0, std::fmax(0.0, (v - lo[c]) * cells))) << c;
+      }
+      order.push_back(key << 32 | (uint64_t)where.size());
+      where.push_back({&o, t});
+    }
+  std::sort(order.begin(), order.end());
+  std::vector<double> T(16 * (size_t)g->NT + ((size_t)g->NT + 1) / 2), F(16 * (size_t)g->NT);
+  int *idx = (int *)(T.data() + 16 * (size_t)g->NT);      // the order, behind the tables
+  for (int i = 0; i < g->NT; i++) {
+    idx[i] = (int)(uint32_t)order[i];
+    const Object &o = *where[idx[i]].first;
+    const int t = where[idx[i]].second;
+    double *Ti = &T[16 * (size_t)i], *Fi = &F[16 * (size_t)i];
+    double ctr[3] = {0, 0, 0};
+    for (int k = 0; k < 4; k++)
+      for (int c = 0; c < 3; c++) {
+        double v = o.V[3 * o.VI[4 * t + k] + c];
+        Ti[3 * k + c] = v;
+        ctr[c] += 0.25 * v;
+      }
+    double Rall = 0.0;
+    for (int k = 0; k < 4; k++) {
+      const double *v = Ti + 3 * k;
+      rmax = std::fmax(rmax, std::sqrt((v[0] - ctr[0]) * (v[0] - ctr[0]) + (v[1] - ctr[1]) * (v[1] - ctr[1]) +
+                                       (v[2] - ctr[2]) * (v[2] - ctr[2])));
+    }
+    for (int k = 0; k < 4; k++) {
+      int f = o.FI[4 * t + k];
+      if (f >= 0 && f < o.nif) {
+        const Face &Fc = o.F[f];
+        double d = std::sqrt((Fc.cen[0] - ctr[0]) * (Fc.cen[0] - ctr[0]) + (Fc.cen[1] - ctr[1]) * (Fc.cen[1] - ctr[1]) +
+                             (Fc.cen[2] - ctr[2]) * (Fc.cen[2] - ctr[2]));
+        Rall = std::fmax(Rall, 10.0 * Fc.radius + d);
+        Fi[4 * k] = Fc.cen[0];
+        Fi[4 * k + 1] = Fc.cen[1];
+        Fi[4 * k + 2] = Fc.cen[2];
+        Fi[4 * k + 3] = Fc.radius;
+      }
+    }
+    // margin so that rounding never calls a face far that the per-face test would not
+    Rall = Rall * (1.0 + 1e-12) + 1e-300;
+    for (int c = 0; c < 3; c++) Ti[12 + c] = ctr[c];
+    Ti[15] = Rall;
   }
   double *dT = nullptr, *dF = nullptr;
   cudaError_t e = cudaMalloc(&dT, sizeof(double) * T.size());
@@ -475,7 +531,8 @@ int get_fields(bg_geometry *g, double wr, double wi, const void *dJ, const doubl
       set_error("GetFields scratch: %s", cudaGetErrorString(e));
       return BG_ERR_CUDA;
     }
-    k_fields_coef<<<(NT + 255) / 256, 256, 0, stream()>>>(g->dev, (const z *)dJ, coef);
+    k_fields_coef<<<(NT + 255) / 256, 256, 0, stream()>>>(
+        g->dev, (const int *)(g->d_fieldTet + 16 * (size_t)NT), (const z *)dJ, coef);
     BG_LAUNCHED();
     dim3 grid(ny, nbx);
     // the largest |k| |y - centroid| of any quadrature point (see field_point)
