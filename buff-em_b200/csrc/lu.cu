@@ -667,14 +667,15 @@ template <class C>
 static int trsm(int n, int m, const C *T, size_t ldt, C *B, size_t ldb, int upper) {
   if (n <= 0 || m <= 0) return BG_OK;
   if (n <= TRS_MAX) {
-    const int blocks4 = (m + 4 * TRS_WARPS - 1) / (4 * TRS_WARPS);   // with four columns a warp
+    const int cap = 148 * (sizeof(C) == 16 ? 1 : 2);      // CTAs the shared memory lets run at once
+    const int cpw = m <= cap * TRS_WARPS ? 1 : m <= 2 * cap * TRS_WARPS ? 2 : 4;
     if (upper)
-      return blocks4 >= 148   ? trsm_launch<C, 4, true>(n, m, T, ldt, B, ldb)
-             : blocks4 >= 74  ? trsm_launch<C, 2, true>(n, m, T, ldt, B, ldb)
-                              : trsm_launch<C, 1, true>(n, m, T, ldt, B, ldb);
-    return blocks4 >= 148   ? trsm_launch<C, 4, false>(n, m, T, ldt, B, ldb)
-           : blocks4 >= 74  ? trsm_launch<C, 2, false>(n, m, T, ldt, B, ldb)
-                            : trsm_launch<C, 1, false>(n, m, T, ldt, B, ldb);
+      return cpw == 4   ? trsm_launch<C, 4, true>(n, m, T, ldt, B, ldb)
+             : cpw == 2 ? trsm_launch<C, 2, true>(n, m, T, ldt, B, ldb)
+                        : trsm_launch<C, 1, true>(n, m, T, ldt, B, ldb);
+    return cpw == 4   ? trsm_launch<C, 4, false>(n, m, T, ldt, B, ldb)
+           : cpw == 2 ? trsm_launch<C, 2, false>(n, m, T, ldt, B, ldb)
+                      : trsm_launch<C, 1, false>(n, m, T, ldt, B, ldb);
   }
   int n1 = (n / 2 + TRS_MAX - 1) / TRS_MAX * TRS_MAX;   // multiples of the leaf (n > TRS_MAX, so n1 < n)
   int n2 = n - n1;
