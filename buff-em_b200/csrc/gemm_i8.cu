@@ -12,30 +12,32 @@
 // summed exactly in 32-bit integers, all products with i + j = d in one
 // accumulator, d = 2 .. 9; products with i + j > 9 are below 2^-60 of the
 // largest product of the row and the column and are left out.  The eight sums
-// are added in FP64 from the smallest up and subtracted from C once, so C is
-// rounded about once per call, where a chain of K fused multiply-adds rounds K
+// are added in FP64 from the smallest up, in two halves, so C is rounded twice per
+// call and 2,048 columns of K, where a chain of fused multiply-adds rounds it K
 // times.
 //
 // Real embedding: A as M x 2K (re, im interleaved along K), B as 2K x 2N with
 // columns (br, -bi) and (bi, br), so that columns 2n, 2n + 1 of the product are
 // the two parts of column n.
 //
-// Kernel: persistent, tiles of 128 rows x 64 real columns, eight accumulators =
-// all 512 TMEM columns; four stages of 32 bytes of K of all 16 slices (48 KB
-// each, two contiguous copies); warp 0 loads, warp 1 issues the 36 MMAs of a
-// stage, warps 2-17 hold their part of C in registers since before the
-// accumulators are ready and combine.  Every wait is bounded; on a timeout the
-// error word is set, copies in flight are waited for and TMEM is freed.
+// Kernel: persistent, tiles of 128 rows x 128 real columns in two passes over K:
+// first the digit products with d = 6 .. 9, then (half of the digits) d = 2 .. 5,
+// four accumulators of 128 columns = all 512 TMEM columns each time.  Stages of
+// 32 bytes of K of all 16 slices (64 KB, two contiguous copies; half of it in the
+// second pass), three deep; warp 0 loads, warp 1 issues the 26 or 10 MMAs of a
+// stage, warps 2-17 combine and update C.  Every wait is bounded; on a timeout
+// the error word is set, copies in flight are waited for and TMEM is freed.
 //
-// What bounds it: shared memory, 6 KB of operands read per 128 x 64 x 32 MMA and
-// 48 KB written per 36 of them, 57 cycles an MMA at 128 bytes where the
-// arithmetic takes 32 (a 64-column MMA alone runs at 3.04 of 4.56 POP/s), and
-// the combination, which no second set of accumulators can hide (about 4 us a
-// tile).  A CTA pair (256 rows, half of B in each) was slower: 14.9 ms where
-// this takes 12.9.  9936 x 9936 x 1024: FP64 tiles 24.9 ms (32.5 TFLOP/s) -> 12.9
-// ms (62.6); 4096 x 4096 x 128: 0.64 -> 0.37 ms.  Factorisation of N = 19,872:
-// products 660 -> 367 ms.  Error of 256 x 256 x 512 products against 80-bit
-// sums: rms 1.7e-16 of the largest entry with FP64 tiles, 2.2e-17 here.
+// What bounds it: shared memory, 8 KB of operands read per 128 x 128 x 32 MMA and
+// 96 KB written per 36 of them, 85 cycles an MMA at 128 bytes where the arithmetic
+// takes 64, and the combinations, which no second set of accumulators can hide
+// (8.9 us a tile).  All eight sums of a 64-column tile at once took less of C's
+// traffic but 57 cycles per half as large an MMA (a 64-column MMA alone runs at
+// 3.04 of 4.56 POP/s): 12.9 ms for 9936 x 9936 x 1024; a CTA pair (256 rows, half
+// of B in each) 14.9.  Now 11.0 (73 TFLOP/s), FP64 tiles 24.9 (32.5); 1024^3:
+// 0.304 -> 0.163 ms.  Factorisation of N = 19,872: products 660 -> 315 ms.  Error
+// of 1024 x 1024 x 2048 products against 80-bit sums: rms 2.1e-17 of the largest
+// entry (FP64 tiles 3.7e-16 at 512 x 512 x 2048).
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -52,9 +54,9 @@ struct z2i { double r, i; };
 
 #define I8_S 8                    // digits per number
 #define I8_BM 128                 // rows of a tile
-#define I8_BN 64                  // real columns of a tile (32 complex)
+#define I8_BN 128                 // real columns of a tile (64 complex)
 #define I8_BK 32                  // bytes of K per stage: one MMA deep, one 32-byte swizzle row
-#define I8_STAGES 4
+#define I8_STAGES 3
 #define I8_GROUP 16               // row blocks per raster group
 #define I8_THREADS 576
 #define I8_A_BYTES (I8_S * I8_BM * I8_BK)
@@ -127,13 +129,13 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
       for (int t = blockIdx.x; t < ntiles && !s_fail; t += gridDim.x) {
         int tm, tn;
         i8_tile(P, t, tm, tn);
-        for (int kb = 0; kb < nk; kb++, kc++) {
-          const int s = kc % I8_STAGES;
+        for (int it = 0; it < 2 * nk; it++, kc++) {
+          const int s = kc % I8_STAGES, kb = it < nk ? it : it - nk, half = it < nk ? 1 : 2;   // pass 1: digits 0 .. 3
           if (kc >= I8_STAGES && !mbar_wait(&empty[s], ((kc / I8_STAGES) - 1) & 1)) { s_fail = 1; break; }
           unsigned char *sa = ring + s * I8_STAGE;
-          mbar_expect_tx(&full[s], I8_STAGE);
-          bulk_load(sa, P.A + ((size_t)tm * nk + kb) * I8_A_BYTES, I8_A_BYTES, &full[s]);
-          bulk_load(sa + I8_A_BYTES, P.B + ((size_t)tn * nk + kb) * I8_B_BYTES, I8_B_BYTES, &full[s]);
+          mbar_expect_tx(&full[s], I8_STAGE / half);
+          bulk_load(sa, P.A + ((size_t)tm * nk + kb) * I8_A_BYTES, I8_A_BYTES / half, &full[s]);
+          bulk_load(sa + I8_A_BYTES, P.B + ((size_t)tn * nk + kb) * I8_B_BYTES, I8_B_BYTES / half, &full[s]);
           s_issued = kc + 1;
         }
       }
@@ -144,84 +146,94 @@ __global__ void __launch_bounds__(I8_THREADS, 1)
       // 8-bit (1 at bits 7-9 and 10-12), both K-major, N>>3 at 17-22, M>>4 at 24-28
       const uint32_t idesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(I8_BN >> 3) << 17) |
                              ((uint32_t)(I8_BM >> 4) << 24);
-      int kc = 0, i = 0;
-      for (int t = blockIdx.x; t < ntiles && !s_fail; t += gridDim.x, i++) {
-        if (i >= 1 && !mbar_wait(acc_empty, (i - 1) & 1)) { s_fail = 4; break; }
-        asm volatile("tcgen05.fence::after_thread_sync;");
-        for (int kb = 0; kb < nk; kb++, kc++) {
-          const int s = kc % I8_STAGES;
-          if (!mbar_wait(&full[s], (kc / I8_STAGES) & 1)) { s_fail = 2; break; }
+      auto mma = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t acc) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d), "l"(da), "l"(db), "r"(idesc), "r"(acc));
+      };
+      int kc = 0, i = 0;      // i: passes of this CTA so far
+      for (int t = blockIdx.x; t < ntiles && !s_fail; t += gridDim.x) {
+#pragma unroll
+        for (int pass = 0; pass < 2; pass++, i++) {
+          if (s_fail) break;
+          if (i >= 1 && !mbar_wait(acc_empty, (i - 1) & 1)) { s_fail = 4; break; }
           asm volatile("tcgen05.fence::after_thread_sync;");
-          const uint32_t sa = smem_u32(ring + s * I8_STAGE), sb = sa + I8_A_BYTES;
-          const uint64_t da0 = sw32_desc(sa), db0 = sw32_desc(sb);
+          for (int kb = 0; kb < nk; kb++, kc++) {
+            const int s = kc % I8_STAGES;
+            if (!mbar_wait(&full[s], (kc / I8_STAGES) & 1)) { s_fail = 2; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint32_t sa = smem_u32(ring + s * I8_STAGE);
+            const uint64_t da0 = sw32_desc(sa), db0 = sw32_desc(sa + I8_A_BYTES);
+            // pass 0: a + b = 4 .. 7, pass 1: a + b = 0 .. 3, each group first met at a = 0
 #pragma unroll
-          for (int a = 0; a < I8_S; a++) {
+            for (int a = 0; a < (pass ? 4 : I8_S); a++)
 #pragma unroll
-            for (int b = 0; b < I8_S - a; b++) {
-              const uint64_t da = da0 + ((a * I8_BM * I8_BK) >> 4);
-              const uint64_t db = db0 + ((b * I8_BN * I8_BK) >> 4);
-              const uint32_t acc = (kb > 0 || a > 0) ? 1u : 0u;   // group a + b is first met at a = 0
-              asm volatile(
-                  "{\n\t.reg .pred p;\n\t"
-                  "setp.ne.b32 p, %4, 0;\n\t"
-                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-                  ::"r"(tmem + (uint32_t)((a + b) * I8_BN)), "l"(da), "l"(db), "r"(idesc), "r"(acc));
-            }
+              for (int b = 0; b < I8_S; b++) {
+                const int g = a + b - (pass ? 0 : 4);
+                if (g < 0 || g > 3) continue;
+                mma(tmem + (uint32_t)(g * I8_BN), da0 + ((a * I8_BM * I8_BK) >> 4), db0 + ((b * I8_BN * I8_BK) >> 4),
+                    (kb > 0 || a > 0) ? 1u : 0u);
+              }
+            mma_commit(&empty[s]);
+            s_consumed = kc + 1;
           }
-          mma_commit(&empty[s]);
-          s_consumed = kc + 1;
+          if (s_fail) break;
+          mma_commit(acc_full);
         }
-        if (s_fail) break;
-        mma_commit(acc_full);
       }
       // no MMA may still run when the TMEM is freed, whichever way the loop ended
       mma_commit(mma_done);
       if (!mbar_wait(mma_done, 0) && !s_fail) s_fail = 5;
     }
   } else {
-    // warps 2 .. 17: TMEM lanes 32 (warp % 4) .. + 31, 8 complex columns each
+    // warps 2 .. 17: TMEM lanes 32 (warp % 4) .. + 31, 16 complex columns each
     const int q = warp & 3, h = (warp - 2) >> 2;
     int i = 0;
-    for (int t = blockIdx.x; t < ntiles && !s_fail; t += gridDim.x, i++) {
+    for (int t = blockIdx.x; t < ntiles && !s_fail; t += gridDim.x) {
       int tm, tn;
       i8_tile(P, t, tm, tn);
-      const int row = tm * I8_BM + q * 32 + lane, col0 = tn * (I8_BN / 2) + 8 * h;
+      const int row = tm * I8_BM + q * 32 + lane, col0 = tn * (I8_BN / 2) + 16 * h;
       z2i *pc = P.C + (size_t)col0 * P.ldc + row;
-      z2i cv[8];
-      const double sa = row < P.M ? P.sa[row] : 0.0;
+      double sa = row < P.M ? P.sa[row] * 0x1p-32 : 0.0;      // the second pass's groups weigh 2^32 more
+#pragma unroll 1
+      for (int pass = 0; pass < 2; pass++, i++) {
+        // eight columns of C ahead: the first before the accumulators are ready
+        z2i cv[8];
 #pragma unroll
-      for (int j = 0; j < 8; j++)
-        cv[j] = row < P.M && col0 + j < P.N ? pc[(size_t)j * P.ldc] : z2i{0.0, 0.0};
-      if (!mbar_wait(acc_full, i & 1)) { s_fail = 3; break; }
-      asm volatile("tcgen05.fence::after_thread_sync;");
+        for (int j = 0; j < 8; j++)
+          cv[j] = row < P.M && col0 + j < P.N ? pc[(size_t)j * P.ldc] : z2i{0.0, 0.0};
+        if (!mbar_wait(acc_full, i & 1)) { s_fail = 3; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
-      for (int c = 0; c < 8; c += 2) {      // two complex = four real columns at a time
-        uint32_t r[8][4];
-        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(16 * h + 2 * c);
+        for (int c = 0; c < 16; c += 2) {      // two complex = four real columns at a time
+          uint32_t r[4][4];
+          const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(32 * h + 2 * c);
 #pragma unroll
-        for (int g = 0; g < I8_S; g++)
-          asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                       : "=r"(r[g][0]), "=r"(r[g][1]), "=r"(r[g][2]), "=r"(r[g][3])
-                       : "r"(taddr + (uint32_t)(g * I8_BN)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;");
-        double v[4];
+          for (int g = 0; g < 4; g++)
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                         : "=r"(r[g][0]), "=r"(r[g][1]), "=r"(r[g][2]), "=r"(r[g][3])
+                         : "r"(taddr + (uint32_t)(g * I8_BN)));
+          asm volatile("tcgen05.wait::ld.sync.aligned;");
+          double v[4];
 #pragma unroll
-        for (int x = 0; x < 4; x++) {
-          double y = pair_to_double((int)r[6][x], (int)r[7][x]);
-          y = fma(y, 0x1p-16, pair_to_double((int)r[4][x], (int)r[5][x]));
-          y = fma(y, 0x1p-16, pair_to_double((int)r[2][x], (int)r[3][x]));
-          v[x] = fma(y, 0x1p-16, pair_to_double((int)r[0][x], (int)r[1][x])) * sa;
+          for (int x = 0; x < 4; x++)
+            v[x] = fma(pair_to_double((int)r[2][x], (int)r[3][x]), 0x1p-16, pair_to_double((int)r[0][x], (int)r[1][x])) * sa;
+#pragma unroll
+          for (int j = 0; j < 2; j++)
+            if (row < P.M && col0 + c + j < P.N) {
+              const double sb = P.sb[col0 + c + j];
+              z2i &x = cv[(c + j) & 7];
+              pc[(size_t)(c + j) * P.ldc] = z2i{fma(-v[2 * j], sb, x.r), fma(-v[2 * j + 1], sb, x.i)};
+              if (c < 8 && col0 + c + j + 8 < P.N) x = pc[(size_t)(c + j + 8) * P.ldc];
+            }
         }
-#pragma unroll
-        for (int j = 0; j < 2; j++)
-          if (row < P.M && col0 + c + j < P.N) {
-            const double sb = P.sb[col0 + c + j];
-            pc[(size_t)(c + j) * P.ldc] = z2i{fma(-v[2 * j], sb, cv[c + j].r), fma(-v[2 * j + 1], sb, cv[c + j].i)};
-          }
+        sa *= 0x1p+32;
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty);
       }
-      asm volatile("tcgen05.fence::before_thread_sync;");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(acc_empty);
     }
   }
   __syncthreads();
@@ -292,7 +304,7 @@ __global__ void __launch_bounds__(128) k_i8_rowmax(int M, int K, const z2i *A, s
 }
 
 // Digit blocks: 32 bytes of K (16 columns, re and im interleaved) of 128 rows of
-// A or 64 rows of B, [digit][row][32 bytes], one contiguous piece per block in the
+// A or 128 rows of B, [digit][row][32 bytes], one contiguous piece per block in the
 // order the stages read them, the two 16-byte halves of a row exchanged where
 // bit 2 of the row is set (the tensor core's 32-byte swizzle).  Loads are then
 // whole lines; as planes of rows, a stage read half a line per row.
@@ -332,8 +344,8 @@ __global__ void __launch_bounds__(128) k_i8_slice_a(int M, int K, const z2i *A, 
 }
 
 // slices of B, K <= I8_KC: a block takes a column; rows 2n: (br, -bi), 2n + 1: (bi, br)
-#define I8_KC 1024
-__global__ void __launch_bounds__(128) k_i8_slice_b(int K, const z2i *B, size_t ldb, int8_t *S, int nk, double *sb) {
+#define I8_KC 2048
+__global__ void __launch_bounds__(I8_KC / 8) k_i8_slice_b(int K, const z2i *B, size_t ldb, int8_t *S, int nk, double *sb) {
   const int n = blockIdx.x, t = threadIdx.x;
   const z2i *b = B + (size_t)n * ldb;
   z2i v[4][2];
@@ -342,20 +354,21 @@ __global__ void __launch_bounds__(128) k_i8_slice_b(int K, const z2i *B, size_t 
   for (int i = 0; i < 4; i++)
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int k = 2 * t + 256 * i + h;
+      const int k = 2 * t + I8_KC / 4 * i + h;
       v[i][h] = k < K ? b[k] : z2i{0.0, 0.0};
       x = max(x, max(abs_bits(v[i][h].r), abs_bits(v[i][h].i)));
     }
-  __shared__ unsigned long long red[4];
+  __shared__ unsigned long long red[I8_KC / 256];
   for (int o = 16; o > 0; o >>= 1) x = max(x, __shfl_xor_sync(0xffffffffu, x, o));
   if ((t & 31) == 0) red[t >> 5] = x;
   __syncthreads();
-  x = max(max(red[0], red[1]), max(red[2], red[3]));
+#pragma unroll
+  for (int i = 0; i < I8_KC / 256; i++) x = max(x, red[i]);
   const DigitScale sc = split_scale(x);
   if (t == 0) sb[n] = digit_scale(x);
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    const int k = 2 * t + 256 * i;
+    const int k = 2 * t + I8_KC / 4 * i;
     if (k / 16 >= nk) continue;
     long long r[2], m[2];
 #pragma unroll
@@ -379,7 +392,7 @@ __global__ void __launch_bounds__(128) k_i8_slice_b(int K, const z2i *B, size_t 
 }
 
 // ------------------------------------------------------------------ host side
-#define I8_MC 8192                // rows of A and complex columns of B sliced at a time at most
+#define I8_MC 4096                // rows of A and complex columns of B sliced at a time at most
 #define I8_NC 4096
 
 static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -418,7 +431,7 @@ int zgemm_i8(int M, int N, int K, const void *Av, size_t lda, const void *Bv, si
     const int kk = std::min(kc, K - k0), nk = (kk + 15) / 16;
     for (int n0 = 0; n0 < N; n0 += nc) {
       const int nn = std::min(nc, N - n0);
-      k_i8_slice_b<<<nn, 128, 0, stream()>>>(kk, B + k0 + (size_t)n0 * ldb, ldb, Sb, nk, sb);
+      k_i8_slice_b<<<nn, I8_KC / 8, 0, stream()>>>(kk, B + k0 + (size_t)n0 * ldb, ldb, Sb, nk, sb);
       BG_LAUNCHED();
       for (int m0 = 0; m0 < M; m0 += mc) {
         const int mm = std::min(mc, M - m0);

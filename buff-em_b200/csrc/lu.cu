@@ -403,17 +403,17 @@ struct I8Scratch {
   int *err;
 };
 static thread_local I8Scratch *t_i8 = nullptr;
-// Which products go there, from measured times in us: 128 x 32 tiles in waves of
-// 148 at 0.078 us per column of K and 1.5 us of epilogue, 25 us of launches,
-// splitting at 64 bytes per element of A and B and 3 TB/s; the FP64 tiles at 28
-// TFLOP/s.  Measured INT8 / FP64: 2048 x 1024 x 128 90 / 90 us, 4096 x 4096 x
-// 128 370 / 640, 1024^3 196 / 304, 9936 x 9936 x 1024 13.2 / 24.9 ms; 3968 x 128
-// x 128 50 / 27.
+// Which products go there, from measured times in us: 128 x 64 tiles in waves of
+// 148 at 0.117 us per column of K and 8.9 us for the two combinations, 15 us of
+// launches, splitting at 64 bytes per element of A and B and 5 TB/s; the FP64
+// tiles at 28 TFLOP/s.  Measured INT8 / FP64: 2048 x 512 x 512 95 /
+// 141 us, 1350 x 672 x 672 117 / 203, 4096 x 4096 x 128 380 / 640, 1024^3 163 /
+// 304, 9936 x 9936 x 1024 11.0 / 24.9 ms; 2048 x 1024 x 128 78 / 90 us.
 static bool i8_takes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return false;
-  const double tiles = std::ceil((double)M / 128) * std::ceil((double)N / 32);
-  const double split = 25.0 + ((double)M + N) * K * (64 / 3e6);
-  const double i8 = std::ceil(tiles / 148) * (0.078 * K + 1.5) + split, fp64 = 8.0 * M * (double)N * K / 28e6;
+  const double tiles = std::ceil((double)M / 128) * std::ceil((double)N / 64);
+  const double split = 15.0 + ((double)M + N) * K * (64 / 5e6);
+  const double i8 = std::ceil(tiles / 148) * (0.117 * K + 8.9) + split, fp64 = 8.0 * M * (double)N * K / 28e6;
   return i8 < 0.95 * fp64;
 }
 

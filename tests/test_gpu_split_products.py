@@ -1,8 +1,8 @@
 """Products on the INT8 tensor cores against FP64 ones (needs a B200: -m gpu).
 
 C - A B through the public GEMM entry at sizes that take the split path: edges
-of its 128 x 32 tiles, of the 32-number K steps, of the 1,024-column K chunks
-and of the 8,192-row and 4,096-column chunks.  Tolerances, per entry:
+of its 128 x 64 tiles, of the 16-column K blocks, of the 2,048-column K chunks
+and of the 4,096-row and 4,096-column chunks.  Tolerances, per entry:
   * the FP64 reference is off by at most (K + 2) sqrt(2) 2^-52 (|A| |B|);
   * the split result by one rounding of C, 2^-53 of |C| and of the result, and
     the digit products it leaves out: 2 K terms of at most 9 x 2^14 x 2^-76 of
@@ -41,7 +41,7 @@ def check(A, B, C, out):
     assert bool(((out - ref).abs() <= bound).all())
 
 
-@pytest.mark.parametrize("M,N,K", [(1024, 1024, 512), (1025, 1057, 521), (1151, 1000, 1100), (8200, 600, 240),
+@pytest.mark.parametrize("M,N,K", [(1024, 1024, 512), (1025, 1057, 521), (1151, 1000, 2100), (8200, 600, 240),
                                    (1000, 4130, 330), (4000, 900, 129)])
 def test_split_product_matches_fp64(M, N, K):
     A, B, C = draw((K, M), 1), draw((N, K), 2), draw((N, M), 3)
