@@ -34,8 +34,8 @@
 // (8.9 us a tile).  All eight sums of a 64-column tile at once took less of C's
 // traffic but 57 cycles per half as large an MMA (a 64-column MMA alone runs at
 // 3.04 of 4.56 POP/s): 12.9 ms for 9936 x 9936 x 1024; a CTA pair (256 rows, half
-// of B in each) 14.9.  Now 11.0 (73 TFLOP/s), FP64 tiles 24.9 (32.5); 1024^3:
-// 0.304 -> 0.163 ms.  Factorisation of N = 19,872: products 660 -> 315 ms.  Error
+// of B in each) 14.9.  Now 11.0 (73 TFLOP/s; 84 at 4096^3), FP64 tiles 24.9 (32.5);
+// 1024^3: 0.304 -> 0.163 ms.  Factorisation of N = 19,872: products 660 -> 315 ms.  Error
 // of 1024 x 1024 x 2048 products against 80-bit sums: rms 2.1e-17 of the largest
 // entry (FP64 tiles 3.7e-16 at 512 x 512 x 2048).
 #include <cuda.h>
