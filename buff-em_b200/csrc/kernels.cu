@@ -1315,6 +1315,47 @@ __global__ void __launch_bounds__(128) k_pft_ext(PftArgs P, PWave pw, double *pa
   }
 }
 
+// The overlap power of point i of tetrahedron t where eps may jump between two
+// points (Janus, expressions): a basis function's rule starts at its own vertex
+// Q, and the points are rounded as QA + (u . L); a point that lies on the jump
+// takes the side this rounding gives it, for each of the four faces by itself.
+__device__ __noinline__ double opft_point_by_face(const DevGeom &g, const cd *J, int t, int i, int obj, cd pre) {
+  const int4 vi = g.tetVI[t], fi = g.tetFI[t];
+  const int v[4] = {vi.x, vi.y, vi.z, vi.w}, fl[4] = {fi.x, fi.y, fi.z, fi.w};
+  const double *u = c_tcr33 + 4 * i;
+  const double vol = g.tetVol[t], wt = 6.0 * vol * u[3];
+  double V[4][3], contrib = 0.0;
+  for (int q = 0; q < 4; q++) load3(g.V4, v[q], V[q]);
+  for (int q = 0; q < 4; q++) {
+    const int a = fl[q];
+    if (a < 0) continue;
+    double QA[3], L[3][3], bA[3], x[3];
+    load3(g.V4, v[q], QA);
+    for (int m = 0; m < 3; m++) {
+      double tmp[3];
+      load3(g.V4, v[(q + 1 + m) % 4], tmp);
+      for (int c = 0; c < 3; c++) L[m][c] = tmp[c] - QA[c];
+    }
+    for (int c = 0; c < 3; c++) {
+      bA[c] = u[0] * L[0][c] + u[1] * L[1][c] + u[2] * L[2][c];
+      x[c] = bA[c] + QA[c];
+    }
+    cd j[3], E[3][3], Ei[3][3], s = cmk(0, 0);
+    tet_current(g, J, t, V, x, j);
+    mat_eval(g.mats[obj], g.expr ? g.expr + obj : nullptr, x, E);
+    E[0][0].r -= 1.0; E[1][1].r -= 1.0; E[2][2].r -= 1.0;
+    inv3(E, Ei);
+    const double pa = (g.bfTet[a].x == t ? 1.0 : -1.0) * g.bfArea[a] / (3.0 * vol);
+    for (int mu = 0; mu < 3; mu++) {
+      const cd r = cadd(cadd(cmul(Ei[mu][0], j[0]), cmul(Ei[mu][1], j[1])), cmul(Ei[mu][2], j[2]));
+      s = cadd(s, cscale(r, pa * bA[mu]));
+    }
+    const cd Ja = J[a];
+    contrib += cmul(cmul(cscale(pre, 0.5 * wt), cmk(Ja.r, -Ja.i)), s).r;
+  }
+  return contrib;
+}
+
 // OPFT absorbed power (OPFT.cc:62-119, OverlapIntegrand_PFT PAbs term,
 // OverlapIntegrals.cc:79-170,242-298): sum Re(conj(Ja) Jb ME_ab),
 // ME_ab = 1/2 int b_a . (i Z0/w)(eps-1)^-1 . b_b on the shared tetrahedron.
@@ -1330,21 +1371,27 @@ __global__ void __launch_bounds__(128) k_opft(PftArgs P, cd omega, double *part,
   int obj = 0;
   if (t < g.NT) {
     obj = g.tetObj[t];
-    double V[4][3], x[3], wt;
-    tet_point33(g, t, id - 33 * t, V, x, wt);
-    cd j[3];
-    tet_current(g, P.J, t, V, x, j);
-    const cd pre = cscale(cdiv(cmk(0, 376.73031346177), omega), 0.5 * wt);
-    cd E[3][3], Ei[3][3], s = cmk(0, 0);
-    mat_eval(g.mats[obj], g.expr ? g.expr + obj : nullptr, x, E);
-    E[0][0].r -= 1.0; E[1][1].r -= 1.0; E[2][2].r -= 1.0;
-    inv3(E, Ei);
+    const cd pre0 = cdiv(cmk(0, 376.73031346177), omega);
+    const int kind = g.mats[obj].kind;
+    if (kind != BG_MAT_CONST_ISO && kind != BG_MAT_CONST_TENSOR && kind != BG_MAT_GAUSSIAN) {
+      contrib = opft_point_by_face(g, P.J, t, id - 33 * t, obj, pre0);
+    } else {
+      double V[4][3], x[3], wt;
+      tet_point33(g, t, id - 33 * t, V, x, wt);
+      cd j[3];
+      tet_current(g, P.J, t, V, x, j);
+      const cd pre = cscale(pre0, 0.5 * wt);
+      cd E[3][3], Ei[3][3], s = cmk(0, 0);
+      mat_eval(g.mats[obj], g.expr ? g.expr + obj : nullptr, x, E);
+      E[0][0].r -= 1.0; E[1][1].r -= 1.0; E[2][2].r -= 1.0;
+      inv3(E, Ei);
 #pragma unroll
-    for (int mu = 0; mu < 3; mu++) {
-      const cd r = cadd(cadd(cmul(Ei[mu][0], j[0]), cmul(Ei[mu][1], j[1])), cmul(Ei[mu][2], j[2]));
-      s = cadd(s, cmul(cmk(j[mu].r, -j[mu].i), r));
+      for (int mu = 0; mu < 3; mu++) {
+        const cd r = cadd(cadd(cmul(Ei[mu][0], j[0]), cmul(Ei[mu][1], j[1])), cmul(Ei[mu][2], j[2]));
+        s = cadd(s, cmul(cmk(j[mu].r, -j[mu].i), r));
+      }
+      contrib = cmul(pre, s).r;
     }
-    contrib = cmul(pre, s).r;
   }
   __shared__ double red[4][PMAXOBJ];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;

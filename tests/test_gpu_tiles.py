@@ -120,3 +120,17 @@ def test_pair_table_grows(tmp_path, oracle_lib):
     assert Gb.TotalBFs == n
     ok, worst = entry_close(Gb.AssembleVIEMatrix(0.8).download(), Go.assemble(0.8 + 0j))
     assert ok, worst
+
+
+@pytest.mark.parametrize("n,z", [(2, 0.11), (3, 0.0637), (4, -0.21)])
+def test_overlap_power_of_a_jump(sphere, oracle_lib, n, z):
+    """eps that jumps across a plane through the cells: the overlap power takes
+    every face's points by itself (no point of these meshes lies on the plane)."""
+    kw = dict(eps=4 + 0.2j, eps2=12 + 1j, center=(0.0, 0.0, z))
+    Gb, Go = pair(sphere(n), buffem.Material(kind=buffem.BG_MAT_JANUS_Z, **kw),
+                  oracle_lib.material(kind=oracle_lib.MAT_JANUS_Z, **kw), oracle_lib=oracle_lib)
+    rng = np.random.default_rng(n)
+    J = rng.normal(size=Gb.TotalBFs) + 1j * rng.normal(size=Gb.TotalBFs)
+    for omega in (0.9, 0.7 + 0.1j):
+        got = Gb.GetPFTMatrix(J, omega, method=buffem.BG_PFT_OVERLAP)[0, 0]
+        np.testing.assert_allclose(got, Go.pft_opft(complex(omega), J)[0], rtol=1e-9)
