@@ -327,6 +327,7 @@ GmInfo gmres_last_info();
 int gmres_solve_mixed(bg_matrix *A, bg_matrix *F, const bg_precond *P, void *dB, int ldb, int nrhs, double tol,
                       int restart, int maxit, double inner_tol, double *stats);
 int precond_jacobi(bg_matrix *A, bg_precond **out);
+int zgemm_fp64_device(int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C, int ldc);
 int zgemm_sub_device(int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C, int ldc);
 int cgemm_sub_device(int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C, int ldc);
 int matrix_convert(const bg_matrix *src, bg_matrix *dst);

@@ -264,12 +264,8 @@ __device__ __forceinline__ void dmma8(double (&d)[4], const double (&a)[4], cons
 #define ZS_BP 36                 // Bs[n][k] stride, = 4 mod 8
 #define ZS_STAGE (32 * ZS_AP + 32 * ZS_BP)
 #define ZS_SMEM (ZS_ST * ZS_STAGE * 16)
-__global__ void __launch_bounds__(128) k_zgemm_small(int M, int N, int K, const cdl *__restrict__ A, size_t lda,
-                                                      const cdl *__restrict__ B, size_t ldb, cdl *C, size_t ldc) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  pdl_enter();
-  cdl *sm = (cdl *)smem_raw;
-  const int m0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
+__device__ __forceinline__ void zgemm_small_tile(cdl *sm, int m0, int n0, int M, int N, int K, const cdl *__restrict__ A,
+                                                 size_t lda, const cdl *__restrict__ B, size_t ldb, cdl *C, size_t ldc) {
   const int tid = threadIdx.x, lane = tid & 31, wk = tid >> 5, t0 = lane & 3, t1 = lane >> 2;
   double cr[2][4][4], ci[2][4][4];
 #pragma unroll
@@ -362,6 +358,52 @@ __global__ void __launch_bounds__(128) k_zgemm_small(int M, int N, int K, const 
     if (m0 + lane < M && col < N) C[(size_t)col * ldc + m0 + lane] = cdl{x[e].r - s.r, x[e].i - s.i};
   }
 }
+__global__ void __launch_bounds__(128) k_zgemm_small(int M, int N, int K, const cdl *__restrict__ A, size_t lda,
+                                                      const cdl *__restrict__ B, size_t ldb, cdl *C, size_t ldc) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  pdl_enter();
+  zgemm_small_tile((cdl *)smem_raw, blockIdx.x * 32, blockIdx.y * 32, M, N, K, A, lda, B, ldb, C, ldc);
+}
+// The parts of C that the INT8 path leaves out: 128 x 64 tiles with a flag (tile (tm, tn)
+// at tn * ntm + tm), eight 32 x 32 tiles each, so that the CTAs share few of them evenly
+// (a CTA per 128 x 64 tile: one of K = 2,048 takes 0.54 ms).  With no flag 3 us.
+#define ZF_MAX 2048              // flags of one launch at most
+__global__ void __launch_bounds__(128) k_zgemm_flagged(int M, int N, int K, const cdl *__restrict__ A, size_t lda,
+                                                        const cdl *__restrict__ B, size_t ldb, cdl *C, size_t ldc,
+                                                        const unsigned char *flag, int ntm, int ntiles) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ unsigned short list[ZF_MAX];
+  __shared__ int wsum[4];
+  pdl_enter();
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  int n = 0, total = 0;
+  for (int i = 0; i < ZF_MAX / 128; i++) {
+    const int t = tid * (ZF_MAX / 128) + i;
+    n += t < ntiles && flag[t] != 0;
+  }
+  if (!__syncthreads_or(n)) return;
+  int x = n;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) wsum[wid] = x;
+  __syncthreads();
+  x -= n;
+  for (int w = 0; w < 4; w++) {
+    if (w < wid) x += wsum[w];
+    total += wsum[w];
+  }
+  for (int i = 0; i < ZF_MAX / 128; i++) {
+    const int t = tid * (ZF_MAX / 128) + i;
+    if (t < ntiles && flag[t]) list[x++] = (unsigned short)t;
+  }
+  for (int u = blockIdx.x; u < 8 * total; u += gridDim.x) {
+    __syncthreads();
+    const int t = list[u >> 3], m0 = t % ntm * 128 + (u & 3) * 32, n0 = t / ntm * 64 + ((u >> 2) & 1) * 32;
+    if (m0 < M && n0 < N) zgemm_small_tile((cdl *)smem_raw, m0, n0, M, N, K, A, lda, B, ldb, C, ldc);
+  }
+}
 static int zgemm_small(int M, int N, int K, const cdl *A, size_t lda, const cdl *B, size_t ldb, cdl *C, size_t ldc) {
   static bool attr = false;
   if (!attr) {
@@ -395,6 +437,21 @@ static int zgemm_launch(int M, int N, int K, const cdl *A, size_t lda, const cdl
   BG_LAUNCHED();
   return BG_OK;
 }
+// the tiles with a flag (gemm_i8.cu: at most 4,096 x 4,096)
+int zgemm_flagged(int M, int N, int K, const void *A, size_t lda, const void *B, size_t ldb, void *C, size_t ldc,
+                  const unsigned char *flag) {
+  static bool attr = false;
+  if (!attr) {
+    BG_CUDA_TRY(cudaFuncSetAttribute(k_zgemm_flagged, cudaFuncAttributeMaxDynamicSharedMemorySize, ZS_SMEM));
+    attr = true;
+  }
+  const int ntm = (M + 127) / 128, ntiles = ntm * ((N + 63) / 64);
+  if (ntiles > ZF_MAX) { set_error("zgemm: too many tiles"); return BG_ERR_ARG; }
+  BG_CUDA_TRY(pdl_launch(k_zgemm_flagged, dim3(std::min(8 * ntiles, 2 * 148)), 128, ZS_SMEM, M, N, K, (const cdl *)A, lda,
+                         (const cdl *)B, ldb, (cdl *)C, ldc, flag, ntm, ntiles));
+  BG_LAUNCHED();
+  return BG_OK;
+}
 
 // scratch of the INT8 path, set around the calls that may take it
 struct I8Scratch {
@@ -404,15 +461,16 @@ struct I8Scratch {
 };
 static thread_local I8Scratch *t_i8 = nullptr;
 // Which products go there, from measured times in us: 128 x 64 tiles in waves of
-// 148 at 0.117 us per column of K and 8.9 us for the two combinations, 15 us of
-// launches, splitting at 64 bytes per element of A and B and 5 TB/s; the FP64
-// tiles at 28 TFLOP/s.  Measured INT8 / FP64: 2048 x 512 x 512 95 /
-// 141 us, 1350 x 672 x 672 117 / 203, 4096 x 4096 x 128 380 / 640, 1024^3 163 /
-// 304, 9936 x 9936 x 1024 11.0 / 24.9 ms; 2048 x 1024 x 128 78 / 90 us.
+// 148 at 0.117 us per column of K and 8.9 us for the two combinations, 36 us of
+// launches and of the guard, exponents and splitting at 96 bytes per element of A and B and
+// 5 TB/s; the FP64 tiles at 28 TFLOP/s.  Measured INT8 / FP64, calls one by one:
+// 2048 x 512 x 512 140 / 157 us, 1350 x 672 x 672 162 / 203, 4096 x 4096 x 128
+// 443 / 641, 1024^3 210 / 304, 9936 x 9936 x 1024 12.0 / 24.9 ms; 2048 x 1024 x 128
+// 113 / 89 us.
 static bool i8_takes(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return false;
   const double tiles = std::ceil((double)M / 128) * std::ceil((double)N / 64);
-  const double split = 15.0 + ((double)M + N) * K * (64 / 5e6);
+  const double split = 36.0 + ((double)M + N) * K * (96 / 5e6);
   const double i8 = std::ceil(tiles / 148) * (0.117 * K + 8.9) + split, fp64 = 8.0 * M * (double)N * K / 28e6;
   return i8 < 0.95 * fp64;
 }
@@ -1700,6 +1758,14 @@ int lu_factor(bg_matrix *m) {
   }
   if ((st = build_perm(m))) return st;
   return info[0];
+}
+
+// by FP64 whatever the size, without a synchronisation: buff-neq's products with S^-1,
+// whose entries fall off so fast that most of their tiles would be left out of the digits
+// (flux of two bodies, N = 2,022: 12.6 -> 12.4 ms, 5,172: 122 -> 119)
+int zgemm_fp64_device(int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C, int ldc) {
+  int st = ensure_device();
+  return st ? st : zgemm_sub(M, N, K, (const cdl *)A, (size_t)lda, (const cdl *)B, (size_t)ldb, (cdl *)C, (size_t)ldc);
 }
 
 int zgemm_sub_device(int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C, int ldc) {

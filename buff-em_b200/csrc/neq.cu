@@ -180,7 +180,7 @@ int neq_prepare(bg_neq *h, double wr, double wi) {
   for (int o = 0; o < NO; o++) {
     int r0 = off[o], n = off[o + 1] - off[o];
     if ((st = launch_zero(h->M1 + r0, ld, n, N))) return st;
-    if ((st = zgemm_sub_device(n, N, n, h->Sinv + r0 + (size_t)r0 * ld, N, h->M2 + r0, N, h->M1 + r0, N))) return st;
+    if ((st = zgemm_fp64_device(n, N, n, h->Sinv + r0 + (size_t)r0 * ld, N, h->M2 + r0, N, h->M1 + r0, N))) return st;
   }
   // M2 <- V M1 = -V S^-1 G
   for (int c0 = 0; c0 < N; c0 += YMAX) {
@@ -195,7 +195,7 @@ int neq_prepare(bg_neq *h, double wr, double wi) {
   for (int o = 0; o < NO; o++) {
     int r0 = off[o], n = off[o + 1] - off[o];
     if ((st = launch_zero(Wd + r0, ldw, n, N))) return st;
-    if ((st = zgemm_sub_device(n, N, n, h->Sinv + r0 + (size_t)r0 * ld, N, h->M2 + r0, N, Wd + r0, (int)ldw))) return st;
+    if ((st = zgemm_fp64_device(n, N, n, h->Sinv + r0 + (size_t)r0 * ld, N, h->M2 + r0, N, Wd + r0, (int)ldw))) return st;
   }
   k_add_identity<<<(N + 255) / 256, 256, 0, stream()>>>(Wd, ldw, N, 1.0);
   BG_LAUNCHED();
@@ -224,7 +224,7 @@ int neq_dr(bg_neq *h, int s) {
   }
   // M1 <- -(S^-1 R_s) S^-1 = -SRS, nonzero in the (s, s) block only
   if ((st = launch_zero(h->M1, ld, N, N))) return st;
-  if ((st = zgemm_sub_device(ns, ns, ns, h->M2 + c0 + (size_t)c0 * ld, N, h->Sinv + c0 + (size_t)c0 * ld, N,
+  if ((st = zgemm_fp64_device(ns, ns, ns, h->M2 + c0 + (size_t)c0 * ld, N, h->Sinv + c0 + (size_t)c0 * ld, N,
                              h->M1 + c0 + (size_t)c0 * ld, N)))
     return st;
   // M1[:, s] <- W^-1 (-SRS)[:, s]; the other columns stay exactly zero
