@@ -1806,12 +1806,16 @@ int zgemm_sub_device(int M, int N, int K, const void *A, int lda, const void *B,
 // also makes the other CTAs give up early.
 // The chain from block to block sets the time: flag and data through L2, one
 // 64 x 64 product, the diagonal solve.  The 16 x 16 diagonal blocks are
-// inverted while the CTA waits, so the solve is four 16-wide products and the
-// updates between them instead of 64 dependent substitutions with a shuffle
-// each; every thread polls the flag and fetches its own entry of the solved
-// block (one barrier a block).  Two sweeps of one right-hand side: 1.31 ->
-// 0.62 ms at N = 4,092, complex64 at N = 19,872 3.9 -> 1.9 ms (10 -> 4.8 us a
-// block).
+// inverted while the CTA waits, so the solve of one is three 16-wide products
+// (x = T^{-1} b, r = b - T x, x += T^{-1} r) instead of 16 dependent substitutions
+// with a shuffle each; every thread polls the flag and fetches its own entry of the
+// solved block (one barrier a block).  The correction makes the residual that of
+// substitution, a few units in the last place of |T||x|: x = T^{-1} b alone leaves
+// cond(T) times that (componentwise backward error of a solve at N = 4,092, 48 systems:
+// 6.2e-16 with substitution, 8.7e-16 without the correction, 6.6e-16 with it).  One
+// correction squares cond(T) eps, so blocks beyond TrsvCond are solved by substitution.
+// Solve of one right-hand side: 1.10 ms by substitution throughout, 0.73 ms now (0.51
+// without the correction) at N = 4,092; complex64 at N = 19,872 3.9 and 2.7 ms (1.9).
 // =========================================================================
 #define TV_B 64
 #define TV_MAXRHS 4
@@ -1824,9 +1828,14 @@ __global__ void k_gather_rows(int N, int nrhs, const int *perm, const C *src, si
   if (i < N && j < nrhs) dst[(size_t)j * ldd + i] = src[(size_t)j * lds + perm[i]];
 }
 
+// 1-norm condition of a 16 x 16 block up to which it is solved by its inverse: 16 cond eps
+// squared stays below eps
+template <class C> struct TrsvCond;
+template <> struct TrsvCond<cdl> { static constexpr double MAX = 1e6; };
+template <> struct TrsvCond<cfl> { static constexpr float MAX = 200.f; };
 template <class C>
 constexpr int trsv_smem() {
-  return TV_B * (TV_B + 1) * (int)sizeof(C) + 3 * TV_B * TV_MAXRHS * (int)sizeof(C);
+  return TV_B * (TV_B + 1) * (int)sizeof(C) + 4 * TV_B * TV_MAXRHS * (int)sizeof(C) + TV_B * 17 * (int)sizeof(C);
 }
 
 __device__ __forceinline__ int ld_acquire(const int *p) {
@@ -1843,13 +1852,15 @@ __global__ void __launch_bounds__(128) k_trsv(int N, const C *A, size_t ld, C *X
                                               int epoch, int *ticket, int *err) {
   typedef typename CxT<C>::R R;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  C(*D)[TV_B + 1] = (C(*)[TV_B + 1])smem_raw;   // diagonal block; its 16 x 16 diagonal blocks become their inverses
+  C(*D)[TV_B + 1] = (C(*)[TV_B + 1])smem_raw;   // diagonal block, the other triangle of its 16 x 16 diagonal blocks zero
   C(*part)[TV_MAXRHS] = (C(*)[TV_MAXRHS])(smem_raw + TV_B * (TV_B + 1) * sizeof(C));   // part[row][rhs]
   C(*xs)[TV_B][TV_MAXRHS] = (C(*)[TV_B][TV_MAXRHS])(part + TV_B);                     // solved blocks, two buffers
-  __shared__ int s_blk, s_abort;
+  C(*sol)[TV_MAXRHS] = (C(*)[TV_MAXRHS])(xs + 2);                                    // solution and residual of a diagonal block
+  C(*Iv)[17] = (C(*)[17])(sol + TV_B);                                               // inverses of the four diagonal blocks
+  __shared__ int s_blk, s_abort, s_subst;                                            // s_subst: blocks to solve by substitution
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nb = (N + TV_B - 1) / TV_B;
-  if (tid == 0) { s_blk = atomicAdd(ticket, 1); s_abort = 0; }
+  if (tid == 0) { s_blk = atomicAdd(ticket, 1); s_abort = s_subst = 0; }
   __syncthreads();
   const int lb = s_blk;
   const int bi = UPPER ? nb - 1 - lb : lb;
@@ -1872,8 +1883,12 @@ __global__ void __launch_bounds__(128) k_trsv(int N, const C *A, size_t ld, C *X
     }
 #pragma unroll
     for (int u = 0; u < 8; u++) {
-      const int e = e0 + u * 128 + tid;
-      D[e % TV_B][e / TV_B] = v[u];
+      const int e = e0 + u * 128 + tid, r = e % TV_B, c = e / TV_B;
+      if (r / 16 == c / 16) {
+        if (UPPER ? r > c : r < c) v[u] = C{0, 0};
+        if (!UPPER && r == c) v[u] = C{1, 0};
+      }
+      D[r][c] = v[u];
     }
   }
   __syncthreads();
@@ -1902,10 +1917,20 @@ __global__ void __launch_bounds__(128) k_trsv(int N, const C *A, size_t ld, C *X
         }
       }
     }
-    __syncthreads();
-    if (tid < TV_B)
+    if (tid < TV_B) {
+      R si = 0, st = 0;      // column sums of the inverse and of the block
 #pragma unroll
-      for (int i = 0; i < 16; i++) D[o + i][o + c] = v[i];
+      for (int i = 0; i < 16; i++) {
+        Iv[o + i][c] = v[i];
+        const C t = D[o + i][o + c];
+        si += fabs(v[i].r) + fabs(v[i].i);
+        st += fabs(t.r) + fabs(t.i);
+      }
+      R mt = st;
+#pragma unroll
+      for (int k = 8; k > 0; k >>= 1) mt = max(mt, __shfl_xor_sync(0xffffffffu, mt, k));
+      if (!(si * mt <= TrsvCond<C>::MAX && st == st)) atomicOr(&s_subst, 1 << s);
+    }
   }
   C acc[TV_MAXRHS];
 #pragma unroll
@@ -1978,17 +2003,43 @@ __global__ void __launch_bounds__(128) k_trsv(int N, const C *A, size_t ld, C *X
 #pragma unroll
     for (int t = 0; t < 4; t++) {
       const int o = 16 * (UPPER ? 3 - t : t);
-      // y = inverse times b of this block: row r, columns 8 h .. 8 h + 7
-      C y{0, 0}, z{0, 0};
+      // row r of M v, columns 8 h .. 8 h + 7 by each half of the warp
+      auto times = [&](const C *M, const C(*v)[TV_MAXRHS]) {
+        C y[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
 #pragma unroll
-      for (int k = 0; k < 8; k += 2) {
-        y = cmac(y, D[o + r][o + 8 * h + k], part[o + 8 * h + k][j]);
-        z = cmac(z, D[o + r][o + 8 * h + k + 1], part[o + 8 * h + k + 1][j]);
+        for (int k = 0; k < 8; k++) y[k & 3] = cmac(y[k & 3], M[8 * h + k], v[8 * h + k][j]);
+        C w{(y[0].r + y[1].r) + (y[2].r + y[3].r), (y[0].i + y[1].i) + (y[2].i + y[3].i)};
+        w.r += __shfl_xor_sync(0xffffffffu, w.r, 16);
+        w.i += __shfl_xor_sync(0xffffffffu, w.i, 16);
+        return w;
+      };
+      C y;
+      if (!(s_subst >> (o / 16) & 1)) {
+        y = times(Iv[o + r], part + o);
+        if (h == 0) sol[o + r][j] = y;
+        __syncwarp();
+        const C t = times(&D[o + r][o], sol + o), b = part[o + r][j];
+        __syncwarp();
+        if (h == 0) sol[o + r][j] = C{b.r - t.r, b.i - t.i};
+        __syncwarp();
+        const C d = times(Iv[o + r], sol + o);
+        y.r += d.r;
+        y.i += d.i;
+      } else {
+        y = part[o + r][j];
+        for (int n = 0; n < 16; n++) {
+          const int i = UPPER ? 15 - n : n;
+          C x = cshfl(y, i);
+          if (UPPER) {
+            const C u = D[o + i][o + i];
+            const R d = u.r * u.r + u.i * u.i;
+            const C iu{u.r / d, -u.i / d};
+            x = C{x.r * iu.r - x.i * iu.i, x.r * iu.i + x.i * iu.r};
+          }
+          if (r == i) y = x;
+          else if (UPPER ? r < i : r > i) y = cfms(y, D[o + r][o + i], x);
+        }
       }
-      y.r += z.r;
-      y.i += z.i;
-      y.r += __shfl_xor_sync(0xffffffffu, y.r, 16);
-      y.i += __shfl_xor_sync(0xffffffffu, y.i, 16);
       __syncwarp();
       if (h == 0) {
         part[o + r][j] = y;
@@ -1999,15 +2050,12 @@ __global__ void __launch_bounds__(128) k_trsv(int N, const C *A, size_t ld, C *X
       if (t < 3) {
         const int left = 16 * (3 - t), base = UPPER ? 0 : o + 16;
         for (int q = lane; q < left; q += 32) {
-          C s{0, 0}, s2{0, 0};
+          C s[4] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}};
 #pragma unroll
-          for (int k = 0; k < 16; k += 2) {
-            s = cmac(s, D[base + q][o + k], part[o + k][j]);
-            s2 = cmac(s2, D[base + q][o + k + 1], part[o + k + 1][j]);
-          }
+          for (int k = 0; k < 16; k++) s[k & 3] = cmac(s[k & 3], D[base + q][o + k], part[o + k][j]);
           C p = part[base + q][j];
-          p.r -= s.r + s2.r;
-          p.i -= s.i + s2.i;
+          p.r -= (s[0].r + s[1].r) + (s[2].r + s[3].r);
+          p.i -= (s[0].i + s[1].i) + (s[2].i + s[3].i);
           part[base + q][j] = p;
         }
         __syncwarp();
