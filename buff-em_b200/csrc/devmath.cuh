@@ -1,11 +1,14 @@
 // Device arithmetic shared by the kernels.
 #pragma once
 
-// 1/sqrt(x) for normal positive x: the hardware approximation (about 2^-22)
-// and one step of the third-order iteration y + y e (1/2 + 3/8 e),
-// e = 1 - x y^2 (the binomial series of (1 - e)^{-1/2}; what it omits is
-// 5/16 e^3, below 2^-64).  Five FP64 operations without a branch, so the point
-// loops that call it can be interleaved; within 2 ulp of the exact value.
+// 1/sqrt(x) for normal positive x: the hardware approximation y (about 2^-22)
+// and one step of Householder's iteration of order three (A. S. Householder, The
+// Numerical Treatment of a Single Nonlinear Equation, 1970) for y^-2 - x,
+//   y + y e (1/2 + 3/8 e),  e = 1 - x y^2,
+// which is the binomial series of (1 - e)^{-1/2} cut after e^2 (omitted: 5/16 e^3,
+// below 2^-64).  Five FP64 operations without a branch, so the point loops that
+// call it can be interleaved.  Relative error at most 1.5 2^-53 (x y rounded once,
+// 2^-53 in e, half of that in the result; the last operation 2^-53).
 __device__ __forceinline__ double rsqrt_fast(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
