@@ -1696,10 +1696,32 @@ static int lu_work_alloc(bg_matrix *m, size_t need) {
   return BG_OK;
 }
 
+// the products (M, N, K) of a triangular solve and of a factorisation, as trsm and getrf_rec form them
+template <class F>
+static void trsm_products(int n, int m, F &&f) {
+  if (n <= TRS_MAX) return;
+  const int n1 = (n / 2 + TRS_MAX - 1) / TRS_MAX * TRS_MAX;
+  trsm_products(n1, m, f);
+  f(n - n1, m, n1);
+  trsm_products(n - n1, m, f);
+}
+template <class F>
+static void getrf_products(int N, int k0, int n, F &&f) {
+  if (n <= LU_BLOCK) return;
+  const int n1 = (n / 2 + LU_BLOCK - 1) / LU_BLOCK * LU_BLOCK;
+  getrf_products(N, k0, n1, f);
+  trsm_products(n1, n - n1, f);
+  f(N - k0 - n1, n - n1, n1);
+  getrf_products(N, k0 + n1, n - n1, f);
+}
+
 // scratch of the INT8 products of a factorisation (0: every product is too small for them)
 static size_t i8_factor_bytes(int N) {
-  const int h = N / 2 + LU_BLOCK;
-  return i8_takes(N, h, h) ? zgemm_i8_bytes(N, h, h) : 0;
+  size_t b = 0;
+  getrf_products(N, 0, N, [&](int m, int n, int k) {
+    if (i8_takes(m, n, k)) b = std::max(b, zgemm_i8_bytes(m, n, k));
+  });
+  return b;
 }
 
 int lu_factor(bg_matrix *m) {
@@ -2133,9 +2155,13 @@ int lu_solve_many(bg_matrix *m, void *dB, size_t ldb, int nrhs) {
   int w = std::min(chunk, nrhs);
   if (w <= 0) return BG_OK;
   BG_CUDA_TRY(cudaMallocAsync((void **)&T, sizeof(cdl) * (size_t)N * w, stream()));
-  // scratch of the INT8 products, where some are large enough for them
-  const int h = N / 2 + TRS_MAX;
-  I8Scratch sc{nullptr, i8_takes(h, w, h) ? zgemm_i8_bytes(h, w, h) : 0, nullptr};
+  // scratch of the INT8 products, where some are large enough for them (the products
+  // of the upper solve have rows and inner index exchanged)
+  I8Scratch sc{nullptr, 0, nullptr};
+  trsm_products(N, w, [&](int m, int n, int k) {
+    if (i8_takes(m, n, k)) sc.bytes = std::max(sc.bytes, zgemm_i8_bytes(m, n, k));
+    if (i8_takes(k, n, m)) sc.bytes = std::max(sc.bytes, zgemm_i8_bytes(k, n, m));
+  });
   if (sc.bytes && cudaMallocAsync(&sc.p, sc.bytes + 256, stream()) != cudaSuccess) {
     cudaGetLastError();
     sc.p = nullptr;
