@@ -15,12 +15,12 @@
 //    thousands of launches of the recursive LU;
 //  * a geometry's jobs are spread over S slots, each with its own stream,
 //    matrix and buffers, so that small factorisations run concurrently;
-//  * an online autotuner picks, per size class (N rounded up to 1024), the
-//    LU panel slice height (rows per CTA of the shared-memory panel kernel, which
-//    only matrices above 37,888 rows still use: 16, 32 or 64), the CTA tile of the complex128 tensor-core GEMM (64 x 64,
-//    128 x 64 or 64 x 128) and the number of concurrent slots (1, 2, 4, ... up
-//    to the caller's maximum) by
-//    timing the sweep's own first jobs (their results are kept), and
+//  * an online autotuner picks, per size class (N rounded up to 1024), the number
+//    of concurrent slots (1, 2, 4, ... up to the caller's maximum) and, where the size
+//    reaches the kernels they belong to, the rows per CTA of the shared-memory panel (16,
+//    32 or 64; above 37,888 rows) and the CTA tile of the FP64 products (64 x 64,
+//    128 x 64 or 64 x 128; products too large for the 32 x 32 tiles and too small for
+//    the INT8 path) by timing the sweep's own first jobs (their results are kept), and
 //    remembers the choice for later geometries of the same class.
 #include <cuda_runtime.h>
 
@@ -221,11 +221,12 @@ static int sweep_geometry(bg_geometry *g, const double *omega, int nw, const dou
   const int saved_rows = lu_get_panel_rows(), saved_tile = lu_get_gemm_tile();
   const bool tuned_now = tn.rows == 0;
   if (tuned_now) {
-    // panel slice height, one slot, one job each (the first is also the warm-up)
+    // one slot, one job each: the panel slice height where it matters, else only the
+    // default (the first job is also the warm-up)
     double best = 1e30;
     int best_rows = saved_rows;
-    const int cand_rows[3] = {32, 16, 64};
-    for (int c = 0; c < 3 && j < nw; c++) {
+    const int cand_rows[3] = {32, 16, 64}, nrows = lu_uses_panel_rows(g->N) ? 3 : 1;
+    for (int c = 0; c < nrows && j < nw; c++) {
       lu_set_panel_rows(cand_rows[c]);
       slots.resize(1);
       if ((st = slot_init(g, slots[0], E0, nhat, use_graph))) break;
@@ -245,7 +246,7 @@ static int sweep_geometry(bg_geometry *g, const double *omega, int nw, const dou
     lu_set_panel_rows(best_rows);
     // GEMM tile: the 64 x 64 default was timed above; one job each for the others
     int best_tile = saved_tile;
-    for (int tile = 1; tile <= 2 && j < nw && !st; tile++) {
+    for (int tile = 1; tile <= 2 && j < nw && !st && lu_uses_gemm_tile(g->N); tile++) {
       lu_set_gemm_tile(tile);
       slots.resize(1);
       if ((st = slot_init(g, slots[0], E0, nhat, use_graph))) break;

@@ -1724,6 +1724,17 @@ static size_t i8_factor_bytes(int N) {
   return b;
 }
 
+// whether a factorisation in complex128 depends on the settings that a batched sweep tunes:
+// rows per CTA of the shared-memory panel, CTA tile of the FP64 products
+bool lu_uses_panel_rows(int N) { return N > std::min(panel_max_grid, panel_grid ? panel_grid : panel_max_grid) * PRG_T; }
+bool lu_uses_gemm_tile(int N) {
+  bool used = false;
+  getrf_products(N, 0, N, [&](int m, int n, int k) {
+    used |= !i8_takes(m, n, k) && (long)((m + 63) / 64) * ((n + 63) / 64) > ZG_SMALL;
+  });
+  return used;
+}
+
 int lu_factor(bg_matrix *m) {
   int st = ensure_device();
   if (!st) st = panel_init();

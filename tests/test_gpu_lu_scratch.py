@@ -45,3 +45,20 @@ def test_scratch_only_for_products_that_use_it(N, digits):
     x = np.asfortranarray(A @ np.ones((N, 1), complex))
     M.LUSolve(x)
     np.testing.assert_allclose(x, np.ones((N, 1)), rtol=0, atol=1e-9)
+
+
+def test_sweep_tunes_only_what_the_size_reaches(sphere):
+    """A first sweep of a size class on one slot records the job's launches once for the
+    tuning job and once for the sweep (no panel height and no GEMM tile to choose at
+    N = 2,376), a later one once."""
+    wave = buffem.PlaneWave([1, 0, 0], [0, 0, 1])
+    small = buffem.SWGGeometry(meshfiles=sphere(2), materials=buffem.Material(eps=4 + 0.2j))
+    buffem.BatchSweep([small], [0.5, 0.6], wave, max_streams=1)      # kernel attributes and tables in place
+    G = buffem.SWGGeometry(meshfiles=sphere(6), materials=buffem.Material(eps=4 + 0.2j))
+    G.precompute()
+    omegas = np.linspace(0.5, 1.0, 14)
+    n = [buffem.launch_count()]
+    for _ in range(2):
+        buffem.BatchSweep([G], omegas, wave, max_streams=1)
+        n.append(buffem.launch_count())
+    assert n[1] - n[0] <= 2 * (n[2] - n[1])
