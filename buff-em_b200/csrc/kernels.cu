@@ -1369,7 +1369,10 @@ __global__ void __launch_bounds__(128) k_opft(PftArgs P, cd omega, double *part,
   const int id = blockIdx.x * blockDim.x + threadIdx.x, t = id / 33;
   double contrib = 0.0;
   int obj = 0;
-  if (t < g.NT) {
+  // a tetrahedron without a basis function adds nothing, whatever eps is there
+  // (eps = 1 has no inverse)
+  const int4 fi = t < g.NT ? g.tetFI[t] : make_int4(-1, -1, -1, -1);
+  if (max(max(fi.x, fi.y), max(fi.z, fi.w)) >= 0) {
     obj = g.tetObj[t];
     const cd pre0 = cdiv(cmk(0, 376.73031346177), omega);
     const int kind = g.mats[obj].kind;

@@ -36,3 +36,19 @@ def test_points_on_the_jump(sphere, oracle_lib, cells, radius):
     for omega in (0.9, 0.7 + 0.1j):
         got = Gb.GetPFTMatrix(J, omega, method=buffem.BG_PFT_OVERLAP)[:, 0]
         np.testing.assert_allclose(got, Go.pft_opft(complex(omega), J), rtol=1e-9)
+
+
+def test_tetrahedron_without_basis_functions(sphere, tmp_path):
+    """An object of one tetrahedron has no basis function and absorbs nothing, also
+    where its permittivity is that of vacuum."""
+    path = str(tmp_path / "one.vmsh")
+    with open(path, "w") as f:
+        f.write("$MeshFormat\n2.2 0 8\n$EndMeshFormat\n$Nodes\n4\n1 0 0 0\n2 1 0 0\n3 0 1 0\n4 0 0 1\n$EndNodes\n"
+                "$Elements\n1\n1 4 2 0 1 1 2 3 4\n$EndElements\n")
+    G = buffem.SWGGeometry(meshfiles=[sphere(2), path], materials=[buffem.Material(eps=4 + 0.2j), buffem.Material(eps=1.0)],
+                           displacements=[[0, 0, 0], [0, 0, 3.0]])
+    alone = buffem.SWGGeometry(meshfiles=sphere(2), materials=buffem.Material(eps=4 + 0.2j))
+    J = np.exp(1j * np.arange(G.TotalBFs))
+    got = G.GetPFTMatrix(J, 0.9, method=buffem.BG_PFT_OVERLAP)[:, 0]
+    assert got[1] == 0
+    np.testing.assert_allclose(got[0], alone.GetPFTMatrix(J, 0.9, method=buffem.BG_PFT_OVERLAP)[0, 0], rtol=1e-13)
