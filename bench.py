@@ -12,7 +12,8 @@ One step = one frequency.
     network (shipped weights), assemble the RHS, solve by GMRES(80) on the
     complex64 copy with FP64 refinement against the complex128 matrix to a
     1e-10 relative residual, LU fallback if 1000 Krylov steps do not reach it.
-  fp64_path: assemble, FP64 LU (DMMA tensor cores), FP64 solve -- the plain
+  fp64_path: assemble, complex128 LU (large products by INT8 digits within FP64's
+  error bound, the rest on the FP64 tensor cores), solve -- the plain
     path and the reference answer: the learned answer's error is measured against it.
 The same two paths plus the precision form (complex64 tcgen05 LU + FP64
 refinement) also run on the 12^3-cell sphere (N = 19,872) with the
@@ -917,7 +918,7 @@ def main():
                     help="headline learned steps only (no FP64 arm, e2e, secondary, CPU baseline): profiler runs")
     ap.add_argument("--kernel", default=None, choices=["gemm", "cgemm", "fields", "neq", "precision"],
                     help="one small case for profilers: gemm = the LU trailing-update GEMM on an M=N=K=--size "
-                         "problem (complex128, DMMA); cgemm = the same on the complex64 tcgen05 GEMM of the "
+                         "problem (complex128, INT8 digits or DMMA); cgemm = the same on the complex64 tcgen05 GEMM of the "
                          "precision form; fields = two GetFields calls, 2048 far points on the --size-cell "
                          "sphere; neq = two buff-neq flux frequencies on the --size-cell sphere; precision = "
                          "one precision-form step (complex64 LU + FP64 refinement) on the --n-cell sphere")

@@ -1,7 +1,7 @@
 // Batching form: frequency sweeps over several geometries of uneven N.
 //
 // A job is one (geometry, omega): assemble the complex128 VIE matrix, LU
-// factor it (FP64 tensor-core path), solve one plane-wave right-hand side
+// factor it (complex128), solve one plane-wave right-hand side
 // and reduce the absorbed power of every object (overlap method) -- the
 // per-frequency work of a sweep such as a heat-transfer spectrum.  No
 // reference counterpart: the reference runs such sweeps one frequency at a

@@ -518,8 +518,8 @@ __device__ __forceinline__ C cshfl(C v, int src) {
 // later rows, those of the following blocks included, so the off-diagonal
 // products need no further pass where a 64-row leaf left them to GEMM launches
 // of 64 rows.  TRSM class of one factorisation: 5.2 -> 1.5 ms at N = 4,092,
-// 41 -> 23 ms at N = 19,872 (complex64 32 -> 13 ms).  CPW is the largest of
-// 4, 2, 1 that still gives every SM a CTA.
+// 41 -> 23 ms at N = 19,872 (complex64 32 -> 13 ms).  CPW is the smallest of
+// 1, 2, 4 with which all CTAs run at once.
 // =========================================================================
 #define TRS_WARPS 8
 #define TRS_MAX 128

@@ -13,7 +13,7 @@
 // B200 layout: every matrix is dense complex128 in HBM, column-major with
 // leading dimension N.  S^-1 is frequency independent and kept for the
 // geometry's lifetime.  Products with S^-1 and the two N-column solves run
-// on the FP64 tensor-core GEMM (the same recursive kernels as the LU); the
+// on the products of the LU (those with S^-1 by FP64 outright); the
 // sparse V and R_s products are gathers of <= 7 entries per row.  S, V and
 // R_s couple only basis functions of one object, so S^-1 is block diagonal
 // and S^-1 R_s S^-1 lives in the (s, s) block: the chain skips the columns

@@ -35,7 +35,7 @@ extern "C" {
 #define BG_ERR_NUMERIC (-7)   /* non-finite value detected */
 
 /* matrix storage precisions */
-#define BG_C128 0             /* complex128 (the plain FP64 path) */
+#define BG_C128 0             /* complex128 (the plain path, FP64 accuracy throughout) */
 #define BG_C64 1              /* complex64 (precision form)          */
 
 /* permittivity functors (replace SVTensor / MatProp expressions,
@@ -265,9 +265,16 @@ int bg_lu_solve_device(bg_matrix *m, void *B_dev, int ldb, int nrhs);
 int bg_lu_solve_device_noalloc(bg_matrix *m, void *B_dev, int ldb, int nrhs);
 
 /* C <- C - A*B for device column-major complex128 matrices (A: M x K, B: K x N,
-   C: M x N), the FP64 tensor-core GEMM of the LU trailing update.  Also the
-   building block of buff-neq's dressed-Rytov chain (GetFlux.cc:155-272, four
-   GEMMs per source object).  Runs on the library stream. */
+   C: M x N), the GEMM of the LU trailing update.  Runs on the library stream.
+   Large products are formed from 8-bit digits on the INT8 tensor cores, tile by
+   tile where no entry can lose more than FP64 arithmetic does (every entry within
+   about K 2^-52 of sum |A||B| by real and imaginary part, as a chain of FP64
+   operations), the rest and all small products on the FP64 tensor cores.  The
+   digits need scratch (at most about 0.5 GB, from the stream-ordered pool); without
+   it FP64 forms the whole product, so two calls on the same data may differ in
+   the last bits.  A call that takes digits synchronises the stream; a timeout
+   inside a kernel is reported as BG_ERR_CUDA.  The same products serve bg_lu_factor
+   on a BG_C128 matrix, bg_neq_* and bg_batch_sweep. */
 int bg_zgemm_sub_device(int M, int N, int K, const void *A, int lda, const void *B, int ldb, void *C, int ldc);
 
 /* C <- C - A*B for device column-major complex64 matrices: the tcgen05
