@@ -851,8 +851,10 @@ __global__ void __launch_bounds__(256) k_panel(PanelArgs<C> P) {
         int ob = __shfl_xor_sync(0xffffffffu, b, o);
         if (better(ov, oi, v, i)) { v = ov; i = oi; b = ob; }
       }
-      if (lane < w) prow[lane] = P.crow[((size_t)buf * G + b) * 32 + lane];
-      if (lane == 0) s_piv = i;
+      // a column of NaNs has no candidate and takes its own row
+      const bool none = i == 0x7fffffff;
+      if (lane < w) prow[lane] = none ? P.jrow[buf * 32 + lane] : P.crow[((size_t)buf * G + b) * 32 + lane];
+      if (lane == 0) s_piv = none ? gj : i;
     }
     __syncthreads();
     const int piv = s_piv;

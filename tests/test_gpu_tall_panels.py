@@ -24,13 +24,40 @@ class Device:
                                          "data": (ptr, False), "version": 2}
 
 
-def test_panels_of_all_ctas(tmp_path):
-    import torch
-    N = 37888 + 128
-    path = os.path.join(str(tmp_path), "chain.vmsh")
+N = 37888 + 128
+
+
+@pytest.fixture(scope="module")
+def matrix(tmp_path_factory):
+    path = os.path.join(str(tmp_path_factory.mktemp("tall")), "chain.vmsh")
     _chain_mesh(path, N)
-    F = buffem.SWGGeometry(meshfiles=path, materials=buffem.Material(eps=2.0)).AllocateVIEMatrix(buffem.BG_C64)
-    V = torch.as_tensor(Device(F), device="cuda")      # V[column, row]
+    return buffem.SWGGeometry(meshfiles=path, materials=buffem.Material(eps=2.0)).AllocateVIEMatrix(buffem.BG_C64)
+
+
+def view(F):
+    import torch
+    return torch.as_tensor(Device(F), device="cuda")   # [column, row]
+
+
+def test_columns_without_a_number_keep_their_rows(matrix):
+    """NaNs in column 40 make every later column one of NaNs: no candidate is left to
+    name a row, and the interchanges stay inside the matrix."""
+    import torch
+    V = view(matrix)
+    V.zero_()
+    V.diagonal().fill_(2.0)
+    V[40] = float("nan")
+    torch.cuda.synchronize()
+    matrix.LUFactorize()
+    assert np.array_equal(matrix.pivots() - 1, np.arange(N))
+    assert bool(torch.isnan(V[40:300, 41:N].abs()).all())
+    V.zero_()
+    torch.cuda.synchronize()
+
+
+def test_panels_of_all_ctas(matrix):
+    import torch
+    F, V = matrix, view(matrix)
     g = torch.Generator(device="cuda").manual_seed(1)
     for c in range(0, N, 4096):
         V[c:c + 4096] = torch.randn(min(4096, N - c), N, dtype=torch.complex64, device="cuda", generator=g)
