@@ -88,9 +88,9 @@ struct FieldK {
   z ik;      // i k
 };
 
-// phase of a tetrahedron's points: e^{ikr} = e^{ik rc} e^{ik(r - rc)}, rc the
+// phase of a tetrahedron's points: e^{ikr} = e^{ik rc} e^{i(k r - k rc)}, rc the
 // distance of its centroid
-struct FieldPhase { double krc; z ec; };
+struct FieldPhase { double k, krc; z ec; };
 
 // One quadrature point: current alpha y - beta at y with weight w.  MODE 3:
 // complex k.  For real k, with a = 1/kr,
@@ -109,7 +109,7 @@ __device__ __forceinline__ void field_point(const FieldK &K, const FieldPhase &F
   for (int c = 0; c < 3; c++) J[c] = z{al.r * y[c] - be[c].r, al.i * y[c] - be[c].i};
   const double R[3] = {x[0] - y[0], x[1] - y[1], x[2] - y[2]};
   const double rr = R[0] * R[0] + R[1] * R[1] + R[2] * R[2];
-  const bool on = rr >= 1e-24;
+  const bool on = !(rr < 1e-24);            // a NaN stays one
   const double r2 = on ? rr : 1.0, ir = rsqrt_fast(r2), r = r2 * ir, m = on ? w * ir : 0.0;
   z A, Bc, C;      // factors of J, (R.J) R and R x J
   if (MODE == 3) {
@@ -129,7 +129,7 @@ __device__ __forceinline__ void field_point(const FieldK &K, const FieldPhase &F
       g = z{m * c, m * s};
     } else {
       z e;
-      const double th = fma(K.k.r, r, -F.krc);
+      const double th = fma(F.k, r, -F.krc);
       if (MODE == 2) cossin_small_short(th, e.r, e.i);
       else cossin_small(th, e.r, e.i);
       e = zmul(F.ec, e);
@@ -242,10 +242,12 @@ __device__ __forceinline__ void tet_point(const FieldK &K, const double *x, cons
                                           double *acc) {
   double d2 = (x[0] - T.ctr[0]) * (x[0] - T.ctr[0]) + (x[1] - T.ctr[1]) * (x[1] - T.ctr[1]) +
               (x[2] - T.ctr[2]) * (x[2] - T.ctr[2]);
-  FieldPhase F{0.0, {1.0, 0.0}};
+  FieldPhase F{K.k.r, 0.0, {1.0, 0.0}};
   if (MODE == 1 || MODE == 2) {
     F.krc = K.k.r * sqrt(d2);
     sincos(F.krc, &F.ec.i, &F.ec.r);
+    // beyond, k r - k rc is rounding only and would leave the range of the series: one phase
+    if (!(fabs(F.krc) < 0x1p48)) F.k = F.krc = 0.0;
   }
   if (d2 > T.Rall * T.Rall) {
     rule4<MODE>(K, F, x, T.V, T.al, T.be, acc);
