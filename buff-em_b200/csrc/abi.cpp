@@ -564,6 +564,7 @@ int bg_matrix_upload(bg_matrix *m, const void *host) {
   size_t esz = m->precision == BG_C128 ? 16 : 8;
   BG_CUDA_TRY(cudaStreamSynchronize(stream()));
   BG_CUDA_TRY(cudaMemcpy2D(m->d, esz * m->ld, host, esz * m->N, esz * m->N, m->N, cudaMemcpyHostToDevice));
+  BG_CUDA_TRY(uploads_done());
   m->factored = false;
   m->symmetric = false;
   return BG_OK;
@@ -815,7 +816,7 @@ int bg_lu_solve(bg_matrix *m, double *B, int nrhs) {
     void *d = nullptr;
     BG_CUDA_TRY(cudaMalloc(&d, sizeof(float) * h.size()));
     int st = BG_OK;
-    cudaError_t e = cudaMemcpy(d, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpyAsync(d, h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice, stream());
     if (e != cudaSuccess) { set_error("H2D: %s", cudaGetErrorString(e)); st = BG_ERR_CUDA; }
     if (!st) st = bg_lu_solve_device(m, d, m->N, nrhs);
     if (!st) {

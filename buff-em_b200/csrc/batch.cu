@@ -100,6 +100,7 @@ static int slot_init(bg_geometry *g, Slot &S, const double *E0, const double *nh
   BG_CUDA_TRY(cudaMemset(S.out, 0, sizeof(double) * BATCH_MAXOBJ));
   const double one[2] = {1.0, 0.0};
   BG_CUDA_TRY(cudaMemcpy(S.fq, one, sizeof one, cudaMemcpyHostToDevice));
+  BG_CUDA_TRY(uploads_done());
   set_thread_stream(S.s);
   st = lu_capture_prepare(S.M);
   if (!st && use_graph && !s_warm) {
@@ -353,6 +354,7 @@ int bg_batch_sweep(bg_geometry *const *geoms, int ngeom, const double *omega, in
   for (int i = 0; i < ngeom && !st; i++) {
     double tun[4] = {0, 0, 0, 0};
     cudaError_t e0 = cudaMemset(d_out, 0, sizeof(double) * BATCH_MAXOBJ * (size_t)nomega);
+    if (e0 == cudaSuccess) e0 = uploads_done();
     if (e0 != cudaSuccess) { set_error("bg_batch_sweep: %s", cudaGetErrorString(e0)); st = BG_ERR_CUDA; break; }
     st = sweep_geometry(geoms[i], h_w, nomega, E0, nhat, max_streams, use_graph, d_out, tun);
     if (!st) {

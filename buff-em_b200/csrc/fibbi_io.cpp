@@ -139,9 +139,11 @@ int bg_fibbi_load(bg_geometry *g, int obj, const char *path, int *matched) {
     std::memcpy(data.data() + kDataDoubles * k, it->second.data(), sizeof(double) * kDataDoubles);
     n++;
   }
-  if (n && g->near.npairs)
+  if (n && g->near.npairs) {
     BG_CUDA_TRY(cudaMemcpy(g->near.fibbi, data.data(), sizeof(double) * kDataDoubles * g->near.npairs,
                            cudaMemcpyHostToDevice));
+    BG_CUDA_TRY(uploads_done());
+  }
   if (matched) *matched = n;
   return BG_OK;
 }

@@ -75,6 +75,7 @@ int init_rule16() {
       p += 3;
     }
   BG_CUDA_TRY(cudaMemcpyToSymbol(c_fr16, h, sizeof h));
+  BG_CUDA_TRY(uploads_done());
   s_fr16_ok = true;
   return BG_OK;
 }
@@ -480,6 +481,7 @@ static int field_tables(bg_geometry *g) {
   if (e == cudaSuccess) e = cudaMalloc(&dF, sizeof(double) * F.size());
   if (e == cudaSuccess) e = cudaMemcpy(dT, T.data(), sizeof(double) * T.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dF, F.data(), sizeof(double) * F.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = uploads_done();
   if (e != cudaSuccess) {
     // both tables or neither: a failed build leaves the geometry as it was
     cudaFree(dT);

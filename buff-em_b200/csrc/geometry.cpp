@@ -209,8 +209,9 @@ int refresh_materials(bg_geometry *g, double wr, double wi) {
       DevExpr prog{};
       int st = svtensor_compile(*o.svt, wr, wi, &prog);
       if (st) return st;
-      // synchronous from pageable memory: prog may leave scope at once
+      // pageable source: prog may leave scope at once
       BG_CUDA_TRY(cudaMemcpy(g->dev.expr + i, &prog, sizeof(DevExpr), cudaMemcpyHostToDevice));
+      BG_CUDA_TRY(uploads_done());
     } else if (o.svt) {
       const double x0[3] = {0.0, 0.0, 0.0};   // position-independent by construction
       o.mat = bg_material{};
@@ -343,6 +344,7 @@ int upload_geometry(bg_geometry *g) {
     BG_CUDA_TRY(cudaMalloc((void **)&d.expr, sizeof(DevExpr) * g->objs.size()));
     BG_CUDA_TRY(cudaMemset(d.expr, 0, sizeof(DevExpr) * g->objs.size()));
   }
+  BG_CUDA_TRY(uploads_done());
   g->uploaded = true;
   return BG_OK;
 }
@@ -505,6 +507,7 @@ int build_near_lists(bg_geometry *g) {
     return st;
   BG_CUDA_TRY(cudaMalloc(&nd.fibbi, sizeof(double) * 6 * std::max(1, nd.npairs)));
   BG_CUDA_TRY(cudaMalloc(&nd.tpMom, sizeof(double) * 24 * std::max(1, ntp)));
+  BG_CUDA_TRY(uploads_done());
   return BG_OK;
 }
 

@@ -937,6 +937,7 @@ static int ensure_graph(bg_geometry *g) {
   BG_CUDA_TRY(cudaMemcpy(G.rowptr, rowptr.data(), sizeof(int) * (N + 1), cudaMemcpyHostToDevice));
   BG_CUDA_TRY(cudaMemcpy(G.col, col.data(), sizeof(int) * E, cudaMemcpyHostToDevice));
   BG_CUDA_TRY(cudaMemcpy(G.etr, etr.data(), sizeof(int) * E, cudaMemcpyHostToDevice));
+  BG_CUDA_TRY(uploads_done());
   g->graph = G;
   return BG_OK;
 }
@@ -1276,6 +1277,7 @@ int bg_gnn_create(unsigned long long seed, bg_gnn **out) {
   net->sumsq = (double *)(net->params + ((4 * (size_t)n + 1) & ~(size_t)1));
   e = cudaMemset(net->params, 0, sizeof(float) * (nalloc + 2));
   if (e == cudaSuccess) e = cudaMemcpy(net->params, p.data(), sizeof(float) * n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = uploads_done();
   if (e != cudaSuccess) {
     cudaFree(net->params);
     delete net;
@@ -1307,6 +1309,7 @@ int bg_gnn_set_params(bg_gnn *net, const float *host) {
   BG_CUDA_TRY(cudaMemcpy(net->params, host, sizeof(float) * LAY.total, cudaMemcpyHostToDevice));
   net->step = 0;
   BG_CUDA_TRY(cudaMemset(net->m, 0, sizeof(float) * 2 * LAY.total));
+  BG_CUDA_TRY(uploads_done());
   return BG_OK;
 }
 

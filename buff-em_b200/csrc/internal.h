@@ -42,6 +42,12 @@ extern std::atomic<long long> g_launches;
     }                                                                              \
   } while (0)
 
+// A copy from pageable memory may return once its last bytes are staged, and a
+// memset as soon as it is queued, both still on their way on the null stream.
+// The library's streams do not wait for that one, so whoever fills device
+// memory through it calls this before a kernel may read the memory.
+inline cudaError_t uploads_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 cudaStream_t stream();
 void set_thread_stream(cudaStream_t s);   // nullptr: back to the library stream
 int ensure_device();

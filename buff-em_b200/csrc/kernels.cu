@@ -59,6 +59,7 @@ static int init_tables() {
   fill_rule(h_tcr33, "IJJ IJK IKJ JIJ JIK JJI JJK JKI JKJ KIJ KJI KJJ", v33, 0.013950789384495153, &np);
   BG_CUDA_TRY(cudaMemcpyToSymbol(c_tcr16, h_tcr16, sizeof h_tcr16));
   BG_CUDA_TRY(cudaMemcpyToSymbol(c_tcr33, h_tcr33, sizeof h_tcr33));
+  BG_CUDA_TRY(uploads_done());
   s_tables_ok = 1;
   return BG_OK;
 }

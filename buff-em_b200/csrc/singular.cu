@@ -74,6 +74,7 @@ static int sg_tables() {
   for (int n = 1; n <= 16; n++) gauss_legendre01(n, x[n], w[n]);
   BG_CUDA_TRY(cudaMemcpyToSymbol(c_sgx, x, sizeof x));
   BG_CUDA_TRY(cudaMemcpyToSymbol(c_sgw, w, sizeof w));
+  BG_CUDA_TRY(uploads_done());
   s_sg_tables = true;
   return BG_OK;
 }
